@@ -310,8 +310,8 @@ void finish_csr_from_arc_keys(stc_ctx* c, DeviceGraph& g, uint64_t* akeys, uint6
   range_scan(LoadU32{g.fdeg}, EmitOffset{g.off}, g.n, sums, c->stream, &c->launches);
   STC_CUDA(cudaMemcpyAsync(g.off + g.n, sums + range_partition(g.n, kScanTile, kMaxSortGrid).grid,
                            sizeof(uint64_t), cudaMemcpyDeviceToDevice, c->stream));
-  g.nbr = buffer<uint32_t>(c, B_NBR, g.m_fwd + 4);  // + 4: the engine reads whole int4 chunks
-  g.sgn = buffer<int8_t>(c, B_SGN, g.m_fwd + 4);
+  g.nbr = buffer<uint32_t>(c, B_NBR, g.m_fwd + 8);  // + 8: the engine reads whole 32-byte chunks
+  g.sgn = buffer<int8_t>(c, B_SGN, g.m_fwd + 8);
   g.asrc = buffer<uint32_t>(c, B_ASRC, g.m_fwd);
   g.nkey = buffer<uint32_t>(c, B_NKEY, g.m_fwd + 8);
   k_csr_fill<<<grid_for(g.m_fwd, 4), kThreads, 0, c->stream>>>(sorted, g.m_fwd, g.bits, g.fdeg,
@@ -809,8 +809,8 @@ void build_totals(stc_ctx* c, const EdgeIds& e, const int8_t* d_sign, uint64_t m
                                cudaMemcpyDeviceToDevice, st));
       g.m_unique = g.m_fwd = m;
       g.m_dev = ctr + C_BATCH_MU;
-      g.nbr = buffer<uint32_t>(c, B_NBR, m + 4);
-      g.sgn = buffer<int8_t>(c, B_SGN, m + 4);
+      g.nbr = buffer<uint32_t>(c, B_NBR, m + 8);
+      g.sgn = buffer<int8_t>(c, B_SGN, m + 8);
       g.asrc = buffer<uint32_t>(c, B_ASRC, m);
       g.nkey = buffer<uint32_t>(c, B_NKEY, m + 8);
       range_apply(flag, EmitArc{sorted, g.bits, g.nbr, g.sgn, g.asrc, g.nkey}, m, sums, st,
@@ -823,8 +823,8 @@ void build_totals(stc_ctx* c, const EdgeIds& e, const int8_t* d_sign, uint64_t m
                                cudaMemcpyDeviceToHost, st));
       STC_CUDA(cudaStreamSynchronize(st));
       g.m_unique = g.m_fwd = c->h_pinned[C_WORK];
-      g.nbr = buffer<uint32_t>(c, B_NBR, g.m_fwd + 4);  // + 4: the engine reads whole int4 chunks
-      g.sgn = buffer<int8_t>(c, B_SGN, g.m_fwd + 4);
+      g.nbr = buffer<uint32_t>(c, B_NBR, g.m_fwd + 8);  // + 8: the engine reads whole 32-byte chunks
+      g.sgn = buffer<int8_t>(c, B_SGN, g.m_fwd + 8);
       g.asrc = buffer<uint32_t>(c, B_ASRC, g.m_fwd);
       g.nkey = buffer<uint32_t>(c, B_NKEY, g.m_fwd + 8);
       range_apply(flag, EmitArc{sorted, g.bits, g.nbr, g.sgn, g.asrc, g.nkey}, g.m_valid, sums,

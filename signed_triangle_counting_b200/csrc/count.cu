@@ -1334,7 +1334,8 @@ void launch_classes(cudaStream_t st, const Csr& csr, const uint32_t* lists, cons
 constexpr uint32_t kHeadMaxB = kLargeCap - 1;  // |N+(v)| of a HEAD arc: bucket <= 12
 static_assert(32 - __builtin_clz(kHeadMaxB) == 12 && 32 - __builtin_clz(kHeadMaxB + 1) == 13,
               "HEAD cells (bucket |B| <= 12) are exactly the arcs whose head fits the large class");
-constexpr int kHeadClasses = 3;
+constexpr int kHeadClasses = 4;
+constexpr uint32_t kHeadBits = 3;  // the bitmap class (k_head_bits)
 // Head list buffer: plan words first (start of class c's list, then from
 // kHeadPlanCount its count), the class lists after them, then one byte per
 // vertex: whether it keeps arcs for the tail side.
@@ -1344,7 +1345,7 @@ constexpr uint32_t kHeadItemMin = 2048;  // the smallest class item size
 
 // In-arcs per work item of head class c (powers of two).
 __host__ __device__ __forceinline__ uint32_t head_item(uint32_t c) {
-  return c == 0 ? kHeadItemMin : c == 1 ? 8192u : 16384u;
+  return c == 0 ? kHeadItemMin : c == 2 ? 16384u : 8192u;
 }
 
 // Table class of a list of d arcs (tiny lists use the warp class's table).
@@ -1356,6 +1357,42 @@ __device__ __forceinline__ uint32_t table_class(uint32_t d) {
 __device__ __forceinline__ uint32_t head_class(uint32_t d) {
   return d <= kWarpCap ? 0u : d <= kBlockCap ? 1u : 2u;
 }
+
+// Ranks a bitmap covers (two bits each: 64 KB, so two CTAs of 512 threads and
+// an L1 for the stream share an SM), and the shortest |N+(v)| that is worth a
+// CTA and a bitmap of its own.  At RMAT scale 24 the top 2^18 ranks are the
+// heads of 90% of the arcs and 97% of the probes; the heads below keep the
+// hash.
+constexpr uint32_t kBitsWindow = 1u << 18;
+constexpr uint32_t kBitsWords = kBitsWindow / 16;
+constexpr uint32_t kBitsMinB = kWarpCap;
+constexpr int kBitsThreads = 512;
+
+// Which head vertices take the bitmap: v's list and every A' of its in-arcs
+// lie in (v, last rank of v's graph], so the bitmap, indexed by the low bits
+// of the rank, holds them without collision when that range is at most
+// `window` long (0: no bitmap).
+struct BitsRule {
+  uint32_t window;
+  uint32_t n;
+  const uint64_t* gbase;  // G + 1 rank boundaries of a batch, or null
+  uint32_t G;
+  __device__ __forceinline__ uint32_t head_class_of(uint32_t v, uint32_t d) const {
+    if (d > kBitsMinB && window) {
+      uint32_t end = n;
+      if (gbase) {
+        uint32_t lo = 0, hi = G;
+        while (hi - lo > 1) {
+          const uint32_t mid = (lo + hi) >> 1;
+          if (gbase[mid] <= v) lo = mid; else hi = mid;
+        }
+        end = (uint32_t)gbase[lo + 1];
+      }
+      if (end - v <= window) return kHeadBits;
+    }
+    return head_class(d);
+  }
+};
 
 struct HeadArcs {
   const uint64_t* __restrict__ keys;  // sorted: v << 32 | arc index
@@ -1452,10 +1489,10 @@ __global__ void __launch_bounds__(256) k_head_runs(const uint64_t* __restrict__ 
                                                    const uint64_t* __restrict__ off,
                                                    unsigned long long* __restrict__ ctr,
                                                    uint32_t* __restrict__ hl,
-                                                   uint32_t* __restrict__ end) {
+                                                   uint32_t* __restrict__ end, BitsRule rule) {
   const uint64_t m = ctr[C_HEAD_NKEYS];
   const uint32_t lane = lane_id();
-  uint32_t cnt[kHeadClasses] = {0, 0, 0};
+  uint32_t cnt[kHeadClasses] = {0, 0, 0, 0};
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < m;
        base += stride) {
@@ -1464,8 +1501,11 @@ __global__ void __launch_bounds__(256) k_head_runs(const uint64_t* __restrict__ 
     if (j < m) {
       const uint64_t kv = keys[j] >> 32;
       const uint32_t v = (uint32_t)kv;
-      const uint32_t hc = head_class((uint32_t)(off[v + 1] - off[v]));
-      if (j == 0 || (keys[j - 1] >> 32) != kv || (j & (head_item(hc) - 1)) == 0) c = hc;
+      const bool run = j == 0 || (keys[j - 1] >> 32) != kv;
+      if (run || (j & (kHeadItemMin - 1)) == 0) {
+        const uint32_t hc = rule.head_class_of(v, (uint32_t)(off[v + 1] - off[v]));
+        if (run || (j & (head_item(hc) - 1)) == 0) c = hc;
+      }
       if (kFill && (j + 1 == m || (keys[j + 1] >> 32) != kv)) end[v] = (uint32_t)(j + 1);
     }
     if (!kFill) {
@@ -1717,6 +1757,173 @@ __global__ void __launch_bounds__(THREADS) k_head_block(Csr g, HeadArcs h,
   if (!kVC) flush_counts<THREADS>(tc, ctr);
 }
 
+// Sign bits of the arcs, one byte per eight: entry e of the group at bit
+// 7 - e (the order in which k_head_bits collects its hits).
+__global__ void __launch_bounds__(256) k_sign_bits(const int8_t* __restrict__ sgn, uint64_t m,
+                                                   const unsigned long long* __restrict__ m_dev,
+                                                   uint8_t* __restrict__ sbits) {
+  if (m_dev) m = min(m, (uint64_t)*m_dev);
+  const uint64_t groups = (m + 7) / 8;
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < groups; i += stride) {
+    const uint2 q = reinterpret_cast<const uint2*>(sgn)[i];
+    // Sign bits at 7, 15, 23, 31; the multiply gathers them at 31..28.
+    const uint32_t a = ((q.x >> 7) & 0x01010101u) * 0x80402010u >> 28;
+    const uint32_t b = ((q.y >> 7) & 0x01010101u) * 0x80402010u >> 28;
+    sbits[i] = (uint8_t)((a << 4) | b);
+  }
+}
+
+// Head vertices whose lists fit a bitmap: one CTA per work item from a
+// dynamic queue.  N+(v) is staged as a bitmap over the ranks (mod
+// kBitsWindow), two bits per rank, 16 ranks per 32-bit word: for rank x, the
+// bit at x & 31 says that x is in N+(v) with a positive sign, the bit at
+// (x & 31) ^ 16 that it is with a negative one.  Rotating the word right by x
+// brings the two to bits 0 and 16, so a streamed entry costs one 4-byte
+// shared load and five integer instructions (address: shift and mask;
+// rotate, mask, append to the lane's hit masks), against about 18 and an
+// 8-byte load for the hash, and staging an entry is one shared atomic.
+// Entries outside an arc's extent alias some other rank's bits; their hits
+// are masked out per chunk.
+//
+// Warps take 32 in-arcs at a time: each lane holds one arc's extent, and the
+// arcs' aligned 8-entry chunks form one sequence.  The arc of a lane's chunk
+// follows from a bit mask of the arc starts inside the warp's 32 chunks (one
+// or-reduction, as every arc has at least one chunk) and its extent from
+// shuffles, so there is no tile in shared memory and no CTA barrier between
+// tiles.  The eight hits of a chunk are classified together: three
+// population counts of the hit masks against the chunk's sign byte.
+//
+// RMAT scale 24 (97% of the 41.8 G probes): 42.4 ms, against 78.8 ms of hash
+// probes for the same heads; scale 22: 3.85 G warp instructions against
+// 9.98 G.  What bounds it now is waiting, at the two barriers of a work item
+// and for the streamed chunks (issue slots 38% used, DRAM 2.1 TB/s).
+template <int THREADS, class Sink>
+__global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_head_bits(
+    Csr g, HeadArcs h, const uint8_t* __restrict__ sbits, const uint32_t* __restrict__ hl,
+    unsigned long long* __restrict__ ctr, Sink sink) {
+  constexpr bool kVC = Sink::kPerVertex;
+  constexpr int U = 2;  // chunks in flight per lane
+  constexpr uint32_t kDrainRounds = 255 / (8 * U);  // 8-bit fields, 8 adds a chunk at most
+  extern __shared__ __align__(16) uint32_t bm[];  // kBitsWords
+  __shared__ uint32_t s_item, s_next;
+  const uint32_t lane = lane_id(), le = lanemask_lt() | (1u << lane);
+  const uint32_t* list = hl + kHeadPlanWords + hl[kHeadBits];
+  const uint32_t cnt = hl[kHeadPlanCount + kHeadBits];
+  TypeCounts tc;
+  uint32_t cur = 0xFFFFFFFFu;  // per-key counts as in k_head_block
+  auto flush = [&]() {
+    if (kVC && cur != 0xFFFFFFFFu) {
+      block_key_flush<THREADS>(tc, cur, sink);
+      tc = TypeCounts{};
+    }
+  };
+  for (uint32_t i = threadIdx.x; i < kBitsWords; i += THREADS) bm[i] = 0;
+  while (true) {
+    if (threadIdx.x == 0) {
+      s_item = (uint32_t)atomicAdd(ctr + C_HEAD_QUEUE + kHeadBits, 1ull);
+      s_next = 0;
+    }
+    __syncthreads();  // the last item's bits are cleared
+    const uint32_t item = s_item;
+    if (item >= cnt) break;
+    uint32_t v, j1;
+    const uint32_t j0 = list[item];
+    h.item(j0, kHeadBits, v, j1);
+    const uint64_t vb = g.off[v];
+    const uint32_t d = (uint32_t)(g.off[v + 1] - vb);
+    if (kVC) {
+      const uint32_t key = sink.key(v);  // uniform over the CTA
+      if (key != cur) {
+        flush();
+        cur = key;
+      }
+    }
+    for (uint32_t i = threadIdx.x; i < d; i += THREADS) {
+      const uint32_t x = g.nbr[vb + i];
+      const uint32_t neg = g.sgn[vb + i] < 0;
+      atomicOr(&bm[(x >> 4) & (kBitsWords - 1)], 1u << ((x & 31u) ^ (neg << 4)));
+    }
+    __syncthreads();
+    const uint32_t arcs = j1 - j0;
+    PackedCounts8 p8;
+    uint32_t rounds = 0;
+    while (true) {
+      uint32_t b = 0;
+      if (lane == 0) b = atomicAdd(&s_next, 32u);
+      b = __shfl_sync(kFull, b, 0);
+      if (b >= arcs) break;
+      // This lane's in-arc: A' extent [lo, hi), chunks, 8 * (arc negative).
+      uint32_t lo = 0, hi = 0, c = 0, sh = 0;
+      if (b + lane < arcs) {
+        const uint32_t i = (uint32_t)h.keys[j0 + b + lane];
+        lo = i + 1;
+        hi = h.aend[i];  // > lo: a HEAD arc has a non-empty A'
+        c = ((hi + 7) >> 3) - (lo >> 3);
+        sh = ((sbits[i >> 3] >> (7u - (i & 7u))) & 1u) << 3;
+      }
+      const uint32_t inc = warp_inclusive_scan(c);
+      const uint32_t start = c ? inc - c : 0xFFFFFFFFu;
+      const uint32_t cb = (lo >> 3) - start;  // group index = cb + chunk index
+      const uint32_t total = __shfl_sync(kFull, inc, 31);
+      uint32_t k0 = 0xFFFFFFFFu;  // arcs started before the round, less one
+      for (uint32_t base = 0; base < total; base += 32 * U) {
+        uint4 qa[U], qb[U];
+        uint32_t sb[U], vm[U], ash[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          const uint32_t w0 = base + 32 * u;
+          const uint32_t rel = start - w0;
+          const uint32_t starts = __reduce_or_sync(kFull, rel < 32u ? 1u << rel : 0u);
+          const uint32_t k = k0 + __popc(starts & le);
+          k0 += __popc(starts);
+          const uint32_t ci = __shfl_sync(kFull, cb, k) + w0 + lane;
+          const uint32_t klo = __shfl_sync(kFull, lo, k), khi = __shfl_sync(kFull, hi, k);
+          ash[u] = __shfl_sync(kFull, sh, k);
+          vm[u] = 0;
+          if (w0 + lane < total) {
+            const uint4* src = reinterpret_cast<const uint4*>(g.nbr) + 2ull * ci;
+            qa[u] = src[0];
+            qb[u] = src[1];
+            sb[u] = sbits[ci];
+            const uint32_t g0 = 8 * ci;
+            const uint32_t first = klo > g0 ? klo - g0 : 0u;
+            const uint32_t last = min(khi - g0, 8u);
+            vm[u] = (0xFFu >> first) & (0xFFu << (8u - last));
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          if (vm[u] == 0) continue;
+          uint32_t acc = 0;  // hits: positive in bits 0-7, negative in bits 16-23
+#pragma unroll
+          for (uint32_t e = 0; e < 8; e++) {
+            const uint32_t x = e < 4 ? pick4(qa[u], e) : pick4(qb[u], e - 4);
+            const uint32_t w = bm[(x >> 4) & (kBitsWords - 1)];
+            acc = 2 * acc + (__funnelshift_r(w, w, x) & 0x10001u);
+          }
+          acc &= vm[u] * 0x10001u;
+          const uint32_t neg = acc & (sb[u] * 0x10001u);
+          const uint32_t e2 = __popc(neg >> 16);
+          const uint32_t e0 = __popc((acc ^ neg) & 0xFFFFu);
+          const uint32_t e1 = __popc(acc) - e0 - e2;
+          p8.w += (e0 + (e1 << 8) + (e2 << 16)) << ash[u];
+        }
+        if (++rounds == kDrainRounds) {
+          p8.drain(tc);
+          rounds = 0;
+        }
+      }
+    }
+    p8.drain(tc);
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < d; i += THREADS)
+      bm[(g.nbr[vb + i] >> 4) & (kBitsWords - 1)] = 0;
+  }
+  flush();
+  if (!kVC) flush_counts<THREADS>(tc, ctr);
+}
+
 // Device buffers of the head-side pass (allocated before any capture).
 struct HeadBufs {
   uint64_t* keys = nullptr;
@@ -1726,6 +1933,7 @@ struct HeadBufs {
   uint32_t* hl = nullptr;    // plan words, class lists of work items
   uint8_t* need = nullptr;   // per tail: it keeps arcs for the tail side
   uint32_t* sort_counts = nullptr;
+  uint8_t* sbits = nullptr;  // sign bits of the arcs
 };
 
 HeadBufs head_buffers(stc_ctx* c, const DeviceGraph& g) {
@@ -1740,6 +1948,7 @@ HeadBufs head_buffers(stc_ctx* c, const DeviceGraph& g) {
   b.hl = buffer<uint32_t>(c, B_HEAD_LIST, kHeadPlanWords + items + (g.n + 3) / 4);
   b.need = reinterpret_cast<uint8_t*>(b.hl + kHeadPlanWords + items);
   b.sort_counts = buffer<uint32_t>(c, B_SORT_COUNTS, (size_t)kRadix * kMaxSortGrid);
+  b.sbits = buffer<uint8_t>(c, B_SBITS, (g.m_fwd + 7) / 8);
   return b;
 }
 
@@ -1765,6 +1974,10 @@ void prepare_head(const Tuning& tu) {
       STC_CUDA(cudaFuncSetAttribute(k_head_block<512, Sink, kTime, kU>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sl));
   });
+  if constexpr (!kTime)
+    STC_CUDA(cudaFuncSetAttribute(k_head_bits<kBitsThreads, Sink>,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)(kBitsWords * sizeof(uint32_t))));
 }
 
 // The head-side pass is enqueued on `st` (no host synchronisation) in two
@@ -1778,7 +1991,7 @@ inline void enqueue_head_keys(cudaStream_t st, const Csr& csr, const uint32_t* a
                               const uint8_t* d_tables,
                               const unsigned long long* range, unsigned long long* ctr,
                               int& launches) {
-  STC_CUDA(cudaMemsetAsync(ctr + C_HEAD_COUNT, 0, 9 * sizeof(unsigned long long), st));
+  STC_CUDA(cudaMemsetAsync(ctr + C_HEAD_COUNT, 0, 3 * kHeadClasses * sizeof(unsigned long long), st));
   STC_CUDA(cudaMemsetAsync(ctr + C_HEAD_NKEYS, 0, sizeof(unsigned long long), st));
   STC_CUDA(cudaMemsetAsync(b.need, 0, csr.n, st));
   const uint32_t grid = (uint32_t)std::min<uint64_t>((m + 1023) / 1024, kSMs * 8);
@@ -1791,6 +2004,7 @@ inline void enqueue_head_keys(cudaStream_t st, const Csr& csr, const uint32_t* a
 
 template <class Sink, bool kTime>
 void enqueue_head(cudaStream_t st, const Csr& csr, const uint32_t* asrc, uint64_t m,
+                  const unsigned long long* m_dev, const uint64_t* gbase, uint32_t G,
                   const HeadBufs& b, unsigned long long* ctr, const Sink& sink,
                   const ArcTimes& at, const Tuning& tu, int& launches,
                   uint32_t class_mask = 0x3F) {
@@ -1800,11 +2014,25 @@ void enqueue_head(cudaStream_t st, const Csr& csr, const uint32_t* asrc, uint64_
   const uint64_t* sorted = radix_sort(b.keys, b.alt, m, 32, 32 + (int)vbits, b.sort_counts, st,
                                       &sort_launches, ctr + C_HEAD_NKEYS);
   uint32_t* end = b.runs;
-  k_head_runs<false><<<kSMs * 4, 256, 0, st>>>(sorted, csr.off, ctr, b.hl, end);
+  // The recorder times single arcs against a staged hash: no bitmap there.
+  const BitsRule rule{kTime ? 0u : kBitsWindow, n, gbase, G};
+  k_head_runs<false><<<kSMs * 4, 256, 0, st>>>(sorted, csr.off, ctr, b.hl, end, rule);
   k_head_plan<<<1, 32, 0, st>>>(ctr, b.hl);
-  k_head_runs<true><<<kSMs * 4, 256, 0, st>>>(sorted, csr.off, ctr, b.hl, end);
+  k_head_runs<true><<<kSMs * 4, 256, 0, st>>>(sorted, csr.off, ctr, b.hl, end, rule);
   const HeadArcs h{sorted, b.aend, end, asrc};
   launches += 3 + sort_launches;
+  if constexpr (!kTime) {
+    if (class_mask & 4u) {
+      k_sign_bits<<<kSMs * 8, 256, 0, st>>>(csr.sgn, m, m_dev, b.sbits);
+      k_head_bits<kBitsThreads, Sink>
+          <<<kSMs * (1024 / kBitsThreads), kBitsThreads, kBitsWords * sizeof(uint32_t), st>>>(
+              csr, h, b.sbits, b.hl, ctr, sink);
+      launches += 2;
+    }
+  }
+  // With every rank inside the window the bitmap takes all lists longer than
+  // the warp class's.
+  const bool low = kTime || gbase || n > kBitsWindow;
   // Head class c runs with class_mask bit c + 1, as the tail side's class of
   // the same tuning (the autotuner times one class at a time).
   with_unroll(kTime ? kStreamUnroll : tu.unroll[0], [&](auto U) {
@@ -1814,7 +2042,7 @@ void enqueue_head(cudaStream_t st, const Csr& csr, const uint32_t* asrc, uint64_
         k_head_warp<Sink, kTime, kU><<<kSMs * 4, 256, 0, st>>>(csr, h, b.hl, ctr, sink, at,
                                                                tu.hash_factor[0]);
   });
-  if (class_mask & 4u) {
+  if (low && (class_mask & 4u)) {
     const uint32_t cap = kBlockCap;
     const uint32_t hf = fit_hash_factor(tu.hash_factor[1], cap);
     const uint32_t nb = hf * cap;
@@ -1830,7 +2058,7 @@ void enqueue_head(cudaStream_t st, const Csr& csr, const uint32_t* asrc, uint64_
       });
     });
   }
-  if (class_mask & 8u) {
+  if (low && (class_mask & 8u)) {
     const uint32_t cap = kLargeCap;
     const uint32_t hf = fit_hash_factor(tu.hash_factor[2], cap);
     const uint32_t nb = hf * cap;
@@ -1842,7 +2070,7 @@ void enqueue_head(cudaStream_t st, const Csr& csr, const uint32_t* asrc, uint64_
                                                                      ctr, sink, at);
     });
   }
-  launches += 3;
+  launches += low ? 3 : 1;
   STC_CUDA(cudaGetLastError());
 }
 
@@ -1928,6 +2156,8 @@ struct HeadPlan {
   const uint32_t* fdeg = nullptr;
   uint64_t m = 0;
   const unsigned long long* m_dev = nullptr;  // arc count on the device when m is a capacity
+  const uint64_t* gbase = nullptr;  // G + 1 rank boundaries of a batch
+  uint32_t G = 0;
   Tuning tuning;
 };
 
@@ -1958,15 +2188,15 @@ void enqueue_persistent(cudaStream_t st, const Csr& csr, const ClassBounds& cb, 
                                                       d_tables + 256 * kTableGiant, none, plan, 4);
   launches += 6;
   if (hp.bufs)
-    enqueue_head<Sink, false>(st, csr, hp.asrc, hp.m, *hp.bufs, ctr, sink, none, hp.tuning,
-                              launches);
+    enqueue_head<Sink, false>(st, csr, hp.asrc, hp.m, hp.m_dev, hp.gbase, hp.G, *hp.bufs, ctr, sink,
+                              none, hp.tuning, launches);
   STC_CUDA(cudaGetLastError());
 }
 
 // Identity of a captured persistent sequence: every pointer and size its
 // kernels were given.
 struct PersistentKey {
-  const void* p[17];
+  const void* p[19];
   uint64_t v[6];
 };
 
@@ -1996,8 +2226,8 @@ void count_persistent(stc_ctx* c, const Csr& csr, const ClassBounds& cb, uint32_
   }
   PersistentKey key{};
   const HeadBufs hb = hp.bufs ? *hp.bufs : HeadBufs{};
-  const void* ptrs[17] = {csr.off, csr.nbr, csr.sgn, csr.verts, lists, plan, ctr, d_tables, s0,
-                          hp.asrc, hb.keys, hb.alt, hb.aend, hb.runs, hb.hl, hp.fdeg, csr.nkey};
+  const void* ptrs[19] = {csr.off, csr.nbr, csr.sgn, csr.verts, lists, plan, ctr, d_tables, s0,
+                          hp.asrc, hb.keys, hb.alt, hb.aend, hb.runs, hb.hl, hp.fdeg, csr.nkey, hb.sbits, hp.gbase};
   memcpy(key.p, ptrs, sizeof(ptrs));
   key.v[0] = csr.n;
   key.v[1] = cb.tiny_max;
@@ -2282,6 +2512,8 @@ void count_triangles(stc_ctx* c, const DeviceGraph& gin, const CountConfig& cfg)
       hp.fdeg = g.fdeg;
       hp.m = g.m_fwd;
       hp.m_dev = g.m_dev;
+      hp.gbase = g.G ? g.gbase : nullptr;
+      hp.G = g.G;
       hp.tuning = c->tuning;
     }
     if (cfg.vertex_counts) {
@@ -2331,8 +2563,8 @@ void count_triangles(stc_ctx* c, const DeviceGraph& gin, const CountConfig& cfg)
                              c->tuning, cfg.class_mask, c->launches);
     if (head) {
       prepare_head<Sink, kT>(c->tuning);
-      enqueue_head<Sink, kT>(st, csr, g.asrc, g.m_fwd, hb, ctr, sink, at, c->tuning,
-                             c->launches, cfg.class_mask);
+      enqueue_head<Sink, kT>(st, csr, g.asrc, g.m_fwd, g.m_dev, g.G ? g.gbase : nullptr, g.G, hb,
+                             ctr, sink, at, c->tuning, c->launches, cfg.class_mask);
     }
   };
   if (timed) {

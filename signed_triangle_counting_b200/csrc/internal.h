@@ -48,6 +48,7 @@ enum BufId {
   B_HEAD_RUNS,                    // head-side pass: in-arc range per head vertex (2 n)
   B_HEAD_LIST,                    // head-side pass: head vertices by class, plan, flags
   B_NKEY,                         // arcs: head << 1 | negative (m + 8)
+  B_SBITS,                        // arcs: sign bits, one byte per 8 arcs (the head bitmap's stream)
   B_RELABEL,                      // ids >= 2^31 - 1: the edges relabelled to dense ids (2 m)
   B_DISTINCT,                     // ids >= 2^31 - 1: the sorted distinct ids
   B_COUNT_
@@ -71,15 +72,15 @@ enum CounterSlot {
   C_SHARD_LO = 18,             // rank range [lo, hi) of a sharded count
   C_SHARD_HI = 19,
   C_QUEUE_WARP = 20,           // warp-granular work queue of the persistent engine
-  C_HEAD_COUNT = 21,           // head-side pass: head vertices per class (3 slots),
-  C_HEAD_CURSOR = 24,          // their list fill cursors (3 slots)
-  C_HEAD_QUEUE = 27,           // and the classes' work queues (3 slots)
   C_PROBE_BYTES = 30,          // probe-model bytes of the CSR
   C_HEAD_NKEYS = 31,           // head-side pass: keys (HEAD arcs) appended
   C_BATCH_N = 32,              // capped batch build: vertices of the union
   C_BATCH_MU = 33,             // capped batch build: unique edges (= arcs)
   C_OVERFLOW = 34,             // capped batch build: a capacity was exceeded (results void)
-  C_SLOTS = 40
+  C_HEAD_COUNT = 36,           // head-side pass: work items per class (4 slots),
+  C_HEAD_CURSOR = 40,          // their list fill cursors (4 slots)
+  C_HEAD_QUEUE = 44,           // and the classes' work queues (4 slots)
+  C_SLOTS = 48
 };
 
 // Values of the device error word: 1 = malformed forward CSR,
@@ -167,7 +168,7 @@ struct stc_ctx {
   // The persistent count captured in a CUDA graph, and the pointers and
   // sizes it was captured with (replayed while they stay the same).
   cudaGraphExec_t graph_exec = nullptr;
-  uint64_t graph_key[24] = {};
+  uint64_t graph_key[32] = {};
   int graph_launches = 0;  // kernels per replay of graph_exec
   stc::Tuning tuning;
   // Batch groups captured whole (at most four, the least recently used
