@@ -318,6 +318,7 @@ void finish_csr_from_arc_keys(stc_ctx* c, DeviceGraph& g, uint64_t* akeys, uint6
                                                                g.off, g.nbr, g.sgn, g.asrc,
                                                                g.nkey,
                                                                (unsigned long long*)counters(c));
+  g.bytes_done = true;
   c->launches += 1;
   STC_CUDA(cudaGetLastError());
 }
@@ -841,11 +842,7 @@ void build_totals(stc_ctx* c, const EdgeIds& e, const int8_t* d_sign, uint64_t m
   } else {
     STC_CUDA(cudaMemsetAsync(g.off, 0, sizeof(uint64_t), st));
   }
-  if (g.m_fwd) {
-    k_alg_bytes<<<grid_for(g.m_fwd, 4), kThreads, 0, st>>>(g.asrc, g.nbr, g.m_fwd, g.m_dev, g.off,
-                                                           g.fdeg, ctr);
-    c->launches++;
-  } else {
+  if (!g.m_fwd) {
     g.nbr = buffer<uint32_t>(c, B_NBR, 4);
     g.sgn = buffer<int8_t>(c, B_SGN, 4);
   }
@@ -929,6 +926,13 @@ uint64_t relabel_dense(stc_ctx* c, const uint32_t** src, const uint32_t** dst, u
 }
 
 }  // namespace
+
+void algorithmic_bytes(stc_ctx* c, const DeviceGraph& g) {
+  k_alg_bytes<<<grid_for(g.m_fwd, 4), kThreads, 0, c->stream>>>(
+      g.asrc, g.nbr, g.m_fwd, g.m_dev, g.off, g.fdeg, (unsigned long long*)counters(c));
+  c->launches++;
+  STC_CUDA(cudaGetLastError());
+}
 
 void build_graph(stc_ctx* c, const uint32_t* d_src, const uint32_t* d_dst, const int8_t* d_sign,
                  uint64_t m, DeviceGraph& g, bool totals) {

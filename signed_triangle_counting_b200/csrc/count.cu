@@ -1317,30 +1317,26 @@ void launch_classes(cudaStream_t st, const Csr& csr, const uint32_t* lists, cons
 // MC/tc_hash_sign_enu.cpp:146-160).
 //
 // The head side finds each vertex's in-arcs by a sort: every HEAD arc i
-// (its index in the CSR) is appended as the key v << 32 | i (a warp adds its
-// keys with one atomic, so their order varies from run to run; the counts
-// are sums and do not depend on it), a radix sort over the vertex bits of
-// the appended keys, their number known on the device only, groups each
-// head's in-arcs, and the runs of equal v are its in-arc ranges.  Head vertices are classed by
-// |N+(v)|, the list they stage: warp (<= 128), block (<= 1024) and large
-// (<= 4095).  A work item is a piece of one head's run that does not cross
-// a multiple of its class's item size (a hub with millions of in-arcs
-// becomes thousands of items, each staging its small N+(v) again), so no
-// warp or CTA is left with one huge run.  Each in-arc is one "arc" of the
-// staged tile with extent
-// [i + 1, end of u's list), its sign s(u, v), strategy HASH: the tail
-// side's stream pass then runs unchanged, with the hash keys carrying
-// s(v, w), the streamed sign bytes s(u, w) and the arc's sign s(u, v).
+// (its index in the CSR) is appended as a key that holds its sign, |A'|, v and
+// i (HeadKey; a CTA adds a tile's keys with one atomic, so their order varies
+// from run to run; the counts are sums and do not depend on it), a radix sort
+// over the vertex bits of the appended keys, their number known on the device
+// only, groups each head's in-arcs, and the runs of equal v are its in-arc
+// ranges.  Head vertices are classed by |N+(v)|, the list they stage: warp
+// (<= 128), block (<= 1024) and large (<= 4095), the lists longer than the
+// warp class's inside the bitmap's window making a fourth class.  A work item
+// is a piece of one head's run that does not cross a multiple of its class's
+// item size (a hub with millions of in-arcs becomes thousands of items, each
+// staging its small N+(v) again), so no warp or CTA is left with one huge
+// run.  In the hash classes each in-arc is one "arc" of the staged tile with
+// extent [i + 1, end of u's list), its sign s(u, v), strategy HASH: the
+// stream pass then probes hash keys that carry s(v, w) with signed heads that
+// carry s(u, w).
 constexpr uint32_t kHeadMaxB = kLargeCap - 1;  // |N+(v)| of a HEAD arc: bucket <= 12
 static_assert(32 - __builtin_clz(kHeadMaxB) == 12 && 32 - __builtin_clz(kHeadMaxB + 1) == 13,
               "HEAD cells (bucket |B| <= 12) are exactly the arcs whose head fits the large class");
 constexpr int kHeadClasses = 4;
-constexpr uint32_t kHeadBits = 3;  // the bitmap class (k_head_bits)
-// Head list buffer: plan words first (start of class c's list, then from
-// kHeadPlanCount its count), the class lists after them, then one byte per
-// vertex: whether it keeps arcs for the tail side.
-constexpr uint32_t kHeadPlanCount = 4;
-constexpr uint32_t kHeadPlanWords = 8;
+constexpr uint32_t kHeadBits = 3;        // the bitmap class (k_head_bits)
 constexpr uint32_t kHeadItemMin = 2048;  // the smallest class item size
 
 // In-arcs per work item of head class c (powers of two).
@@ -1394,159 +1390,235 @@ struct BitsRule {
   }
 };
 
+// A HEAD arc's sort key: the arc index i in the low ibits, then v (vbits),
+// then |A'| in the bits left below the sign in bit 63 (at most 31).  An |A'|
+// that its field cannot hold is stored as all ones and the arc's list end
+// is looked up in `aend` instead.  With the extent in the key, a work item
+// reads its in-arcs with one coalesced load each: gathering list ends and
+// signs by arc index cost two 32-byte sectors and a dependent latency an
+// in-arc.
+struct HeadKey {
+  uint32_t ibits, vbits, amax;
+  static HeadKey of(uint32_t n, uint64_t m) {
+    HeadKey f;
+    f.ibits = std::max<uint32_t>(1, bit_width64(m - 1));
+    f.vbits = std::max<uint32_t>(1, bit_width64(n - 1));
+    f.amax = (1u << std::min<uint32_t>(31, 63 - f.ibits - f.vbits)) - 1;
+    return f;
+  }
+  __device__ __forceinline__ uint64_t pack(uint32_t v, uint64_t i, uint32_t alen, bool neg) const {
+    return ((uint64_t)neg << 63) | ((uint64_t)min(alen, amax) << (ibits + vbits)) |
+           ((uint64_t)v << ibits) | i;
+  }
+  __device__ __forceinline__ uint32_t vertex(uint64_t k) const {
+    return (uint32_t)(k >> ibits) & ((1u << vbits) - 1);
+  }
+  __device__ __forceinline__ uint32_t arc(uint64_t k) const {
+    return (uint32_t)(k & ((1ull << ibits) - 1));
+  }
+  // |A'|, or amax when it did not fit.
+  __device__ __forceinline__ uint32_t alen(uint64_t k) const {
+    return (uint32_t)((k & ~(1ull << 63)) >> (ibits + vbits));
+  }
+};
+
+// The work items (first entries) of the head classes, in two arrays of `cap`
+// words filled from both ends: class 0 from the front of `a`, class 3 from
+// its back, classes 1 and 2 likewise in `b`.  A head has one class, so the
+// two lists of an array never meet, and no counting pass is needed.
+struct HeadLists {
+  uint32_t* a;
+  uint32_t* b;
+  uint32_t cap;
+  __device__ __forceinline__ uint32_t& at(uint32_t c, uint32_t pos) const {
+    uint32_t* p = c == 0 || c == kHeadBits ? a : b;
+    return p[c == 0 || c == 1 ? pos : cap - 1 - pos];
+  }
+};
+
 struct HeadArcs {
-  const uint64_t* __restrict__ keys;  // sorted: v << 32 | arc index
-  const uint32_t* __restrict__ aend;  // per arc: end of its tail's list in the CSR
+  const uint64_t* __restrict__ keys;  // sorted by v (HeadKey)
+  const uint32_t* __restrict__ aend;  // list end of an arc whose |A'| did not fit its key
   const uint32_t* __restrict__ end;   // per head vertex: one past its last in-arc entry
   const uint32_t* __restrict__ asrc;  // per arc: its tail (timing recorder only)
+  HeadKey fmt;
+  HeadLists lists;
   // Work item starting at entry j0 of head class c: its head and its end.
   __device__ __forceinline__ void item(uint32_t j0, uint32_t c, uint32_t& v, uint32_t& j1) const {
-    v = (uint32_t)(keys[j0] >> 32);
+    v = fmt.vertex(keys[j0]);
     j1 = min(end[v], (j0 | (head_item(c) - 1)) + 1);
+  }
+  // A' of the in-arc with this key.
+  __device__ __forceinline__ void extent(uint64_t key, uint32_t& lo, uint32_t& hi) const {
+    const uint32_t i = fmt.arc(key), al = fmt.alen(key);
+    lo = i + 1;
+    hi = al == fmt.amax ? aend[i] : lo + al;  // > lo: a HEAD arc has a non-empty A'
   }
 };
 
 // Appends the keys of the HEAD arcs (count in ctr[C_HEAD_NKEYS]), records
-// the list end of each HEAD arc, and sets need[u] = 1 for each tail u with
-// an arc left to the tail side (the array starts at 0; tails without such
-// arcs are not staged there).  `range` (a sharded count) keeps only tails
-// in [range[0], range[1]).
-// Size bucket of every vertex's out-degree, one byte each: the head keys
-// gather it for every arc's head, from an array a quarter the size of the
-// out-degrees (more of it stays in L2).
-__global__ void k_fdeg_bucket(const uint32_t* __restrict__ fdeg, uint32_t n,
-                              uint8_t* __restrict__ out) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    out[i] = (uint8_t)size_bucket(fdeg[i]);
-}
-
+// the list end of each HEAD arc whose |A'| its key cannot hold, and sets
+// need[u] = 1 for each tail u with an arc left to the tail side (the array
+// starts at 0; tails without such arcs are not staged there).  `range` (a
+// sharded count) keeps only tails in [range[0], range[1]).  With kBytes it
+// also adds up the algorithmic bytes of every arc (arc_bytes), whose inputs
+// it reads anyway: a pass of its own took 0.82 ms at RMAT scale 24.
+// A CTA appends a tile of 1,024 arcs with one atomic; with one per warp and
+// load the 8 M atomics on the one counter took 6.8 ms at RMAT scale 24.
+template <bool kBytes>
 __global__ void __launch_bounds__(256) k_head_keys(Csr g, const uint32_t* __restrict__ asrc,
-                                                   const uint8_t* __restrict__ fbkt, uint64_t m,
+                                                   const uint32_t* __restrict__ fdeg, uint64_t m,
                                                    const unsigned long long* __restrict__ m_dev,
                                                    const uint8_t* __restrict__ gtables,
                                                    const unsigned long long* __restrict__ range,
-                                                   uint64_t* __restrict__ keys,
+                                                   HeadKey fmt, uint64_t* __restrict__ keys,
                                                    uint32_t* __restrict__ aend,
                                                    uint8_t* __restrict__ need,
                                                    unsigned long long* __restrict__ ctr) {
   constexpr int kItems = 4;  // arcs per lane with their gathers in flight together
+  constexpr int kWarps = 8;
   __shared__ uint8_t tab[kTableBytes];
+  __shared__ uint32_t wcnt[2][kWarps];  // alternating tiles
+  __shared__ uint32_t tbase[2];
   if (m_dev) m = min(m, (uint64_t)*m_dev);  // m a capacity, *m_dev the arc count
   for (uint32_t i = threadIdx.x; i < kTableBytes; i += blockDim.x) tab[i] = gtables[i];
   __syncthreads();
   const uint32_t r0 = range ? (uint32_t)range[0] : 0u;
   const uint32_t r1 = range ? (uint32_t)range[1] : 0xFFFFFFFFu;
-  const uint32_t lane = lane_id();
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x * kItems;
-  for (uint64_t base = ((uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) * kItems;
-       base < m; base += stride) {
+  const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+  unsigned long long bytes = 0, probe = 0;
+  uint32_t flip = 0;
+  for (uint64_t tile = (uint64_t)blockIdx.x * (256 * kItems); tile < m;
+       tile += (uint64_t)gridDim.x * (256 * kItems), flip ^= 1) {
+    const uint64_t base = tile + warp * (32 * kItems) + lane;
     uint32_t u[kItems], v[kItems], blen[kItems];
-    uint64_t ub[kItems], ue[kItems];
+    uint32_t ub[kItems], ue[kItems], neg = 0;
 #pragma unroll
     for (int q = 0; q < kItems; q++) {
-      const uint64_t i = base + 32 * q + lane;
+      const uint64_t i = base + 32 * q;
       u[q] = i < m ? asrc[i] : 0u;
       v[q] = i < m ? g.nbr[i] : 0u;
+      neg |= (i < m && g.sgn[i] < 0 ? 1u : 0u) << q;
     }
 #pragma unroll
     for (int q = 0; q < kItems; q++) {
-      const uint64_t i = base + 32 * q + lane;
-      ub[q] = i < m ? g.off[u[q]] : 0;
-      ue[q] = i < m ? g.off[u[q] + 1] : 0;
-      blen[q] = i < m ? fbkt[v[q]] : 0u;
+      const uint64_t i = base + 32 * q;
+      ub[q] = i < m ? (uint32_t)g.off[u[q]] : 0;
+      ue[q] = i < m ? (uint32_t)g.off[u[q] + 1] : 0;
+      blen[q] = i < m ? fdeg[v[q]] : 0u;
     }
+    uint32_t heads = 0, mine = 0, total = 0;  // HEAD flags; keys of the lanes below; of the warp
 #pragma unroll
     for (int q = 0; q < kItems; q++) {
-      const uint64_t i = base + 32 * q + lane;
+      const uint64_t i = base + 32 * q;
       bool head = false;
       if (i < m) {
-        const uint32_t alen = (uint32_t)(ue[q] - i - 1);
+        const uint32_t alen = ue[q] - (uint32_t)i - 1, d = ue[q] - ub[q];
+        if (kBytes) {
+          bytes += 5ull * d + 5ull * blen[q] + 25ull;
+          probe += 5ull * min(alen, blen[q]) + 30ull;
+        }
         if (alen && blen[q] && u[q] >= r0 && u[q] < r1) {
-          head = tab[256 * table_class((uint32_t)(ue[q] - ub[q])) + 16 * size_bucket(alen) +
-                     blen[q]] == STC_STRATEGY_HEAD;
+          head = tab[256 * table_class(d) + 16 * size_bucket(alen) + size_bucket(blen[q])] ==
+                 STC_STRATEGY_HEAD;
           if (!head) need[u[q]] = 1;  // u keeps an arc for the tail side
         }
       }
       const unsigned hb = __ballot_sync(kFull, head);
-      uint32_t at = 0;
-      if (lane == 0 && hb)
-        at = (uint32_t)atomicAdd(ctr + C_HEAD_NKEYS, (unsigned long long)__popc(hb));
-      at = __shfl_sync(kFull, at, 0);
-      if (head) {
-        keys[at + __popc(hb & lanemask_lt())] = ((uint64_t)v[q] << 32) | i;
-        aend[i] = (uint32_t)ue[q];
+      heads |= (uint32_t)head << q;
+      mine += __popc(hb & lanemask_lt());
+      total += __popc(hb);
+    }
+    if (lane == 0) wcnt[flip][warp] = total;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      uint32_t run = 0;
+      for (int w = 0; w < kWarps; w++) {
+        const uint32_t c = wcnt[flip][w];
+        wcnt[flip][w] = run;
+        run += c;
       }
+      tbase[flip] = run ? (uint32_t)atomicAdd(ctr + C_HEAD_NKEYS, (unsigned long long)run) : 0u;
+    }
+    __syncthreads();
+    // The keys of one lane in a row: any order within the tile will do.
+    uint32_t at = tbase[flip] + wcnt[flip][warp] + mine;
+#pragma unroll
+    for (int q = 0; q < kItems; q++) {
+      const uint64_t i = base + 32 * q;
+      if ((heads >> q) & 1u) {
+        const uint32_t alen = ue[q] - (uint32_t)i - 1;
+        keys[at++] = fmt.pack(v[q], i, alen, (neg >> q) & 1u);
+        if (alen >= fmt.amax) aend[i] = ue[q];
+      }
+    }
+  }
+  if (kBytes) {
+    bytes = warp_sum(bytes);
+    probe = warp_sum(probe);
+    if (lane == 0 && bytes) {
+      atomicAdd(ctr + C_ALG_BYTES, bytes);
+      atomicAdd(ctr + C_PROBE_BYTES, probe);
     }
   }
 }
 
 // Work items in the sorted keys: an entry starts one where its head's run
-// starts or where it is a multiple of its class's item size.  Without
-// kFill: counts the items of each class.  With kFill: appends each item's
-// first entry to its class list and records the end of every run.
-template <bool kFill>
-__global__ void __launch_bounds__(256) k_head_runs(const uint64_t* __restrict__ keys,
-                                                   const uint64_t* __restrict__ off,
-                                                   unsigned long long* __restrict__ ctr,
-                                                   uint32_t* __restrict__ hl,
-                                                   uint32_t* __restrict__ end, BitsRule rule) {
+// starts or where it is a multiple of its class's item size.  Appends each
+// item's first entry to its class list (through shared memory, one atomic
+// per class and tile) and records the end of every run.
+constexpr int kItemTile = 2048;
+
+__global__ void __launch_bounds__(256) k_head_items(const uint64_t* __restrict__ keys,
+                                                    const uint64_t* __restrict__ off, HeadKey fmt,
+                                                    BitsRule rule, HeadLists lists,
+                                                    uint32_t* __restrict__ end,
+                                                    unsigned long long* __restrict__ ctr) {
+  constexpr int kPer = kItemTile / 256;
+  __shared__ uint32_t found[kItemTile];  // first entries, by class: cnt[c] from start[c]
+  __shared__ uint32_t cnt[kHeadClasses], start[kHeadClasses], gbase[kHeadClasses];
   const uint64_t m = ctr[C_HEAD_NKEYS];
-  const uint32_t lane = lane_id();
-  uint32_t cnt[kHeadClasses] = {0, 0, 0, 0};
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < m;
-       base += stride) {
-    const uint64_t j = base + lane;
-    uint32_t c = kHeadClasses;  // not an item start
-    if (j < m) {
-      const uint64_t kv = keys[j] >> 32;
-      const uint32_t v = (uint32_t)kv;
-      const bool run = j == 0 || (keys[j - 1] >> 32) != kv;
+  for (uint64_t tile = (uint64_t)blockIdx.x * kItemTile; tile < m;
+       tile += (uint64_t)gridDim.x * kItemTile) {
+    if (threadIdx.x < kHeadClasses) cnt[threadIdx.x] = 0;
+    __syncthreads();
+    uint32_t cls = 0xFFFFFFFFu;  // four bits an entry; 15: starts no item
+    uint32_t pos[kPer];
+#pragma unroll
+    for (int q = 0; q < kPer; q++) {
+      const uint64_t j = tile + q * 256 + threadIdx.x;
+      pos[q] = 0;
+      if (j >= m) continue;
+      const uint32_t v = fmt.vertex(keys[j]);
+      const bool run = j == 0 || fmt.vertex(keys[j - 1]) != v;
+      if (j + 1 == m || fmt.vertex(keys[j + 1]) != v) end[v] = (uint32_t)(j + 1);
       if (run || (j & (kHeadItemMin - 1)) == 0) {
         const uint32_t hc = rule.head_class_of(v, (uint32_t)(off[v + 1] - off[v]));
-        if (run || (j & (head_item(hc) - 1)) == 0) c = hc;
-      }
-      if (kFill && (j + 1 == m || (keys[j + 1] >> 32) != kv)) end[v] = (uint32_t)(j + 1);
-    }
-    if (!kFill) {
-#pragma unroll
-      for (int k = 0; k < kHeadClasses; k++) cnt[k] += c == (uint32_t)k;
-    } else {
-      // Item starts are rare (about one entry in fifty): one ballot per
-      // class, and an atomic only where the warp holds some.
-#pragma unroll
-      for (uint32_t k = 0; k < (uint32_t)kHeadClasses; k++) {
-        const unsigned peers = __ballot_sync(kFull, c == k);
-        if (peers == 0) continue;
-        const uint32_t leader = __ffs(peers) - 1;
-        uint32_t pos = 0;
-        if (lane == leader)
-          pos = (uint32_t)atomicAdd(ctr + C_HEAD_CURSOR + k, (unsigned long long)__popc(peers));
-        pos = __shfl_sync(kFull, pos, leader) + __popc(peers & lanemask_lt());
-        if (c == k) hl[kHeadPlanWords + hl[k] + pos] = (uint32_t)j;
+        if (run || (j & (head_item(hc) - 1)) == 0) {
+          cls ^= (15u ^ hc) << (4 * q);
+          pos[q] = atomicAdd(&cnt[hc], 1u);
+        }
       }
     }
-  }
-  if (!kFill) {
-#pragma unroll
-    for (int k = 0; k < kHeadClasses; k++) {
-      const uint32_t s = __reduce_add_sync(kFull, cnt[k]);
-      if (lane == 0 && s) atomicAdd(ctr + C_HEAD_COUNT + k, (unsigned long long)s);
+    __syncthreads();
+    if (threadIdx.x < kHeadClasses) {
+      uint32_t s = 0;
+      for (uint32_t c = 0; c < threadIdx.x; c++) s += cnt[c];
+      start[threadIdx.x] = s;
+      const uint32_t k = cnt[threadIdx.x];
+      gbase[threadIdx.x] =
+          k ? (uint32_t)atomicAdd(ctr + C_HEAD_COUNT + threadIdx.x, (unsigned long long)k) : 0u;
     }
-  }
-}
-
-// Class list starts from the counts; clears the fill cursors and queues.
-__global__ void k_head_plan(unsigned long long* __restrict__ ctr, uint32_t* __restrict__ hl) {
-  if (threadIdx.x != 0) return;
-  uint32_t start = 0;
-  for (int c = 0; c < kHeadClasses; c++) {
-    const uint32_t n = (uint32_t)ctr[C_HEAD_COUNT + c];
-    hl[c] = start;
-    hl[kHeadPlanCount + c] = n;
-    start += n;
-    ctr[C_HEAD_CURSOR + c] = 0;
-    ctr[C_HEAD_QUEUE + c] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kPer; q++) {
+      const uint32_t c = (cls >> (4 * q)) & 15u;
+      if (c < kHeadClasses) found[start[c] + pos[q]] = (uint32_t)(tile + q * 256 + threadIdx.x);
+    }
+    __syncthreads();
+    for (uint32_t c = 0; c < kHeadClasses; c++)
+      for (uint32_t p = threadIdx.x; p < cnt[c]; p += 256) lists.at(c, gbase[c] + p) = found[start[c] + p];
+    __syncthreads();
   }
 }
 
@@ -1573,10 +1645,9 @@ __device__ __forceinline__ void stage_in_arcs(const Csr& g, const HeadArcs& h, u
                                               uint32_t tn, uint32_t t, const StageMem& m,
                                               Sync sync) {
   for (uint32_t k = t; k < tn; k += TS) {
-    const uint32_t i = (uint32_t)h.keys[j0 + k];
-    m.lo[k] = i + 1;
-    m.hi[k] = h.aend[i];  // > i + 1: a HEAD arc has a non-empty A'
-    m.s[k] = g.sgn[i];
+    const uint64_t key = h.keys[j0 + k];
+    h.extent(key, m.lo[k], m.hi[k]);
+    m.s[k] = (key >> 63) ? (int8_t)-1 : (int8_t)1;
     m.st[k] = STC_STRATEGY_HASH;
   }
   sync();
@@ -1610,7 +1681,7 @@ __device__ __forceinline__ void timed_head_pass(const Csr& g, const HeadArcs& h,
 // queue, N+(v) and up to kWarpCap in-arcs at a time staged in the warp's
 // slice of shared memory.
 template <class Sink, bool kTime, int U>
-__global__ void __launch_bounds__(256) k_head_warp(Csr g, HeadArcs h, const uint32_t* __restrict__ hl,
+__global__ void __launch_bounds__(256) k_head_warp(Csr g, HeadArcs h,
                                                    unsigned long long* __restrict__ ctr, Sink sink,
                                                    ArcTimes at, uint32_t hf) {
   constexpr bool kVC = Sink::kPerVertex;
@@ -1618,8 +1689,7 @@ __global__ void __launch_bounds__(256) k_head_warp(Csr g, HeadArcs h, const uint
   __shared__ __align__(16) unsigned char smem[kWarps * kWarpStageBytes];
   const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
   const StageMem m = StageMem::carve(smem + w * kWarpStageBytes, kWarpCap, kWarpBuckets);
-  const uint32_t* list = hl + kHeadPlanWords + hl[0];
-  const uint32_t cnt = hl[kHeadPlanCount + 0];
+  const uint32_t cnt = (uint32_t)ctr[C_HEAD_COUNT + 0];
   TypeCounts tc;
   // Per-key counts (a sink that reports per graph): a warp's items come in
   // increasing order of their heads, so the counts of one key are added up
@@ -1640,7 +1710,7 @@ __global__ void __launch_bounds__(256) k_head_warp(Csr g, HeadArcs h, const uint
     item = __shfl_sync(kFull, item, 0);
     if (item >= cnt) break;
     uint32_t v, j1;
-    const uint32_t j00 = list[item];
+    const uint32_t j00 = h.lists.at(0, item);
     h.item(j00, 0, v, j1);
     const uint64_t vb = g.off[v];
     const uint32_t d = (uint32_t)(g.off[v + 1] - vb);
@@ -1685,7 +1755,6 @@ __global__ void __launch_bounds__(256) k_head_warp(Csr g, HeadArcs h, const uint
 // in-arcs at a time staged in dynamic shared memory.
 template <int THREADS, class Sink, bool kTime, int U>
 __global__ void __launch_bounds__(THREADS) k_head_block(Csr g, HeadArcs h,
-                                                        const uint32_t* __restrict__ hl,
                                                         uint32_t hclass, uint32_t cap, uint32_t nb,
                                                         uint32_t hf,
                                                         unsigned long long* __restrict__ ctr,
@@ -1697,8 +1766,7 @@ __global__ void __launch_bounds__(THREADS) k_head_block(Csr g, HeadArcs h,
   __shared__ uint32_t s_item;
   const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
   const StageMem m = StageMem::carve(smem, cap, nb);
-  const uint32_t* list = hl + kHeadPlanWords + hl[hclass];
-  const uint32_t cnt = hl[kHeadPlanCount + hclass];
+  const uint32_t cnt = (uint32_t)ctr[C_HEAD_COUNT + hclass];
   unsigned long long* queue = ctr + C_HEAD_QUEUE + hclass;
   uint32_t* next = scan_tmp + kWarps + 1;  // the stream's claim counter
   TypeCounts tc;
@@ -1717,7 +1785,7 @@ __global__ void __launch_bounds__(THREADS) k_head_block(Csr g, HeadArcs h,
     const uint32_t item = s_item;
     if (item >= cnt) break;
     uint32_t v, j1;
-    const uint32_t j00 = list[item];
+    const uint32_t j00 = h.lists.at(hclass, item);
     h.item(j00, hclass, v, j1);
     const uint64_t vb = g.off[v];
     const uint32_t d = (uint32_t)(g.off[v + 1] - vb);
@@ -1794,22 +1862,31 @@ __global__ void __launch_bounds__(256) k_sign_bits(const int8_t* __restrict__ sg
 // tiles.  The eight hits of a chunk are classified together: three
 // population counts of the hit masks against the chunk's sign byte.
 //
-// RMAT scale 24 (97% of the 41.8 G probes): 42.4 ms, against 78.8 ms of hash
-// probes for the same heads; scale 22: 3.85 G warp instructions against
-// 9.98 G.  What bounds it now is waiting, at the two barriers of a work item
-// and for the streamed chunks (issue slots 38% used, DRAM 2.1 TB/s).
+// A CTA waits as little as its two barriers an item allow: the next item's
+// four dependent loads run under this item's stream, the old list's bits go
+// off in the step that sets the new ones, a claim's keys are loaded while the
+// claim before is streamed, and small items are claimed in small pieces.
+//
+// RMAT scale 24 (97% of the 41.8 G probes): 37.6 ms, against 78.8 ms of hash
+// probes for the same heads (42.4 ms before the steps of the last
+// paragraph); scale 22: 4.2 G warp instructions against 10.0 G, issue slots
+// 51% used, DRAM at 1.4 TB/s.
 template <int THREADS, class Sink>
 __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_head_bits(
-    Csr g, HeadArcs h, const uint8_t* __restrict__ sbits, const uint32_t* __restrict__ hl,
-    unsigned long long* __restrict__ ctr, Sink sink) {
+    Csr g, HeadArcs h, const uint8_t* __restrict__ sbits, unsigned long long* __restrict__ ctr,
+    Sink sink) {
   constexpr bool kVC = Sink::kPerVertex;
+  constexpr uint32_t kWarps = THREADS / 32;
   constexpr int U = 2;  // chunks in flight per lane
   constexpr uint32_t kDrainRounds = 255 / (8 * U);  // 8-bit fields, 8 adds a chunk at most
   extern __shared__ __align__(16) uint32_t bm[];  // kBitsWords
-  __shared__ uint32_t s_item, s_next;
+  struct Item {
+    uint32_t v, j0, arcs, vb, d;  // arcs 0: no more items
+  };
+  __shared__ Item s_item[2];
+  __shared__ uint32_t s_next;
   const uint32_t lane = lane_id(), le = lanemask_lt() | (1u << lane);
-  const uint32_t* list = hl + kHeadPlanWords + hl[kHeadBits];
-  const uint32_t cnt = hl[kHeadPlanCount + kHeadBits];
+  const uint32_t cnt = (uint32_t)ctr[C_HEAD_COUNT + kHeadBits];
   TypeCounts tc;
   uint32_t cur = 0xFFFFFFFFu;  // per-key counts as in k_head_block
   auto flush = [&]() {
@@ -1818,49 +1895,74 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_head_bits(
       tc = TypeCounts{};
     }
   };
-  for (uint32_t i = threadIdx.x; i < kBitsWords; i += THREADS) bm[i] = 0;
-  while (true) {
-    if (threadIdx.x == 0) {
-      s_item = (uint32_t)atomicAdd(ctr + C_HEAD_QUEUE + kHeadBits, 1ull);
-      s_next = 0;
+  // Thread 0: the next work item, by four dependent loads.
+  auto fetch = [&](Item& it) {
+    const uint32_t item = (uint32_t)atomicAdd(ctr + C_HEAD_QUEUE + kHeadBits, 1ull);
+    it.arcs = 0;
+    if (item >= cnt) return;
+    uint32_t j1;
+    it.j0 = h.lists.at(kHeadBits, item);
+    h.item(it.j0, kHeadBits, it.v, j1);
+    it.arcs = j1 - it.j0;
+    it.vb = (uint32_t)g.off[it.v];
+    it.d = (uint32_t)g.off[it.v + 1] - it.vb;
+  };
+  // Switches the bits of the list [vb, vb + d) on, or off again.
+  auto toggle = [&](uint32_t vb, uint32_t d) {
+    for (uint32_t i = threadIdx.x; i < d; i += THREADS) {
+      const uint32_t x = g.nbr[vb + i];
+      const uint32_t neg = g.sgn[vb + i] < 0;
+      atomicXor(&bm[(x >> 4) & (kBitsWords - 1)], 1u << ((x & 31u) ^ (neg << 4)));
     }
-    __syncthreads();  // the last item's bits are cleared
-    const uint32_t item = s_item;
-    if (item >= cnt) break;
-    uint32_t v, j1;
-    const uint32_t j0 = list[item];
-    h.item(j0, kHeadBits, v, j1);
-    const uint64_t vb = g.off[v];
-    const uint32_t d = (uint32_t)(g.off[v + 1] - vb);
+  };
+  for (uint32_t i = threadIdx.x; i < kBitsWords; i += THREADS) bm[i] = 0;
+  if (threadIdx.x == 0) fetch(s_item[0]);
+  __syncthreads();
+  uint32_t ovb = 0, od = 0, p = 0;  // the list whose bits are on
+  while (true) {
+    const Item it = s_item[p];
+    if (it.arcs == 0) break;
     if (kVC) {
-      const uint32_t key = sink.key(v);  // uniform over the CTA
+      const uint32_t key = sink.key(it.v);  // uniform over the CTA
       if (key != cur) {
         flush();
         cur = key;
       }
     }
-    for (uint32_t i = threadIdx.x; i < d; i += THREADS) {
-      const uint32_t x = g.nbr[vb + i];
-      const uint32_t neg = g.sgn[vb + i] < 0;
-      atomicOr(&bm[(x >> 4) & (kBitsWords - 1)], 1u << ((x & 31u) ^ (neg << 4)));
-    }
+    // Exclusive ors commute, so the old list's bits go off and the new one's
+    // on in one step, whatever the two share.
+    toggle(ovb, od);
+    toggle(it.vb, it.d);
+    ovb = it.vb;
+    od = it.d;
+    if (threadIdx.x == 0) s_next = 0;
     __syncthreads();
-    const uint32_t arcs = j1 - j0;
+    // The next item's loads run under this item's stream.
+    if (threadIdx.x == 0) fetch(s_item[p ^ 1]);
+    // In-arcs per claim: up to a lane each, but small items are shared out
+    // over all warps, twice over.
+    const uint32_t claim = min(32u, max(4u, (it.arcs + 2 * kWarps - 1) / (2 * kWarps)));
     PackedCounts8 p8;
     uint32_t rounds = 0;
-    while (true) {
+    auto take = [&](uint64_t& key) {  // claims the next in-arcs and loads the lane's key
       uint32_t b = 0;
-      if (lane == 0) b = atomicAdd(&s_next, 32u);
+      if (lane == 0) b = atomicAdd(&s_next, claim);
       b = __shfl_sync(kFull, b, 0);
-      if (b >= arcs) break;
+      if (lane < claim && b + lane < it.arcs) key = h.keys[it.j0 + b + lane];
+      return b;
+    };
+    uint64_t nkey = 0;
+    uint32_t nb = take(nkey);
+    while (nb < it.arcs) {
+      const uint32_t b = nb;
+      const uint64_t key = nkey;
+      nb = take(nkey);  // in flight while this claim is streamed
       // This lane's in-arc: A' extent [lo, hi), chunks, 8 * (arc negative).
-      uint32_t lo = 0, hi = 0, c = 0, sh = 0;
-      if (b + lane < arcs) {
-        const uint32_t i = (uint32_t)h.keys[j0 + b + lane];
-        lo = i + 1;
-        hi = h.aend[i];  // > lo: a HEAD arc has a non-empty A'
+      uint32_t lo = 0, hi = 0, c = 0;
+      const uint32_t sh = (uint32_t)(key >> 63) << 3;
+      if (lane < claim && b + lane < it.arcs) {
+        h.extent(key, lo, hi);
         c = ((hi + 7) >> 3) - (lo >> 3);
-        sh = ((sbits[i >> 3] >> (7u - (i & 7u))) & 1u) << 3;
       }
       const uint32_t inc = warp_inclusive_scan(c);
       const uint32_t start = c ? inc - c : 0xFFFFFFFFu;
@@ -1916,9 +2018,8 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_head_bits(
       }
     }
     p8.drain(tc);
+    p ^= 1;
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < d; i += THREADS)
-      bm[(g.nbr[vb + i] >> 4) & (kBitsWords - 1)] = 0;
   }
   flush();
   if (!kVC) flush_counts<THREADS>(tc, ctr);
@@ -1930,7 +2031,7 @@ struct HeadBufs {
   uint64_t* alt = nullptr;
   uint32_t* aend = nullptr;
   uint32_t* runs = nullptr;  // end of each head's run (n)
-  uint32_t* hl = nullptr;    // plan words, class lists of work items
+  HeadLists lists{};         // the classes' work items
   uint8_t* need = nullptr;   // per tail: it keeps arcs for the tail side
   uint32_t* sort_counts = nullptr;
   uint8_t* sbits = nullptr;  // sign bits of the arcs
@@ -1942,11 +2043,13 @@ HeadBufs head_buffers(stc_ctx* c, const DeviceGraph& g) {
   b.alt = buffer<uint64_t>(c, B_KEYS_B, g.m_fwd);
   b.aend = buffer<uint32_t>(c, B_HEAD_END, g.m_fwd);
   b.runs = buffer<uint32_t>(c, B_HEAD_RUNS, g.n);
-  // Items: at most one per run (head) plus one per multiple of the
-  // smallest item size.
-  const size_t items = (size_t)g.n + g.m_fwd / kHeadItemMin + 1;
-  b.hl = buffer<uint32_t>(c, B_HEAD_LIST, kHeadPlanWords + items + (g.n + 3) / 4);
-  b.need = reinterpret_cast<uint8_t*>(b.hl + kHeadPlanWords + items);
+  // Items: at most one per run (a head with an in-arc and a list) plus one
+  // per multiple of the smallest item size.
+  const size_t items = (size_t)std::min<uint64_t>(g.n, g.m_fwd) + g.m_fwd / kHeadItemMin + 1;
+  b.lists.a = buffer<uint32_t>(c, B_HEAD_LIST, 2 * items + (g.n + 3) / 4);
+  b.lists.b = b.lists.a + items;
+  b.lists.cap = (uint32_t)items;
+  b.need = reinterpret_cast<uint8_t*>(b.lists.b + items);
   b.sort_counts = buffer<uint32_t>(c, B_SORT_COUNTS, (size_t)kRadix * kMaxSortGrid);
   b.sbits = buffer<uint8_t>(c, B_SBITS, (g.m_fwd + 7) / 8);
   return b;
@@ -1987,19 +2090,20 @@ void prepare_head(const Tuning& tu) {
 // follow the tuning of the tail side's same classes.
 inline void enqueue_head_keys(cudaStream_t st, const Csr& csr, const uint32_t* asrc,
                               const uint32_t* fdeg, uint64_t m,
-                              const unsigned long long* m_dev, const HeadBufs& b,
+                              const unsigned long long* m_dev, bool bytes, const HeadBufs& b,
                               const uint8_t* d_tables,
                               const unsigned long long* range, unsigned long long* ctr,
                               int& launches) {
-  STC_CUDA(cudaMemsetAsync(ctr + C_HEAD_COUNT, 0, 3 * kHeadClasses * sizeof(unsigned long long), st));
-  STC_CUDA(cudaMemsetAsync(ctr + C_HEAD_NKEYS, 0, sizeof(unsigned long long), st));
+  STC_CUDA(cudaMemsetAsync(ctr + C_HEAD_NKEYS, 0,
+                           (C_HEAD_QUEUE + kHeadClasses - C_HEAD_NKEYS) * sizeof(unsigned long long),
+                           st));
   STC_CUDA(cudaMemsetAsync(b.need, 0, csr.n, st));
-  const uint32_t grid = (uint32_t)std::min<uint64_t>((m + 1023) / 1024, kSMs * 8);
-  uint8_t* fbkt = reinterpret_cast<uint8_t*>(b.runs);  // free until the runs are found
-  k_fdeg_bucket<<<kSMs * 8, 256, 0, st>>>(fdeg, csr.n, fbkt);
-  k_head_keys<<<std::max(1u, grid), 256, 0, st>>>(csr, asrc, fbkt, m, m_dev, d_tables, range,
-                                                  b.keys, b.aend, b.need, ctr);
-  launches += 2;
+  const uint32_t grid = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((m + 1023) / 1024, kSMs * 8));
+  const HeadKey fmt = HeadKey::of(csr.n, m);
+  auto kernel = bytes ? k_head_keys<true> : k_head_keys<false>;
+  kernel<<<grid, 256, 0, st>>>(csr, asrc, fdeg, m, m_dev, d_tables, range, fmt, b.keys, b.aend,
+                               b.need, ctr);
+  launches += 1;
 }
 
 template <class Sink, bool kTime>
@@ -2009,24 +2113,24 @@ void enqueue_head(cudaStream_t st, const Csr& csr, const uint32_t* asrc, uint64_
                   const ArcTimes& at, const Tuning& tu, int& launches,
                   uint32_t class_mask = 0x3F) {
   const uint32_t n = csr.n;
-  const uint32_t vbits = std::max<uint32_t>(1, bit_width64(n - 1));
-  int sort_launches = 0;
-  const uint64_t* sorted = radix_sort(b.keys, b.alt, m, 32, 32 + (int)vbits, b.sort_counts, st,
-                                      &sort_launches, ctr + C_HEAD_NKEYS);
+  const HeadKey fmt = HeadKey::of(n, m);
+  const uint64_t* sorted = radix_sort(b.keys, b.alt, m, (int)fmt.ibits,
+                                      (int)(fmt.ibits + fmt.vbits), b.sort_counts, st, &launches,
+                                      ctr + C_HEAD_NKEYS);
   uint32_t* end = b.runs;
   // The recorder times single arcs against a staged hash: no bitmap there.
   const BitsRule rule{kTime ? 0u : kBitsWindow, n, gbase, G};
-  k_head_runs<false><<<kSMs * 4, 256, 0, st>>>(sorted, csr.off, ctr, b.hl, end, rule);
-  k_head_plan<<<1, 32, 0, st>>>(ctr, b.hl);
-  k_head_runs<true><<<kSMs * 4, 256, 0, st>>>(sorted, csr.off, ctr, b.hl, end, rule);
-  const HeadArcs h{sorted, b.aend, end, asrc};
-  launches += 3 + sort_launches;
+  const uint32_t tiles = (uint32_t)std::max<uint64_t>(1, (m + kItemTile - 1) / kItemTile);
+  k_head_items<<<std::min<uint32_t>(tiles, kSMs * 8), 256, 0, st>>>(sorted, csr.off, fmt, rule,
+                                                                    b.lists, end, ctr);
+  const HeadArcs h{sorted, b.aend, end, asrc, fmt, b.lists};
+  launches += 1;
   if constexpr (!kTime) {
     if (class_mask & 4u) {
       k_sign_bits<<<kSMs * 8, 256, 0, st>>>(csr.sgn, m, m_dev, b.sbits);
       k_head_bits<kBitsThreads, Sink>
           <<<kSMs * (1024 / kBitsThreads), kBitsThreads, kBitsWords * sizeof(uint32_t), st>>>(
-              csr, h, b.sbits, b.hl, ctr, sink);
+              csr, h, b.sbits, ctr, sink);
       launches += 2;
     }
   }
@@ -2039,7 +2143,7 @@ void enqueue_head(cudaStream_t st, const Csr& csr, const uint32_t* asrc, uint64_
     constexpr int kU = decltype(U)::value;
     if constexpr (!kTime || kU == kStreamUnroll)
       if (class_mask & 2u)
-        k_head_warp<Sink, kTime, kU><<<kSMs * 4, 256, 0, st>>>(csr, h, b.hl, ctr, sink, at,
+        k_head_warp<Sink, kTime, kU><<<kSMs * 4, 256, 0, st>>>(csr, h, ctr, sink, at,
                                                                tu.hash_factor[0]);
   });
   if (low && (class_mask & 4u)) {
@@ -2053,7 +2157,7 @@ void enqueue_head(cudaStream_t st, const Csr& csr, const uint32_t* asrc, uint64_
         if constexpr (!kTime || (kT == 256 && kU == kStreamUnroll)) {
           const uint32_t per_sm = smem <= 110 * 1024 ? 2 : 1;
           k_head_block<kT, Sink, kTime, kU><<<kSMs * per_sm, kT, smem, st>>>(
-              csr, h, b.hl, 1, cap, nb, hf, ctr, sink, at);
+              csr, h, 1, cap, nb, hf, ctr, sink, at);
         }
       });
     });
@@ -2066,7 +2170,7 @@ void enqueue_head(cudaStream_t st, const Csr& csr, const uint32_t* asrc, uint64_
     with_unroll(kTime ? kStreamUnroll : tu.unroll[2], [&](auto U) {
       constexpr int kU = decltype(U)::value;
       if constexpr (!kTime || kU == kStreamUnroll)
-        k_head_block<512, Sink, kTime, kU><<<kSMs, 512, smem, st>>>(csr, h, b.hl, 2, cap, nb, hf,
+        k_head_block<512, Sink, kTime, kU><<<kSMs, 512, smem, st>>>(csr, h, 2, cap, nb, hf,
                                                                      ctr, sink, at);
     });
   }
@@ -2155,6 +2259,7 @@ struct HeadPlan {
   const uint32_t* asrc = nullptr;
   const uint32_t* fdeg = nullptr;
   uint64_t m = 0;
+  bool bytes = false;  // the key pass adds up the arcs' algorithmic bytes
   const unsigned long long* m_dev = nullptr;  // arc count on the device when m is a capacity
   const uint64_t* gbase = nullptr;  // G + 1 rank boundaries of a batch
   uint32_t G = 0;
@@ -2169,8 +2274,8 @@ void enqueue_persistent(cudaStream_t st, const Csr& csr, const ClassBounds& cb, 
   const ArcTimes none{nullptr, nullptr};
   const uint8_t* need = nullptr;
   if (hp.bufs) {
-    enqueue_head_keys(st, csr, hp.asrc, hp.fdeg, hp.m, hp.m_dev, *hp.bufs, d_tables, nullptr, ctr,
-                      launches);
+    enqueue_head_keys(st, csr, hp.asrc, hp.fdeg, hp.m, hp.m_dev, hp.bytes, *hp.bufs, d_tables,
+                      nullptr, ctr, launches);
     need = hp.bufs->need;
   }
   STC_CUDA(cudaMemsetAsync(ctr + C_WORK, 0, 8 * sizeof(uint64_t), st));
@@ -2227,7 +2332,7 @@ void count_persistent(stc_ctx* c, const Csr& csr, const ClassBounds& cb, uint32_
   PersistentKey key{};
   const HeadBufs hb = hp.bufs ? *hp.bufs : HeadBufs{};
   const void* ptrs[19] = {csr.off, csr.nbr, csr.sgn, csr.verts, lists, plan, ctr, d_tables, s0,
-                          hp.asrc, hb.keys, hb.alt, hb.aend, hb.runs, hb.hl, hp.fdeg, csr.nkey, hb.sbits, hp.gbase};
+                          hp.asrc, hb.keys, hb.alt, hb.aend, hb.runs, hb.lists.a, hp.fdeg, csr.nkey, hb.sbits, hp.gbase};
   memcpy(key.p, ptrs, sizeof(ptrs));
   key.v[0] = csr.n;
   key.v[1] = cb.tiny_max;
@@ -2238,7 +2343,7 @@ void count_persistent(stc_ctx* c, const Csr& csr, const ClassBounds& cb, uint32_
              ((uint64_t)hp.tuning.block_threads << 48) ^ ((uint64_t)hp.tuning.unroll[0] << 56) ^
              ((uint64_t)hp.tuning.unroll[1] << 58) ^ ((uint64_t)hp.tuning.unroll[2] << 60) ^
              ((uint64_t)hp.tuning.hash_factor[0] << 40) ^ ((uint64_t)hp.tuning.hash_factor[1] << 42) ^
-             ((uint64_t)hp.tuning.hash_factor[2] << 44);
+             ((uint64_t)hp.tuning.hash_factor[2] << 44) ^ ((uint64_t)hp.bytes << 62);
   static_assert(sizeof(PersistentKey) <= sizeof(c->graph_key), "graph key size");
   if (c->graph_exec && memcmp(c->graph_key, &key, sizeof(key)) == 0) {
     STC_CUDA(cudaGraphLaunch(c->graph_exec, st));
@@ -2485,6 +2590,7 @@ void count_triangles(stc_ctx* c, const DeviceGraph& gin, const CountConfig& cfg)
                     g.nkey != nullptr && g.n >= 2;
   HeadBufs hb;
   if (head) hb = head_buffers(c, g);
+  else if (!g.bytes_done) algorithmic_bytes(c, g);
   const bool timed = cfg.arc_cycles != nullptr;
   const ArcTimes at{(unsigned long long*)cfg.arc_cycles, (unsigned long long*)cfg.arc_counts};
   const unsigned long long* range = nullptr;
@@ -2511,6 +2617,7 @@ void count_triangles(stc_ctx* c, const DeviceGraph& gin, const CountConfig& cfg)
       hp.asrc = g.asrc;
       hp.fdeg = g.fdeg;
       hp.m = g.m_fwd;
+      hp.bytes = !g.bytes_done;
       hp.m_dev = g.m_dev;
       hp.gbase = g.G ? g.gbase : nullptr;
       hp.G = g.G;
@@ -2531,8 +2638,8 @@ void count_triangles(stc_ctx* c, const DeviceGraph& gin, const CountConfig& cfg)
   }
   const uint8_t* need = nullptr;
   if (head) {
-    enqueue_head_keys(st, csr, g.asrc, g.fdeg, g.m_fwd, g.m_dev, hb, d_table, range, ctr,
-                      c->launches);
+    enqueue_head_keys(st, csr, g.asrc, g.fdeg, g.m_fwd, g.m_dev, !g.bytes_done, hb, d_table, range,
+                      ctr, c->launches);
     need = hb.need;
   }
   k_classify_count<<<kSMs * 4, 256, 0, st>>>(g.off, g.n, cb, ctr, range, need);

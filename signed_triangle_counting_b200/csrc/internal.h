@@ -44,9 +44,9 @@ enum BufId {
   B_TEXT,                         // text input of the GPU parser (padded to 16 bytes)
   B_SPLIT_NBR,                    // sign-split copy of the arc heads (m + 4)
   B_SPLIT_POS,                    // positive arcs per vertex (n)
-  B_HEAD_END,                     // head-side pass: end of each arc's tail list (m)
-  B_HEAD_RUNS,                    // head-side pass: in-arc range per head vertex (2 n)
-  B_HEAD_LIST,                    // head-side pass: head vertices by class, plan, flags
+  B_HEAD_END,                     // head-side pass: list ends of arcs with a long A' (m)
+  B_HEAD_RUNS,                    // head-side pass: end of each head's in-arc run (n)
+  B_HEAD_LIST,                    // head-side pass: work items by class, flags per tail
   B_NKEY,                         // arcs: head << 1 | negative (m + 8)
   B_SBITS,                        // arcs: sign bits, one byte per 8 arcs (the head bitmap's stream)
   B_RELABEL,                      // ids >= 2^31 - 1: the edges relabelled to dense ids (2 m)
@@ -73,14 +73,13 @@ enum CounterSlot {
   C_SHARD_HI = 19,
   C_QUEUE_WARP = 20,           // warp-granular work queue of the persistent engine
   C_PROBE_BYTES = 30,          // probe-model bytes of the CSR
-  C_HEAD_NKEYS = 31,           // head-side pass: keys (HEAD arcs) appended
   C_BATCH_N = 32,              // capped batch build: vertices of the union
   C_BATCH_MU = 33,             // capped batch build: unique edges (= arcs)
   C_OVERFLOW = 34,             // capped batch build: a capacity was exceeded (results void)
-  C_HEAD_COUNT = 36,           // head-side pass: work items per class (4 slots),
-  C_HEAD_CURSOR = 40,          // their list fill cursors (4 slots)
-  C_HEAD_QUEUE = 44,           // and the classes' work queues (4 slots)
-  C_SLOTS = 48
+  C_HEAD_NKEYS = 35,           // head-side pass: keys (HEAD arcs) appended,
+  C_HEAD_COUNT = 36,           // work items per class (4 slots)
+  C_HEAD_QUEUE = 40,           // and the classes' work queues (4 slots)
+  C_SLOTS = 44
 };
 
 // Values of the device error word: 1 = malformed forward CSR,
@@ -231,6 +230,7 @@ struct DeviceGraph {
   uint32_t* fdeg = nullptr;   // out-degree by rank
   uint32_t* asrc = nullptr;   // arcs: tail vertex (rank)
   uint32_t* nkey = nullptr;   // arcs: head << 1 | negative, padded by 8 (the head side's stream)
+  bool bytes_done = false;    // C_ALG_BYTES / C_PROBE_BYTES hold the arcs' algorithmic bytes
   // A capped batch build (BatchCaps) leaves n and m_fwd as capacities: the
   // arc count is then on the device (m_dev), vertices past the union's last
   // rank have no arcs.
@@ -284,6 +284,9 @@ void build_graph_batch_capped(stc_ctx* c, const uint32_t* d_src, const uint32_t*
 // count, the data line count and n.
 uint64_t parse_text_device(stc_ctx* c, const char* d_text, uint64_t size, uint32_t** src,
                            uint32_t** dst, int8_t** sign, uint64_t* lines_out, uint32_t* n_out);
+// Adds the arcs' algorithmic bytes to C_ALG_BYTES / C_PROBE_BYTES, for a count
+// without the head-side pass (whose key pass adds them up otherwise).
+void algorithmic_bytes(stc_ctx* c, const DeviceGraph& g);
 // Forward CSR in the reference's id-space layout, copied to host arrays.
 void export_forward_csr(stc_ctx* c, const DeviceGraph& g, stc_forward_csr* out);
 
