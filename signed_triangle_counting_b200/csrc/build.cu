@@ -294,6 +294,9 @@ __global__ void k_export_keys(const uint64_t* __restrict__ ukeys, uint64_t mu, u
   }
 }
 
+// Where a sort reports a device-side wait that expired.
+unsigned long long* sort_error(stc_ctx* c) { return (unsigned long long*)counters(c) + C_ERROR; }
+
 void read_counters(stc_ctx* c, int first, int count) {
   STC_CUDA(cudaMemcpyAsync(c->h_pinned + first, counters(c) + first, count * sizeof(uint64_t),
                            cudaMemcpyDeviceToHost, c->stream));
@@ -302,9 +305,9 @@ void read_counters(stc_ctx* c, int first, int count) {
 
 // Rank-space CSR from unique keys: arc keys, sort, offsets, fill.
 void finish_csr_from_arc_keys(stc_ctx* c, DeviceGraph& g, uint64_t* akeys, uint64_t* alt) {
-  uint32_t* sort_counts = buffer<uint32_t>(c, B_SORT_COUNTS, (size_t)kRadix * kMaxSortGrid);
+  uint32_t* sort_ws = buffer<uint32_t>(c, B_SORT_WS, sort_workspace_words(g.m_fwd));
   uint64_t* sums = buffer<uint64_t>(c, B_SCAN_SUMS, kMaxSortGrid + 1);
-  uint64_t* sorted = radix_sort(akeys, alt, g.m_fwd, 0, 2 * (int)g.bits, sort_counts, c->stream,
+  uint64_t* sorted = radix_sort(akeys, alt, g.m_fwd, 0, 2 * (int)g.bits, sort_ws, sort_error(c), c->stream,
                                 &c->launches);
   g.off = buffer<uint64_t>(c, B_OFF, (size_t)g.n + 1);
   range_scan(LoadU32{g.fdeg}, EmitOffset{g.off}, g.n, sums, c->stream, &c->launches);
@@ -733,7 +736,7 @@ void build_totals(stc_ctx* c, const EdgeIds& e, const int8_t* d_sign, uint64_t m
                   const uint64_t* d_vbase, uint32_t G, const BatchCaps* caps = nullptr) {
   cudaStream_t st = c->stream;
   unsigned long long* ctr = (unsigned long long*)counters(c);
-  uint32_t* sort_counts = buffer<uint32_t>(c, B_SORT_COUNTS, (size_t)kRadix * kMaxSortGrid);
+  uint32_t* sort_ws = buffer<uint32_t>(c, B_SORT_WS, sort_workspace_words(std::max<uint64_t>(m, g.n)));
   uint64_t* sums = buffer<uint64_t>(c, B_SCAN_SUMS, kMaxSortGrid + 1);
   g.ukeys = nullptr;
   g.deg = buffer<uint32_t>(c, B_DEG, g.n);
@@ -786,7 +789,7 @@ void build_totals(stc_ctx* c, const EdgeIds& e, const int8_t* d_sign, uint64_t m
         c->launches++;
       }
     }
-    uint64_t* vs = radix_sort(va, vb, g.n, 32, 32 + (int)g.dbits + gbits, sort_counts, st,
+    uint64_t* vs = radix_sort(va, vb, g.n, 32, 32 + (int)g.dbits + gbits, sort_ws, sort_error(c), st,
                               &c->launches);
     k_rank<<<grid_for(g.n, 4), kThreads, 0, st>>>(vs, g.n, g.verts, g.rank);
     c->launches++;
@@ -801,7 +804,7 @@ void build_totals(stc_ctx* c, const EdgeIds& e, const int8_t* d_sign, uint64_t m
     wait_sign(c);  // a host sign array may still be on its way (stc_count)
     k_arc_keys_raw<<<ep.grid, kThreads, 0, st>>>(e, d_sign, m, g.bits, g.n, g.rank, ka, ctr);
     c->launches++;
-    uint64_t* sorted = radix_sort(ka, kb, m, 0, 2 * (int)g.bits, sort_counts, st, &c->launches);
+    uint64_t* sorted = radix_sort(ka, kb, m, 0, 2 * (int)g.bits, sort_ws, sort_error(c), st, &c->launches);
     const uint64_t mask = (1ull << (2 * g.bits)) - 1;
     if (caps) {
       const UniqueArcFlag flag{sorted, mask};
@@ -899,13 +902,13 @@ __global__ void k_relabel(const uint32_t* __restrict__ u, const uint32_t* __rest
 // points *src / *dst at them; returns the number of distinct ids.
 uint64_t relabel_dense(stc_ctx* c, const uint32_t** src, const uint32_t** dst, uint64_t m) {
   cudaStream_t st = c->stream;
-  uint32_t* sort_counts = buffer<uint32_t>(c, B_SORT_COUNTS, (size_t)kRadix * kMaxSortGrid);
+  uint32_t* sort_ws = buffer<uint32_t>(c, B_SORT_WS, sort_workspace_words(2 * m));
   uint64_t* sums = buffer<uint64_t>(c, B_SCAN_SUMS, kMaxSortGrid + 1);
   uint64_t* ka = buffer<uint64_t>(c, B_KEYS_A, 2 * m);
   uint64_t* kb = buffer<uint64_t>(c, B_KEYS_B, 2 * m);
   k_endpoint_keys<<<grid_for(m, 4), kThreads, 0, st>>>(*src, *dst, m, ka);
   c->launches++;
-  const uint64_t* sorted = radix_sort(ka, kb, 2 * m, 0, 32, sort_counts, st, &c->launches);
+  const uint64_t* sorted = radix_sort(ka, kb, 2 * m, 0, 32, sort_ws, sort_error(c), st, &c->launches);
   const UniqueFlag flag{sorted, 0xFFFFFFFFull};
   const uint32_t grid = range_reduce_scan(flag, 2 * m, sums, st, &c->launches);
   STC_CUDA(cudaMemcpyAsync(c->h_pinned + C_WORK, sums + grid, sizeof(uint64_t),
@@ -965,7 +968,7 @@ void build_graph(stc_ctx* c, const uint32_t* d_src, const uint32_t* d_dst, const
     build_totals(c, EdgeIds{d_src, d_dst, nullptr, nullptr, 0}, d_sign, m, g, nullptr, 0);
     return;
   }
-  uint32_t* sort_counts = buffer<uint32_t>(c, B_SORT_COUNTS, (size_t)kRadix * kMaxSortGrid);
+  uint32_t* sort_ws = buffer<uint32_t>(c, B_SORT_WS, sort_workspace_words(std::max<uint64_t>(m, g.n)));
   uint64_t* sums = buffer<uint64_t>(c, B_SCAN_SUMS, kMaxSortGrid + 1);
 
   // 2. dedup.
@@ -976,7 +979,7 @@ void build_graph(stc_ctx* c, const uint32_t* d_src, const uint32_t* d_dst, const
     wait_sign(c);
     k_pack_dedup<<<grid_for(m, 4), kThreads, 0, st>>>(d_src, d_dst, d_sign, m, g.bits, ka);
     c->launches++;
-    uint64_t* sorted = radix_sort(ka, kb, m, 0, 2 * (int)g.bits, sort_counts, st, &c->launches);
+    uint64_t* sorted = radix_sort(ka, kb, m, 0, 2 * (int)g.bits, sort_ws, sort_error(c), st, &c->launches);
     const uint64_t mask = (1ull << (2 * g.bits)) - 1;
     range_scan(UniqueFlag{sorted, mask}, UniqueEmit{sorted, g.ukeys}, g.m_valid, sums, st,
                &c->launches);
@@ -1007,7 +1010,7 @@ void build_graph(stc_ctx* c, const uint32_t* d_src, const uint32_t* d_dst, const
     c->launches++;
     read_counters(c, C_MAX_DEG, 1);
     g.max_deg = (uint32_t)c->h_pinned[C_MAX_DEG];
-    uint64_t* vs = radix_sort(va, vb, g.n, 32, 32 + (int)bit_width64(g.max_deg), sort_counts, st,
+    uint64_t* vs = radix_sort(va, vb, g.n, 32, 32 + (int)bit_width64(g.max_deg), sort_ws, sort_error(c), st,
                               &c->launches);
     k_rank<<<grid_for(g.n, 4), kThreads, 0, st>>>(vs, g.n, g.verts, g.rank);
     c->launches++;
@@ -1108,7 +1111,7 @@ void build_graph_batch(stc_ctx* c, const uint32_t* d_src, const uint32_t* d_dst,
     build_totals(c, EdgeIds{d_src, d_dst, d_eoff, d_vbase, G}, d_sign, m, g, d_vbase, G);
     return;
   }
-  uint32_t* sort_counts = buffer<uint32_t>(c, B_SORT_COUNTS, (size_t)kRadix * kMaxSortGrid);
+  uint32_t* sort_ws = buffer<uint32_t>(c, B_SORT_WS, sort_workspace_words(std::max<uint64_t>(m, g.n)));
   uint64_t* sums = buffer<uint64_t>(c, B_SCAN_SUMS, kMaxSortGrid + 1);
 
   // 2. dedup over the union.
@@ -1119,7 +1122,7 @@ void build_graph_batch(stc_ctx* c, const uint32_t* d_src, const uint32_t* d_dst,
     k_batch_pack<<<ep.grid, kThreads, 0, st>>>(d_src, d_dst, d_sign, m, d_eoff, d_vbase, G,
                                                 ep.per_cta, g.bits, ka);
     c->launches++;
-    uint64_t* sorted = radix_sort(ka, kb, m, 0, 2 * (int)g.bits, sort_counts, st, &c->launches);
+    uint64_t* sorted = radix_sort(ka, kb, m, 0, 2 * (int)g.bits, sort_ws, sort_error(c), st, &c->launches);
     const uint64_t mask = (1ull << (2 * g.bits)) - 1;
     range_scan(UniqueFlag{sorted, mask}, UniqueEmit{sorted, g.ukeys}, g.m_valid, sums, st,
                &c->launches);
@@ -1158,7 +1161,7 @@ void build_graph_batch(stc_ctx* c, const uint32_t* d_src, const uint32_t* d_dst,
       k_batch_vertex_graph<<<vp.grid, kThreads, 0, st>>>(va, g.n, d_vbase, G, vp.per_cta, 32 + dbits);
       c->launches++;
     }
-    uint64_t* vs = radix_sort(va, vb, g.n, 32, 32 + dbits + gbits, sort_counts, st, &c->launches);
+    uint64_t* vs = radix_sort(va, vb, g.n, 32, 32 + dbits + gbits, sort_ws, sort_error(c), st, &c->launches);
     k_rank<<<grid_for(g.n, 4), kThreads, 0, st>>>(vs, g.n, g.verts, g.rank);
     c->launches++;
   }
@@ -1225,7 +1228,7 @@ void export_forward_csr(stc_ctx* c, const DeviceGraph& g, stc_forward_csr* out) 
   uint64_t* off_id = buffer<uint64_t>(c, B_EXPORT_OFF, (size_t)n + 1);
   uint64_t* ka = buffer<uint64_t>(c, B_KEYS_A, mu);
   uint64_t* kb = buffer<uint64_t>(c, B_KEYS_B, mu);
-  uint32_t* sort_counts = buffer<uint32_t>(c, B_SORT_COUNTS, (size_t)kRadix * kMaxSortGrid);
+  uint32_t* sort_ws = buffer<uint32_t>(c, B_SORT_WS, sort_workspace_words(mu));
   uint64_t* sums = buffer<uint64_t>(c, B_SCAN_SUMS, kMaxSortGrid + 1);
   uint32_t* edges = buffer<uint32_t>(c, B_NBR, mu);
   int8_t* signs = buffer<int8_t>(c, B_SGN, mu);
@@ -1233,7 +1236,7 @@ void export_forward_csr(stc_ctx* c, const DeviceGraph& g, stc_forward_csr* out) 
   uint64_t* sorted = ka;
   if (mu) {
     k_export_keys<<<grid_for(mu, 4), kThreads, 0, st>>>(g.ukeys, mu, g.bits, g.rank, ka, fdeg_id);
-    sorted = radix_sort(ka, kb, mu, 0, 2 * (int)g.bits, sort_counts, st, &c->launches);
+    sorted = radix_sort(ka, kb, mu, 0, 2 * (int)g.bits, sort_ws, sort_error(c), st, &c->launches);
   }
   if (n) {
     range_scan(LoadU32{fdeg_id}, EmitOffset{off_id}, n, sums, st, &c->launches);

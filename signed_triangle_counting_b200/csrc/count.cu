@@ -2033,7 +2033,7 @@ struct HeadBufs {
   uint32_t* runs = nullptr;  // end of each head's run (n)
   HeadLists lists{};         // the classes' work items
   uint8_t* need = nullptr;   // per tail: it keeps arcs for the tail side
-  uint32_t* sort_counts = nullptr;
+  uint32_t* sort_ws = nullptr;
   uint8_t* sbits = nullptr;  // sign bits of the arcs
 };
 
@@ -2050,7 +2050,7 @@ HeadBufs head_buffers(stc_ctx* c, const DeviceGraph& g) {
   b.lists.b = b.lists.a + items;
   b.lists.cap = (uint32_t)items;
   b.need = reinterpret_cast<uint8_t*>(b.lists.b + items);
-  b.sort_counts = buffer<uint32_t>(c, B_SORT_COUNTS, (size_t)kRadix * kMaxSortGrid);
+  b.sort_ws = buffer<uint32_t>(c, B_SORT_WS, sort_workspace_words(g.m_fwd));
   b.sbits = buffer<uint8_t>(c, B_SBITS, (g.m_fwd + 7) / 8);
   return b;
 }
@@ -2115,7 +2115,7 @@ void enqueue_head(cudaStream_t st, const Csr& csr, const uint32_t* asrc, uint64_
   const uint32_t n = csr.n;
   const HeadKey fmt = HeadKey::of(n, m);
   const uint64_t* sorted = radix_sort(b.keys, b.alt, m, (int)fmt.ibits,
-                                      (int)(fmt.ibits + fmt.vbits), b.sort_counts, st, &launches,
+                                      (int)(fmt.ibits + fmt.vbits), b.sort_ws, ctr + C_ERROR, st, &launches,
                                       ctr + C_HEAD_NKEYS);
   uint32_t* end = b.runs;
   // The recorder times single arcs against a staged hash: no bitmap there.
@@ -2339,7 +2339,7 @@ void count_persistent(stc_ctx* c, const Csr& csr, const ClassBounds& cb, uint32_
   key.v[2] = s2;
   key.v[3] = reinterpret_cast<uint64_t>(s1);
   key.v[4] = hp.m;
-  key.v[5] = reinterpret_cast<uint64_t>(hb.sort_counts) ^
+  key.v[5] = reinterpret_cast<uint64_t>(hb.sort_ws) ^
              ((uint64_t)hp.tuning.block_threads << 48) ^ ((uint64_t)hp.tuning.unroll[0] << 56) ^
              ((uint64_t)hp.tuning.unroll[1] << 58) ^ ((uint64_t)hp.tuning.unroll[2] << 60) ^
              ((uint64_t)hp.tuning.hash_factor[0] << 40) ^ ((uint64_t)hp.tuning.hash_factor[1] << 42) ^

@@ -29,7 +29,7 @@ enum BufId {
   B_DEG, B_RANK, B_VERTS, B_FDEG,
   B_VKEYS_A, B_VKEYS_B,
   B_OFF, B_NBR, B_SGN, B_ASRC,
-  B_SORT_COUNTS, B_SCAN_SUMS,
+  B_SORT_WS, B_SCAN_SUMS,
   B_COUNTERS,                     // per-type counters, totals, flags
   B_WORK,                         // work queues / strategy worklists
   B_WORK2,

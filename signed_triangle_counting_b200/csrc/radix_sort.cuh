@@ -3,15 +3,17 @@
 // kernels have internal linkage: every translation unit that includes this
 // header gets its own copy.
 //
-// Design (B200): every pass is a reduce-then-scan over a fixed grid of
-// CTA-contiguous key ranges (4 CTAs per SM), so no kernel ever waits on
-// another CTA:
-//   upsweep   per-CTA digit histogram of its range      (reads 8 B/key;
-//             per-warp shared-memory atomics)
-//   scan      one CTA turns [digit][cta] counts into offsets
-//   downsweep per 4096-key tile: warp-striped match.any ranking (stable),
-//             tile-local reorder through shared memory, coalesced scatter
-//             (reads 8 B/key, writes 8 B/key).
+// Design (B200), after the published one-sweep method (Adinets and Merrill,
+// "Onesweep: A Faster Least Significant Digit Radix Sort for GPUs", 2022):
+//   histogram  one read of the keys counts the digits of every pass; the last
+//              CTA to finish scans the counts into each digit's first output
+//   pass       one kernel per 8-bit digit: a CTA takes the next tile, ranks
+//              its keys by digit (warp multi-split, stable), reorders them in
+//              shared memory, adds up the counts of the tiles before it by
+//              looking back over their published states, and writes each
+//              digit's keys in a row (reads 8 B/key, writes 8 B/key).
+// A CTA waits only for tiles taken before its own, whose CTAs are already
+// running; the wait is bounded all the same.
 // Bits of the key outside [lo, hi) ride along untouched, which is how the
 // edge sign travels in bit 63 without a separate payload array.
 #pragma once
@@ -24,11 +26,12 @@ namespace stc {
 
 constexpr int kSortThreads = 256;
 constexpr int kSortWarps = kSortThreads / 32;
-constexpr int kSortItems = 16;
-constexpr int kSortTile = kSortThreads * kSortItems;  // 4096 keys
+constexpr int kSortTile = 4096;  // granularity of range partitions
 constexpr int kRadix = 256;
+static_assert(kSortThreads == kRadix, "thread d of a pass owns digit d");
 constexpr int kMaxSortGrid = kSMs * 4;
-constexpr int kUpItems = 8;  // keys per thread per upsweep iteration
+constexpr int kMaxPasses = 8;
+constexpr int kHistItems = 8;  // keys in flight per thread of the histogram
 
 struct RangePartition {
   uint32_t grid;     // CTAs
@@ -44,197 +47,326 @@ inline RangePartition range_partition(uint64_t m, uint64_t tile, uint32_t max_gr
   return RangePartition{(uint32_t)grid, per * tile};
 }
 
-static __global__ void __launch_bounds__(kSortThreads) k_radix_upsweep(
-    const uint64_t* __restrict__ keys, uint64_t m, uint64_t per_cta, int shift,
-    uint32_t dmask, uint32_t* __restrict__ counts, uint32_t grid,
+// Workspace of one sort, in 32-bit words: the digit counts of every pass
+// (scanned in place), one tile ticket per pass, the histogram's CTA count and
+// the abort flag, then two arrays of tile states (a pass clears the one the
+// next pass uses).
+constexpr uint32_t kSortTickets = kMaxPasses * kRadix;
+constexpr uint32_t kSortDone = kSortTickets + kMaxPasses;
+constexpr uint32_t kSortAbort = kSortDone + 1;
+constexpr uint32_t kSortStates = kSortTickets + 2 * kMaxPasses;
+
+// Keys per thread of a pass: 16 once the tiles fill the GPU; smaller sorts
+// take smaller tiles, which spreads them over more SMs and shortens each
+// CTA's serial part (a pass over 100,000 keys takes 12 us, over 1,000,000
+// 19 us, over 2,400,000 32 us).
+inline int sort_items(uint64_t m) {
+  return m > (uint64_t)kSMs * 8 * kSortThreads * 8   ? 16
+         : m > (uint64_t)kSMs * 4 * kSortThreads * 4 ? 8
+                                                     : 4;
+}
+inline uint64_t sort_tiles(uint64_t m) {
+  const uint64_t tile = (uint64_t)kSortThreads * sort_items(m);
+  return (m + tile - 1) / tile;
+}
+// A tile state holds a count of keys and two flag bits: 32 bits a word while
+// counts stay below 2^30, else 64.
+inline bool sort_wide(uint64_t m) { return m >= (1ull << 30); }
+inline size_t sort_workspace_words(uint64_t m) {
+  return kSortStates + 2 * (size_t)kRadix * sort_tiles(m) * (sort_wide(m) ? 2 : 1);
+}
+
+// Digit counts of every pass over [lo, hi) into ws[pass][digit]; the last CTA
+// turns them into exclusive prefixes.
+static __global__ void __launch_bounds__(kSortThreads) k_radix_hist(
+    const uint64_t* __restrict__ keys, uint64_t m, int lo, int hi, uint32_t* __restrict__ ws,
     const unsigned long long* __restrict__ m_dev) {
-  __shared__ uint32_t hist[kSortWarps][kRadix + 1];
-  const unsigned tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
-  if (m_dev && *m_dev < m) m = *m_dev;
-  for (unsigned i = tid; i < kSortWarps * (kRadix + 1); i += kSortThreads) (&hist[0][0])[i] = 0;
-  __syncthreads();
-  const uint64_t begin = (uint64_t)blockIdx.x * per_cta;
-  const uint64_t end = begin + per_cta < m ? begin + per_cta : m;
-  // kUpItems independent loads in flight per thread, then one shared-memory
-  // atomic per key into the warp's own histogram.
-  for (uint64_t base = begin + warp * 32 * kUpItems; base < end; base += kSortThreads * kUpItems) {
-    uint32_t d[kUpItems];
-#pragma unroll
-    for (int j = 0; j < kUpItems; j++) {
-      const uint64_t i = base + j * 32 + lane;
-      d[j] = i < end ? (uint32_t)(__ldcs(keys + i) >> shift) & dmask : kRadix;
-    }
-#pragma unroll
-    for (int j = 0; j < kUpItems; j++)
-      if (d[j] != kRadix) atomicAdd(&hist[warp][d[j]], 1u);
-  }
-  __syncthreads();
-  for (unsigned d = tid; d < kRadix; d += kSortThreads) {
-    uint32_t s = 0;
-#pragma unroll
-    for (int w = 0; w < kSortWarps; w++) s += hist[w][d];
-    counts[(uint64_t)d * grid + blockIdx.x] = s;
-  }
-}
-
-// Exclusive scan of `n` 32-bit counts in place by one CTA of 1024 threads.
-// Each warp takes a contiguous run of 32-entry rows, read and written a
-// row at a time (coalesced): a first pass sums its run, the 32 sums are
-// scanned in shared memory, and a second pass scans row by row with the
-// warp's carry.
-static __global__ void __launch_bounds__(1024) k_scan_counts(uint32_t* __restrict__ a, uint32_t n) {
-  __shared__ uint32_t wbase[32];
-  const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
-  const uint32_t rows = (n + 31) / 32;
-  const uint32_t per = (rows + 31) / 32;
-  const uint32_t r0 = min(rows, warp * per), r1 = min(rows, r0 + per);
-  uint32_t s = 0;
-#pragma unroll 4
-  for (uint32_t r = r0; r < r1; r++) {
-    const uint32_t i = r * 32 + lane;
-    s += i < n ? a[i] : 0u;
-  }
-  s = __reduce_add_sync(kFull, s);
-  if (lane == 0) wbase[warp] = s;
-  __syncthreads();
-  if (warp == 0) {
-    const uint32_t t = wbase[lane];
-    const uint32_t inc = warp_inclusive_scan(t);
-    wbase[lane] = inc - t;
-  }
-  __syncthreads();
-  uint32_t carry = wbase[warp];
-#pragma unroll 4
-  for (uint32_t r = r0; r < r1; r++) {
-    const uint32_t i = r * 32 + lane;
-    const uint32_t x = i < n ? a[i] : 0u;
-    const uint32_t inc = warp_inclusive_scan(x);
-    if (i < n) a[i] = carry + inc - x;
-    carry += __shfl_sync(kFull, inc, 31);
-  }
-}
-
-// Ranks one tile's keys (stable): r[j] = the key's rank among the keys of
-// its digit in its warp's slice, whist[warp][digit] = the slice's count.
-// kFull: every key of the tile is valid, so digits fit 8 bits and the warp
-// match takes 8 ballots; a partial tile marks invalid keys with the digit
-// kRadix (9 bits).
-template <bool kFull>
-__device__ __forceinline__ void rank_tile(const uint64_t (&k)[kSortItems], uint64_t wbase,
-                                          uint64_t end, int shift, uint32_t dmask,
-                                          uint16_t (*whist)[kRadix + 1], unsigned warp,
-                                          unsigned lt, uint32_t (&r)[kSortItems]) {
-#pragma unroll
-  for (int j = 0; j < kSortItems; j++) {
-    const bool valid = kFull || wbase + (uint64_t)j * 32 < end;
-    const uint32_t dg = valid ? (uint32_t)(k[j] >> shift) & dmask : kRadix;
-    const unsigned peers = kFull ? match_label<8>(dg) : match_label<9>(dg);
-    const uint32_t base = whist[warp][dg];
-    const uint32_t below = __popc(peers & lt);
-    __syncwarp();
-    if (below == 0 && valid) whist[warp][dg] = (uint16_t)(base + __popc(peers));
-    __syncwarp();
-    r[j] = base + below;
-  }
-}
-
-static __global__ void __launch_bounds__(kSortThreads, 3) k_radix_downsweep(
-    const uint64_t* __restrict__ in, uint64_t* __restrict__ out, uint64_t m, uint64_t per_cta,
-    int shift, uint32_t dmask, const uint32_t* __restrict__ offsets, uint32_t grid,
-    const unsigned long long* __restrict__ m_dev) {
-  __shared__ uint64_t sbuf[kSortTile];
-  __shared__ uint16_t whist[kSortWarps][kRadix + 1];
-  __shared__ uint32_t tile_start[kRadix];
-  __shared__ uint32_t gofs[kRadix];
+  __shared__ uint32_t hist[kMaxPasses][kRadix];
   __shared__ uint32_t scan_tmp[kSortWarps + 1];
-  const unsigned tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
+  __shared__ bool s_last;
+  const unsigned tid = threadIdx.x, lane = lane_id();
   if (m_dev && *m_dev < m) m = *m_dev;
-  const uint64_t begin = (uint64_t)blockIdx.x * per_cta;
-  const uint64_t end = begin + per_cta < m ? begin + per_cta : m;
-  // gofs[d]: where digit d's next key goes in the output
-  for (unsigned d = tid; d < kRadix; d += kSortThreads) gofs[d] = offsets[(uint64_t)d * grid + blockIdx.x];
-  const unsigned lt = lanemask_lt();
-  for (uint64_t tile = begin; tile < end; tile += kSortTile) {
-    for (unsigned i = tid; i < kSortWarps * (kRadix + 1); i += kSortThreads) (&whist[0][0])[i] = 0;
-    __syncthreads();
-    uint64_t k[kSortItems];
-    uint32_t r[kSortItems];
-    const uint64_t wbase = tile + (uint64_t)warp * (32 * kSortItems) + lane;
-    const bool full = end - tile >= (uint64_t)kSortTile;
+  const int passes = (hi - lo + 7) / 8;
+  for (int i = tid; i < passes * kRadix; i += kSortThreads) (&hist[0][0])[i] = 0;
+  __syncthreads();
+  const uint64_t step = (uint64_t)gridDim.x * kSortThreads * kHistItems;
+  for (uint64_t base = ((uint64_t)blockIdx.x * kSortThreads + (tid & ~31u)) * kHistItems; base < m;
+       base += step) {
+    uint64_t k[kHistItems];
 #pragma unroll
-    for (int j = 0; j < kSortItems; j++) {
-      const uint64_t idx = wbase + (uint64_t)j * 32;
-      k[j] = (full || idx < end) ? __ldcs(in + idx) : 0;
+    for (int j = 0; j < kHistItems; j++) {
+      const uint64_t i = base + j * 32 + lane;
+      k[j] = i < m ? __ldcs(keys + i) : ~0ull;
     }
-    if (full)
-      rank_tile<true>(k, wbase, end, shift, dmask, whist, warp, lt, r);
-    else
-      rank_tile<false>(k, wbase, end, shift, dmask, whist, warp, lt, r);
-    __syncthreads();
-    // Thread d: the tile's count of digit d, then every warp's slot for it
-    // as a tile position (digit start + the warps before).
-    const unsigned d = tid;  // kSortThreads == kRadix
-    uint32_t cnt = 0;
+    for (int p = 0; p < passes; p++) {
+      const int shift = lo + 8 * p;
+      const uint32_t dmask = hi - shift < 8 ? (1u << (hi - shift)) - 1 : 255u;
 #pragma unroll
-    for (int w = 0; w < kSortWarps; w++) cnt += whist[w][d];
+      for (int j = 0; j < kHistItems; j++)
+        if (base + j * 32 + lane < m) atomicAdd(&hist[p][(uint32_t)(k[j] >> shift) & dmask], 1u);
+    }
+  }
+  __syncthreads();
+  for (int i = tid; i < passes * kRadix; i += kSortThreads) {
+    const uint32_t c = (&hist[0][0])[i];
+    if (c) atomicAdd(ws + i, c);
+  }
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) s_last = atomicAdd(ws + kSortDone, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  for (int p = 0; p < passes; p++) {
     uint32_t total;
-    const uint32_t st = block_exclusive_scan<kSortThreads>(cnt, scan_tmp, total);
-    {
-      uint32_t run = st;
-#pragma unroll
-      for (int w = 0; w < kSortWarps; w++) {
-        const uint32_t c = whist[w][d];
-        whist[w][d] = (uint16_t)run;
-        run += c;
-      }
-    }
-    tile_start[d] = gofs[d] - st;  // output index of tile position p is tile_start[digit] + p
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < kSortItems; j++) {
-      if (full || wbase + (uint64_t)j * 32 < end) {
-        const uint32_t dg = (uint32_t)(k[j] >> shift) & dmask;
-        sbuf[whist[warp][dg] + r[j]] = k[j];
-      }
-    }
-    __syncthreads();
-    const uint32_t valid = (uint32_t)(end - tile < (uint64_t)kSortTile ? end - tile : kSortTile);
-    for (uint32_t i = tid; i < valid; i += kSortThreads) {
-      const uint64_t key = sbuf[i];
-      const uint32_t dk = (uint32_t)(key >> shift) & dmask;
-      out[(uint32_t)(tile_start[dk] + i)] = key;  // indices are below m < 2^32
-    }
-    __syncthreads();
-    gofs[d] += cnt;
-    __syncthreads();
+    const uint32_t c = __ldcg(ws + p * kRadix + tid);
+    ws[p * kRadix + tid] = block_exclusive_scan<kSortThreads>(c, scan_tmp, total);
   }
 }
 
-// Scratch for radix_sort: `counts` holds kRadix * kMaxSortGrid words.
+// Tile states: flag bits above the count.
+template <class W>
+struct TileState {
+  static constexpr int kShift = sizeof(W) * 8 - 2;
+  static constexpr W kCount = (W(1) << kShift) - 1;
+  static constexpr W kLocal = W(1) << kShift;    // the tile's own count
+  static constexpr W kPrefix = W(2) << kShift;   // with all tiles before it
+  __device__ static void put(W* p, W v) { *(volatile W*)p = v; }
+  __device__ static W get(const W* p) { return *(const volatile W*)p; }
+};
+constexpr uint32_t kLookbackPolls = 1u << 22;  // bound of one wait, a few seconds
+
+// The digit (key >> shift) & dmask; kHigh: it lies in the upper word.
+template <bool kHigh>
+__device__ __forceinline__ uint32_t key_digit(uint64_t key, int shift, uint32_t dmask) {
+  const uint32_t lo = (uint32_t)key, hi = (uint32_t)(key >> 32);
+  return (kHigh ? hi >> (shift & 31) : __funnelshift_r(lo, hi, shift)) & dmask;
+}
+
+template <int ITEMS>
+struct PassSmem {
+  union {
+    uint64_t keys[kSortThreads * ITEMS];       // the tile, by digit
+    uint32_t mask[2][kSortWarps][kRadix];      // lanes by digit, two keys in turn
+  };
+  uint32_t whist[kSortWarps][kRadix];
+  uint32_t gofs[kRadix];
+  uint32_t scan_tmp[kSortWarps + 1];
+  uint32_t tile, abort;
+};
+
+// Stable ranks of the warp's keys among its keys of the digit, 16 bits each,
+// and the digits' counts in `whist`.  Per key, the lanes that share a digit
+// find each other by or-ing their bit into the digit's word of a table (an
+// 8-ballot match took 32 integer instructions a key and made the integer
+// pipe the pass's limit: 0.70 against 0.57 ms a pass over 100 M keys); the
+// lowest of them adds their number to the count, clears the word and hands
+// the old count to the others.  Two tables in turn: a table's next use comes
+// after the barriers of the other's.
+template <int ITEMS, bool kHigh, bool kFullTile>
+__device__ __forceinline__ void rank_keys(const uint64_t (&k)[ITEMS], uint32_t wbase,
+                                          uint32_t valid, int shift, uint32_t dmask,
+                                          PassSmem<ITEMS>& sm, uint32_t (&r)[ITEMS / 2]) {
+  const unsigned lane = lane_id(), warp = threadIdx.x >> 5, lt = lanemask_lt();
+#pragma unroll
+  for (int j0 = 0; j0 < ITEMS; j0 += 2) {
+    unsigned peers[2];
+    uint32_t old[2];
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      uint32_t dg = key_digit<kHigh>(k[j0 + q], shift, dmask);
+      if (!kFullTile && wbase + 32 * (j0 + q) >= valid) dg = kRadix - 1;
+      uint32_t* word = &sm.mask[q][warp][dg];
+      atomicOr(word, 1u << lane);
+      __syncwarp();
+      peers[q] = *word;
+      __syncwarp();
+      old[q] = 0;
+      if ((peers[q] & lt) == 0) {
+        *word = 0;
+        old[q] = atomicAdd(&sm.whist[warp][dg], (uint32_t)__popc(peers[q]));
+      }
+    }
+    uint32_t x[2];
+#pragma unroll
+    for (int q = 0; q < 2; q++)
+      x[q] = __shfl_sync(kFull, old[q], __ffs(peers[q]) - 1) + __popc(peers[q] & lt);
+    r[j0 / 2] = x[0] | (x[1] << 16);
+  }
+}
+
+// One pass: stable by the digit, one tile per CTA.  Bound by the shared-
+// memory pipe (77% busy: about 31 wavefronts per warp and key, for the
+// match, the counts and the exchange), not by DRAM: 2.8 TB/s at 100 M keys.
+// The version before (a count pass over the keys, a one-CTA scan of 256
+// counts per CTA, then this) took 2.0 ms a pass over 268 M keys, this 1.5 with
+// its share of the histogram; over 2.4 M keys 78 us (58 of them the scan),
+// this 31.  Tiles of several pieces with the counts taken first, to look back
+// less often, were slower (1.9 ms), as were warp matches by ballots (1.8) or
+// match.any (2.6).
+template <int ITEMS, class W, bool kHigh>
+static __global__ void __launch_bounds__(kSortThreads, 4) k_radix_pass(
+    const uint64_t* __restrict__ in, uint64_t* __restrict__ out, uint64_t m, int shift,
+    uint32_t dmask, uint32_t* __restrict__ ws, int pass, W* __restrict__ state,
+    W* __restrict__ next_state, const unsigned long long* __restrict__ m_dev,
+    unsigned long long* __restrict__ err) {
+  constexpr uint32_t kTile = kSortThreads * ITEMS;
+  using TS = TileState<W>;
+  __shared__ PassSmem<ITEMS> sm;
+  const unsigned tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
+  if (m_dev && *m_dev < m) m = *m_dev;
+  if (tid == 0) {
+    sm.tile = atomicAdd(ws + kSortTickets + pass, 1u);
+    sm.abort = 0;
+  }
+#pragma unroll
+  for (int w = 0; w < kSortWarps; w++) {
+    sm.whist[w][tid] = 0;
+    sm.mask[0][w][tid] = 0;
+    sm.mask[1][w][tid] = 0;
+  }
+  __syncthreads();
+  const uint32_t tile = sm.tile;
+  const uint64_t begin = (uint64_t)tile * kTile;
+  if (begin >= m) return;
+  const uint32_t valid = m - begin < kTile ? (uint32_t)(m - begin) : kTile;
+  next_state[(size_t)tile * kRadix + tid] = 0;
+  const uint32_t wbase = warp * (32 * ITEMS) + lane;
+  const uint64_t* src = in + begin + wbase;
+  uint64_t k[ITEMS];
+  uint32_t r[ITEMS / 2];
+  if (valid == kTile) {
+#pragma unroll
+    for (int j = 0; j < ITEMS; j++) k[j] = __ldcs(src + 32 * j);
+    rank_keys<ITEMS, kHigh, true>(k, wbase, valid, shift, dmask, sm, r);
+  } else {
+    // Keys past the end take the last digit: they are last in the tile, so
+    // they rank behind every real key.
+#pragma unroll
+    for (int j = 0; j < ITEMS; j++) k[j] = wbase + 32 * j < valid ? __ldcs(src + 32 * j) : ~0ull;
+    rank_keys<ITEMS, kHigh, false>(k, wbase, valid, shift, dmask, sm, r);
+  }
+  __syncthreads();
+  // Thread d: the tile's count of digit d, its first position in the tile
+  // and every warp's slot for it.
+  uint32_t cnt = 0, c[kSortWarps];
+#pragma unroll
+  for (int w = 0; w < kSortWarps; w++) {
+    c[w] = sm.whist[w][tid];
+    cnt += c[w];
+  }
+  if (tid == kRadix - 1) cnt -= kTile - valid;
+  W* own = state + (size_t)tile * kRadix + tid;
+  TS::put(own, (tile == 0 ? TS::kPrefix : TS::kLocal) | cnt);
+  uint32_t total;
+  const uint32_t st = block_exclusive_scan<kSortThreads>(cnt, sm.scan_tmp, total);
+  uint32_t run = st;
+#pragma unroll
+  for (int w = 0; w < kSortWarps; w++) {
+    sm.whist[w][tid] = run;
+    run += c[w];
+  }
+  __syncthreads();
+  const uint32_t* wh = sm.whist[warp];
+#pragma unroll
+  for (int j = 0; j < ITEMS; j++)
+    if (valid == kTile || wbase + 32 * j < valid)
+      sm.keys[wh[key_digit<kHigh>(k[j], shift, dmask)] + ((r[j / 2] >> (16 * (j & 1))) & 0xFFFFu)] =
+          k[j];
+  // Look back: four predecessors' states in flight at a time.
+  W before = 0;
+  if (tile > 0) {
+    const W* p = own - kRadix;
+    uint32_t left = tile, polls = 0;  // predecessors not yet added
+    bool done = false;
+    while (!done) {
+      W s[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) s[q] = (uint32_t)q < left ? TS::get(p - (size_t)q * kRadix) : 0;
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        if (done || s[q] == 0) break;
+        before += s[q] & TS::kCount;
+        done = (s[q] & TS::kPrefix) != 0;
+        p -= kRadix;
+        left--;
+      }
+      if (!done && ++polls > kLookbackPolls) {
+        ((volatile uint32_t*)ws)[kSortAbort] = 1;
+        done = true;
+      }
+      if (!done && (polls & 1023u) == 0 && ((volatile uint32_t*)ws)[kSortAbort]) done = true;
+    }
+    if (polls >= 1023u && ((volatile uint32_t*)ws)[kSortAbort]) sm.abort = 1;
+    TS::put(own, TS::kPrefix | (before + cnt));
+  }
+  sm.gofs[tid] = ws[pass * kRadix + tid] + (uint32_t)before - st;
+  __syncthreads();
+  if (sm.abort) {  // a wait expired: keep every index in range, and report it
+#pragma unroll
+    for (int j = 0; j < ITEMS; j++)
+      if (wbase + 32 * j < valid) out[begin + wbase + 32 * j] = k[j];
+    if (tid == 0) atomicExch(err, 2ull);
+    return;
+  }
+  // Position i of the tile goes to gofs[digit] + i (modulo 2^32; below m).
+#pragma unroll
+  for (int j = 0; j < ITEMS; j++) {
+    const uint32_t i = tid + j * kSortThreads;
+    if (valid == kTile || i < valid) {
+      const uint64_t key = sm.keys[i];
+      out[sm.gofs[key_digit<kHigh>(key, shift, dmask)] + i] = key;
+    }
+  }
+}
+
+template <int ITEMS, class W>
+inline void launch_radix_pass(const uint64_t* in, uint64_t* out, uint64_t m, int shift,
+                              uint32_t dmask, uint32_t* ws, int pass, uint64_t tiles,
+                              cudaStream_t st, const unsigned long long* m_dev,
+                              unsigned long long* err) {
+  W* a = reinterpret_cast<W*>(ws + kSortStates);
+  W* b = a + (size_t)kRadix * tiles;
+  auto kernel = shift >= 32 ? k_radix_pass<ITEMS, W, true> : k_radix_pass<ITEMS, W, false>;
+  kernel<<<(uint32_t)tiles, kSortThreads, 0, st>>>(in, out, m, shift, dmask, ws, pass,
+                                                   pass & 1 ? b : a, pass & 1 ? a : b, m_dev, err);
+}
+
 // Sorts keys[0, m) by bits [lo, hi) stably; returns the buffer that holds the
-// result (`keys` or `alt`).  m must be below 2^32.  With `m_dev`, the sort
-// covers only the first min(m, *m_dev) keys, a count known on the device
-// alone (the launches are sized for m, so the sequence can be captured).
+// result (`keys` or `alt`).  m must be below 2^32.  `ws` holds
+// sort_workspace_words(m) words; `err` receives 2 if a device-side wait
+// expired.  With `m_dev`, the sort covers only the first min(m, *m_dev) keys,
+// a count known on the device alone (the launches are sized for m, so the
+// sequence can be captured).
 inline uint64_t* radix_sort(uint64_t* keys, uint64_t* alt, uint64_t m, int lo, int hi,
-                            uint32_t* counts, cudaStream_t st, int* launches = nullptr,
-                            const unsigned long long* m_dev = nullptr) {
+                            uint32_t* ws, unsigned long long* err, cudaStream_t st,
+                            int* launches = nullptr, const unsigned long long* m_dev = nullptr) {
   if (m <= 1 || hi <= lo) return keys;
-  RangePartition p = range_partition(m, kSortTile, kMaxSortGrid);
+  const uint64_t tiles = sort_tiles(m);
+  const int items = sort_items(m);
+  const bool wide = sort_wide(m);
+  cudaMemsetAsync(ws, 0, (kSortStates + (size_t)kRadix * tiles * (wide ? 2 : 1)) * sizeof(uint32_t), st);
+  const uint64_t per = (uint64_t)kSortThreads * kHistItems;
+  const uint32_t grid = (uint32_t)((m + per - 1) / per < kSMs * 8 ? (m + per - 1) / per : kSMs * 8);
+  k_radix_hist<<<grid, kSortThreads, 0, st>>>(keys, m, lo, hi, ws, m_dev);
   uint64_t* src = keys;
   uint64_t* dst = alt;
-  for (int shift = lo; shift < hi; shift += 8) {
+  int pass = 0;
+  for (int shift = lo; shift < hi; shift += 8, pass++) {
     const int w = hi - shift < 8 ? hi - shift : 8;
     const uint32_t dmask = (1u << w) - 1;
-    k_radix_upsweep<<<p.grid, kSortThreads, 0, st>>>(src, m, p.per_cta, shift, dmask, counts, p.grid,
-                                                     m_dev);
-    k_scan_counts<<<1, 1024, 0, st>>>(counts, kRadix * p.grid);
-    k_radix_downsweep<<<p.grid, kSortThreads, 0, st>>>(src, dst, m, p.per_cta, shift, dmask, counts,
-                                                       p.grid, m_dev);
-    if (launches) *launches += 3;
+    auto run = [&](auto launch) {
+      launch(src, dst, m, shift, dmask, ws, pass, tiles, st, m_dev, err);
+    };
+    if (wide) run(launch_radix_pass<16, uint64_t>);
+    else if (items == 16) run(launch_radix_pass<16, uint32_t>);
+    else if (items == 8) run(launch_radix_pass<8, uint32_t>);
+    else run(launch_radix_pass<4, uint32_t>);
     uint64_t* t = src;
     src = dst;
     dst = t;
   }
+  if (launches) *launches += 1 + pass;
   return src;
 }
 
