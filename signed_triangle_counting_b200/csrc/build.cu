@@ -40,20 +40,29 @@ inline uint32_t grid_for(uint64_t n, uint32_t per_thread = 1) {
   return (uint32_t)g;
 }
 
-// Max kept id and self-loop count.
-__global__ void k_scan_ids(const uint32_t* __restrict__ u, const uint32_t* __restrict__ v,
-                           uint64_t m, unsigned long long* __restrict__ ctr) {
+// Max kept id and self-loop count; four edges of a thread in flight.
+__global__ void __launch_bounds__(256) k_scan_ids(const uint32_t* __restrict__ u,
+                                                  const uint32_t* __restrict__ v, uint64_t m,
+                                                  unsigned long long* __restrict__ ctr) {
   uint32_t mx = 0;
   uint32_t self = 0;
+  auto add = [&](uint32_t a, uint32_t b) {
+    if (a == b) self++;
+    else mx = max(mx, max(a, b));
+  };
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += stride) {
-    const uint32_t a = __ldcs(u + i), b = __ldcs(v + i);
-    if (a == b) {
-      self++;
-    } else {
-      mx = max(mx, max(a, b));
+  uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (; i + 3 * stride < m; i += 4 * stride) {
+    uint32_t a[4], b[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      a[q] = __ldcs(u + i + q * stride);
+      b[q] = __ldcs(v + i + q * stride);
     }
+#pragma unroll
+    for (int q = 0; q < 4; q++) add(a[q], b[q]);
   }
+  for (; i < m; i += stride) add(__ldcs(u + i), __ldcs(v + i));
   mx = __reduce_max_sync(kFull, mx);
   self = __reduce_add_sync(kFull, self);
   if (lane_id() == 0) {
@@ -184,7 +193,7 @@ __global__ void k_rank(const uint64_t* __restrict__ vkeys, uint32_t n, uint32_t*
   const uint32_t stride = gridDim.x * blockDim.x;
   for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += stride) {
     const uint32_t id = (uint32_t)vkeys[r];
-    verts[r] = id;
+    if (verts) verts[r] = id;
     rank[id] = r;
   }
 }
@@ -342,31 +351,39 @@ __device__ __forceinline__ uint32_t first_segment(const uint64_t* __restrict__ b
   return lo;
 }
 
-// Id space of every graph (max endpoint + 1) and the self-loop count.
-__global__ void k_batch_ids(const uint32_t* __restrict__ u, const uint32_t* __restrict__ v,
-                            uint64_t m, const uint64_t* __restrict__ eoff, uint32_t G,
-                            uint64_t per_cta, unsigned int* __restrict__ gspace,
-                            unsigned long long* __restrict__ ctr) {
+// Id space of every graph (max endpoint + 1) and the self-loop count.  Each
+// lane keeps the maximum of its current graph; a warp hands it over when one
+// of its lanes moves on to another graph, which happens about once a graph
+// and warp (a match of the lanes' graphs at every step took 1.2 ms for 98 M
+// edges).
+__global__ void __launch_bounds__(256) k_batch_ids(const uint32_t* __restrict__ u,
+                                                   const uint32_t* __restrict__ v, uint64_t m,
+                                                   const uint64_t* __restrict__ eoff, uint32_t G,
+                                                   uint64_t per_cta, unsigned int* __restrict__ gspace,
+                                                   unsigned long long* __restrict__ ctr) {
   const uint64_t begin = (uint64_t)blockIdx.x * per_cta;
   const uint64_t end = begin + per_cta < m ? begin + per_cta : m;
   if (begin >= end) return;
   uint32_t g = first_segment(eoff, G, begin);
-  uint32_t self = 0;
-  for (uint64_t base = begin + (threadIdx.x & ~31u); base < end; base += blockDim.x) {
-    const uint64_t i = base + lane_id();
-    const bool valid = i < end;
-    uint32_t space = 0;
-    if (valid) {
-      while (eoff[g + 1] <= i) g++;
-      const uint32_t a = u[i], b = v[i];
-      self += a == b;
-      space = max(a, b) + 1;
+  uint64_t gend = eoff[g + 1];
+  uint32_t self = 0, space = 0;
+  for (uint64_t i = begin + threadIdx.x; i < end; i += blockDim.x) {
+    if (i >= gend) {
+      if (space) atomicMax(gspace + g, space);
+      space = 0;
+      do {
+        g++;
+      } while (eoff[g + 1] <= i);
+      gend = eoff[g + 1];
     }
-    const uint32_t key = valid ? g : 0xFFFFFFFFu;
-    const unsigned peers = __match_any_sync(kFull, key);
-    const uint32_t mx = __reduce_max_sync(peers, space);
-    if (valid && (peers & lanemask_lt()) == 0) atomicMax(gspace + g, mx);
+    const uint32_t a = u[i], b = v[i];
+    self += a == b;
+    space = max(space, max(a, b) + 1);
   }
+  // The lanes of a warp mostly end in the same graph.
+  const bool one = __all_sync(kFull, g == __shfl_sync(kFull, g, 0));
+  const uint32_t mx = one ? __reduce_max_sync(kFull, space) : space;
+  if (mx && (!one || lane_id() == 0)) atomicMax(gspace + g, mx);
   self = __reduce_add_sync(kFull, self);
   if (lane_id() == 0 && self) atomicAdd(ctr + C_SELF, (unsigned long long)self);
 }
@@ -457,18 +474,28 @@ struct EdgeCursor {
 // only has to be a total order for exact counts; on dense power-law graphs
 // a sampled degree orders the vertices nearly as well (at RMAT scale 20 a
 // 1/4 sample moves the intersection work by under 0.1%) for a quarter of
-// the atomics.  Endpoints are scattered and a few hubs own millions of
-// copies, so each CTA first adds them in a shared-memory table per tile of
-// kRawTile edges and flushes the slots it used with one global atomic each
-// (an endpoint that finds no free slot within kDegProbes probes is added
-// directly).
-constexpr int kRawTile = 512;
+// the atomics.
+// Endpoints are scattered over the degrees, so they are added there one by
+// one; only the hubs, which may own millions of copies, would serialise on
+// their address.  k_find_hubs names them from a sample, and a CTA counts
+// those in shared memory.  (Counting every endpoint in a shared-memory table
+// flushed per tile, hubs or not, took 3.1 ms at RMAT scale 24, this 0.8;
+// 62 us against 20 for a million-point mesh.)
+
 // Edges of the input are taken in chunks of kEdgeChunk, chunk c by CTA
 // c mod grid: the CTAs of a launch work on neighbouring edges at any time,
 // so for a batch they gather the ranks and degrees of a few neighbouring
-// graphs at once, which stay in L2.
+// graphs at once, which stay in L2.  Lists too short to give every CTA such
+// a chunk take smaller ones.
 constexpr uint64_t kEdgeChunk = 4096;
-constexpr int kRawSlots = 2048;  // 2 kRawTile endpoints per tile: load <= 1/2
+constexpr int kEdgeItems = 4;  // edges of a thread in flight
+constexpr uint32_t kEdgeGrid = kSMs * 6;
+inline uint32_t edge_chunk(uint64_t m) {
+  return m < kEdgeChunk * kEdgeGrid ? kEdgeItems * kThreads : (uint32_t)kEdgeChunk;
+}
+inline uint32_t edge_grid(uint64_t m) {
+  return (uint32_t)std::min<uint64_t>((m + edge_chunk(m) - 1) / edge_chunk(m), kEdgeGrid);
+}
 
 __device__ __forceinline__ bool sampled_edge(uint32_t a, uint32_t b, uint32_t shift) {
   if (shift == 0) return true;
@@ -476,70 +503,222 @@ __device__ __forceinline__ bool sampled_edge(uint32_t a, uint32_t b, uint32_t sh
   return ((lo * 0x9E3779B1u) ^ (hi * 0x7FEB352Du) ^ ((lo ^ hi) >> 15)) >> (32 - shift) == 0;
 }
 
-__global__ void __launch_bounds__(kThreads) k_degree_raw(EdgeIds e, uint64_t m, uint32_t shift,
-                                                         uint32_t n, uint32_t* __restrict__ deg) {
-  __shared__ uint32_t tkey[kRawSlots], tcnt[kRawSlots], used[kRawSlots];
-  __shared__ uint32_t nused;
-  constexpr uint32_t kFree = 0xFFFFFFFFu;
-  for (int i = threadIdx.x; i < kRawSlots; i += kThreads) {
-    tkey[i] = kFree;
-    tcnt[i] = 0;
+// Hub table: kHubSlots ids in buckets of two.
+constexpr uint32_t kHubSlots = 1024;
+constexpr uint32_t kNoHub = 0xFFFFFFFFu;
+// Lists of fewer edges have no hub worth the sample.
+constexpr uint64_t kHubMinEdges = 1u << 20;
+__device__ __forceinline__ uint32_t hub_bucket(uint32_t x) {
+  return ((x * 0x9E3779B1u) >> (32 - 9)) * 2;  // of kHubSlots / 2 buckets
+}
+static_assert(kHubSlots == 2u << 9, "hub_bucket's shift");
+
+// Ids that occur at least kHubHits times among `sample` (a power of two)
+// endpoints taken at even distances: of 8,192, a hub with 1/1,000 of the
+// endpoints is missed once in 20 lists, one with 1/500 never, and what is
+// missed only costs its own serial additions.  One CTA (12 us for 2,048
+// endpoints); ids that find both slots of their bucket taken are left out.
+constexpr uint32_t kHubHits = 4;
+inline uint32_t hub_sample(uint64_t m) { return m < (1u << 24) ? 2048 : 8192; }
+inline size_t hub_smem(uint32_t sample) { return 4ull * sample * sizeof(uint32_t); }
+
+__global__ void __launch_bounds__(1024) k_find_hubs(const uint32_t* __restrict__ u,
+                                                    const uint32_t* __restrict__ v, uint64_t m,
+                                                    uint32_t sample, uint32_t* __restrict__ hubs) {
+  extern __shared__ uint32_t hub_seen[];
+  const uint32_t slots = 2 * sample;  // load <= 1/2
+  uint32_t* id = hub_seen;
+  uint32_t* hits = hub_seen + slots;
+  for (uint32_t i = threadIdx.x; i < slots; i += 1024) {
+    id[i] = kNoHub;
+    hits[i] = 0;
   }
-  if (threadIdx.x == 0) nused = 0;
+  for (uint32_t i = threadIdx.x; i < kHubSlots; i += 1024) hubs[i] = kNoHub;
   __syncthreads();
-  for (uint64_t chunk = blockIdx.x; chunk * kEdgeChunk < m; chunk += gridDim.x) {
-    const uint64_t begin = chunk * kEdgeChunk;
-    const uint64_t end = begin + kEdgeChunk < m ? begin + kEdgeChunk : m;
+  const uint64_t step = m / (sample / 2);
+  for (uint32_t i = threadIdx.x; i < sample; i += 1024) {
+    const uint64_t at = (i >> 1) * step;
+    const uint32_t x = (i & 1) ? v[at] : u[at];
+    if (x == kNoHub) continue;
+    uint32_t s = (x * 0x9E3779B1u) & (slots - 1);
+    while (true) {  // ends: more slots than endpoints
+      const uint32_t old = atomicCAS(&id[s], kNoHub, x);
+      if (old == kNoHub || old == x) break;
+      s = (s + 1) & (slots - 1);
+    }
+    if (atomicAdd(&hits[s], 1u) == kHubHits - 1) {
+      uint32_t* b = hubs + hub_bucket(x);
+      if (atomicCAS(b, kNoHub, x) != kNoHub) atomicCAS(b + 1, kNoHub, x);
+    }
+  }
+}
+
+// `hubs` (kHub only): k_find_hubs's table.  Ids at or past n only reach here
+// when a capped build's union outgrew its capacity (flagged by
+// k_batch_bases).
+template <bool kHub>
+__global__ void __launch_bounds__(kThreads) k_degree_raw(EdgeIds e, uint64_t m,
+                                                         uint32_t edge_chunk, uint32_t shift,
+                                                         uint32_t n,
+                                                         const uint32_t* __restrict__ hubs,
+                                                         uint32_t* __restrict__ deg) {
+  __shared__ __align__(8) uint32_t hid[kHub ? kHubSlots : 2], hcnt[kHub ? kHubSlots : 2];
+  if (kHub) {
+    for (uint32_t i = threadIdx.x; i < kHubSlots; i += kThreads) {
+      hid[i] = hubs[i];
+      hcnt[i] = 0;
+    }
+    __syncthreads();
+  }
+  auto add = [&](uint32_t x, bool valid) {
+    if (kHub) {
+      if (!valid) return;
+      const uint32_t b = hub_bucket(x);
+      const uint2 h = *reinterpret_cast<const uint2*>(hid + b);
+      if (h.x == x) atomicAdd(&hcnt[b], 1u);
+      else if (h.y == x) atomicAdd(&hcnt[b + 1], 1u);
+      else atomicAdd(deg + x, 1u);
+    } else {
+      // A run of one id (a list sorted by source, a star) is added once.
+      const uint32_t x0 = __shfl_sync(kFull, x, 0);
+      const unsigned same = __ballot_sync(kFull, valid && x == x0);
+      if (valid) {
+        if (x != x0) atomicAdd(deg + x, 1u);
+        else if ((same & lanemask_lt()) == 0) atomicAdd(deg + x, (uint32_t)__popc(same));
+      }
+    }
+  };
+  for (uint64_t begin = (uint64_t)blockIdx.x * edge_chunk; begin < m;
+       begin += (uint64_t)gridDim.x * edge_chunk) {
+    const uint64_t end = begin + edge_chunk < m ? begin + edge_chunk : m;
     EdgeCursor cur;
     cur.start(e, begin);
-    for (uint64_t t = begin; t < end; t += kRawTile) {
-  #pragma unroll
-      for (int r = 0; r < kRawTile / kThreads; r++) {
+    for (uint64_t t = begin; t < end; t += kEdgeItems * kThreads) {
+      uint32_t a[kEdgeItems], b[kEdgeItems];
+#pragma unroll
+      for (int r = 0; r < kEdgeItems; r++) {
         const uint64_t i = t + (uint64_t)r * kThreads + threadIdx.x;
-        uint32_t a = kFree, b = kFree;
-        if (i < end) {
-          cur.at(e, i, a, b);
-          // Ids at or past n only reach here when a capped build's union
-          // outgrew its capacity (flagged by k_batch_bases).
-          if (a == b || a >= n || b >= n || !sampled_edge(a, b, shift)) a = b = kFree;
-        }
-  #pragma unroll
-        for (int side = 0; side < 2; side++) {
-          const uint32_t x = side ? b : a;
-          const unsigned px = __match_any_sync(kFull, x);
-          if (x != kFree && (px & lanemask_lt()) == 0) {
-            const uint32_t add = (uint32_t)__popc(px);
-            uint32_t slot = (x * 0x9E3779B1u) >> (32 - 11);
-            bool placed = false;
-            for (int p = 0; p < kDegProbes && !placed; p++) {
-              uint32_t c = tkey[slot];
-              if (c == kFree) {  // claim the slot, or see who claimed it first
-                const uint32_t old = atomicCAS(&tkey[slot], kFree, x);
-                if (old == kFree) used[atomicAdd(&nused, 1u)] = slot;
-                c = old == kFree ? x : old;
-              }
-              if (c == x) {
-                atomicAdd(&tcnt[slot], add);
-                placed = true;
-              }
-              slot = (slot + 1) & (kRawSlots - 1);
-            }
-            if (!placed) atomicAdd(deg + x, add);
-          }
-        }
+        a[r] = b[r] = 0;  // a self-loop: skipped
+        if (i < end) cur.at(e, i, a[r], b[r]);
       }
-      __syncthreads();
-      const uint32_t nu = nused;
-      for (uint32_t j = threadIdx.x; j < nu; j += kThreads) {
-        const uint32_t slot = used[j];
-        atomicAdd(deg + tkey[slot], tcnt[slot]);
-        tkey[slot] = kFree;
-        tcnt[slot] = 0;
+#pragma unroll
+      for (int r = 0; r < kEdgeItems; r++) {
+        const bool valid = a[r] != b[r] && a[r] < n && b[r] < n && sampled_edge(a[r], b[r], shift);
+        add(a[r], valid);
+        add(b[r], valid);
       }
-      __syncthreads();
-      if (threadIdx.x == 0) nused = 0;
-      __syncthreads();
     }
+  }
+  if (kHub) {
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < kHubSlots; i += kThreads)
+      if (hcnt[i]) atomicAdd(deg + hid[i], hcnt[i]);
+  }
+}
+
+// Degrees as 8-bit sort digits: exact below 16, then eight steps per power of
+// two.  (degree step, id) is as good an order as (degree, id): the
+// intersection work at RMAT scale 20 grows by 0.2%, on sparse graphs not at
+// all, and the vertices sort in one 8-bit pass whatever the largest degree,
+// which need not be known on the host.
+__device__ __forceinline__ uint32_t degree_digit(uint32_t d) {
+  if (d < 16) return d;
+  const uint32_t bw = 32 - __clz(d);
+  return 16 + 8 * (bw - 5) + ((d >> (bw - 4)) & 7u);
+}
+
+// One graph's ranks in (degree digit, id) order without moving a key: the
+// counts of the digits, then one pass like the radix sort's whose output is
+// each vertex's position.  ws is a sort workspace; the last CTA of the count
+// turns the counts into each digit's first rank.
+constexpr int kRankItems = 16;
+constexpr uint32_t kRankTile = kSortThreads * kRankItems;
+
+inline size_t rank_workspace_words(uint32_t n) {
+  return kSortStates + (size_t)kRadix * (((uint64_t)n + kRankTile - 1) / kRankTile);
+}
+
+__global__ void __launch_bounds__(kSortThreads) k_degree_hist(const uint32_t* __restrict__ deg,
+                                                              uint32_t n, uint32_t* __restrict__ ws) {
+  __shared__ uint32_t hist[kRadix];
+  __shared__ uint32_t scan_tmp[kSortWarps + 1];
+  __shared__ bool s_last;
+  const uint32_t tid = threadIdx.x;
+  hist[tid] = 0;
+  __syncthreads();
+  for (uint64_t i = (uint64_t)blockIdx.x * kSortThreads + tid; i < n;
+       i += (uint64_t)gridDim.x * kSortThreads)
+    atomicAdd(&hist[degree_digit(deg[i])], 1u);
+  __syncthreads();
+  if (hist[tid]) atomicAdd(ws + tid, hist[tid]);
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) s_last = atomicAdd(ws + kSortDone, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  uint32_t total;
+  const uint32_t c = __ldcg(ws + tid);
+  ws[tid] = block_exclusive_scan<kSortThreads>(c, scan_tmp, total);
+}
+
+__global__ void __launch_bounds__(kSortThreads, 4) k_degree_rank(const uint32_t* __restrict__ deg,
+                                                                 uint32_t n, uint32_t* __restrict__ ws,
+                                                                 uint32_t* __restrict__ rank,
+                                                                 unsigned long long* __restrict__ err) {
+  using TS = TileState<uint32_t>;
+  __shared__ uint32_t mask[2][kSortWarps][kRadix];
+  __shared__ uint32_t whist[kSortWarps][kRadix];
+  __shared__ uint32_t s_tile, s_abort;
+  const uint32_t tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
+  if (tid == 0) {
+    s_tile = atomicAdd(ws + kSortTickets, 1u);
+    s_abort = 0;
+  }
+#pragma unroll
+  for (int w = 0; w < kSortWarps; w++) {
+    whist[w][tid] = 0;
+    mask[0][w][tid] = 0;
+    mask[1][w][tid] = 0;
+  }
+  __syncthreads();
+  const uint32_t tile = s_tile, begin = tile * kRankTile;
+  if (begin >= n) return;
+  const uint32_t valid = min(n - begin, kRankTile);
+  const uint32_t wbase = warp * (32 * kRankItems) + lane;
+  uint64_t k[kRankItems];  // digits
+  uint32_t r[kRankItems / 2];
+#pragma unroll
+  for (int j = 0; j < kRankItems; j++)
+    k[j] = wbase + 32 * j < valid ? degree_digit(deg[begin + wbase + 32 * j]) : 0u;
+  if (valid == kRankTile)
+    rank_keys<kRankItems, false, true>(k, wbase, valid, 0, kRadix - 1, mask, whist[warp], r);
+  else
+    rank_keys<kRankItems, false, false>(k, wbase, valid, 0, kRadix - 1, mask, whist[warp], r);
+  __syncthreads();
+  uint32_t cnt = 0, c[kSortWarps];
+#pragma unroll
+  for (int w = 0; w < kSortWarps; w++) {
+    c[w] = whist[w][tid];
+    cnt += c[w];
+  }
+  if (tid == kRadix - 1) cnt -= kRankTile - valid;  // past the end: the last digit
+  uint32_t* own = ws + kSortStates + (size_t)tile * kRadix + tid;
+  TS::put(own, (tile == 0 ? TS::kPrefix : TS::kLocal) | cnt);
+  uint32_t run = ws[tid] + look_back(own, tile, cnt, ws, s_abort);
+#pragma unroll
+  for (int w = 0; w < kSortWarps; w++) {
+    whist[w][tid] = run;
+    run += c[w];
+  }
+  __syncthreads();
+  if (s_abort && tid == 0) atomicExch(err, 2ull);
+#pragma unroll
+  for (int j = 0; j < kRankItems; j++) {
+    const uint32_t i = wbase + 32 * j;
+    if (i < valid)  // an expired wait leaves a rank below n all the same
+      rank[begin + i] = s_abort ? begin + i
+                                : whist[warp][(uint32_t)k[j]] + ((r[j / 2] >> (16 * (j & 1))) & 0xFFFFu);
   }
 }
 
@@ -548,28 +727,43 @@ __global__ void __launch_bounds__(kThreads) k_degree_raw(EdgeIds e, uint64_t m, 
 // sentinel of the 2 * bits window, which sorts after every real key.  An
 // endpoint at or past n (a capped build whose union outgrew its capacity)
 // also becomes the sentinel and sets C_OVERFLOW.
-__global__ void k_arc_keys_raw(EdgeIds e, const int8_t* __restrict__ sign, uint64_t m,
-                               uint32_t bits, uint32_t n, const uint32_t* __restrict__ rank,
-                               uint64_t* __restrict__ akeys, unsigned long long* __restrict__ ctr) {
+__global__ void __launch_bounds__(kThreads) k_arc_keys_raw(
+    EdgeIds e, const int8_t* __restrict__ sign, uint64_t m, uint32_t edge_chunk, uint32_t bits,
+    uint32_t n, const uint32_t* __restrict__ rank, uint64_t* __restrict__ akeys,
+    unsigned long long* __restrict__ ctr) {
   const uint64_t sentinel = (bits * 2 >= 64) ? ~0ull >> 1 : ((1ull << (2 * bits)) - 1);
-  for (uint64_t chunk = blockIdx.x; chunk * kEdgeChunk < m; chunk += gridDim.x) {
-    const uint64_t begin = chunk * kEdgeChunk;
-    const uint64_t end = begin + kEdgeChunk < m ? begin + kEdgeChunk : m;
+  for (uint64_t begin = (uint64_t)blockIdx.x * edge_chunk; begin < m;
+       begin += (uint64_t)gridDim.x * edge_chunk) {
+    const uint64_t end = begin + edge_chunk < m ? begin + edge_chunk : m;
     EdgeCursor cur;
     cur.start(e, begin);
-    for (uint64_t i = begin + threadIdx.x; i < end; i += blockDim.x) {
-      uint32_t a, b;
-      cur.at(e, i, a, b);
-      uint64_t k = sentinel;
-      if (a == b) {
-        // self-loop: the sentinel
-      } else if (a >= n || b >= n) {
-        atomicExch(ctr + C_OVERFLOW, 1ull);
-      } else {
-        const uint32_t ra = rank[a], rb = rank[b];
-        k = ((uint64_t)min(ra, rb) << bits) | max(ra, rb) | ((uint64_t)(sign[i] < 0) << 63);
+    for (uint64_t t = begin + threadIdx.x; t < end; t += kEdgeItems * kThreads) {
+      uint32_t a[kEdgeItems], b[kEdgeItems], neg = 0;
+#pragma unroll
+      for (int r = 0; r < kEdgeItems; r++) {
+        const uint64_t i = t + (uint64_t)r * kThreads;
+        a[r] = b[r] = 0;
+        if (i < end) {
+          cur.at(e, i, a[r], b[r]);
+          neg |= (uint32_t)(sign[i] < 0) << r;
+        }
       }
-      akeys[i] = k;
+      uint32_t ra[kEdgeItems], rb[kEdgeItems];
+#pragma unroll
+      for (int r = 0; r < kEdgeItems; r++) {
+        const bool in = a[r] != b[r] && a[r] < n && b[r] < n;
+        ra[r] = in ? rank[a[r]] : 0u;
+        rb[r] = in ? rank[b[r]] : 0u;  // equal: no key
+      }
+#pragma unroll
+      for (int r = 0; r < kEdgeItems; r++) {
+        const uint64_t i = t + (uint64_t)r * kThreads;
+        if (i >= end) break;
+        if (a[r] >= n || b[r] >= n) atomicExch(ctr + C_OVERFLOW, 1ull);
+        akeys[i] = ra[r] == rb[r] ? sentinel
+                                  : ((uint64_t)min(ra[r], rb[r]) << bits) | max(ra[r], rb[r]) |
+                                        ((uint64_t)((neg >> r) & 1u) << 63);
+      }
     }
   }
 }
@@ -678,36 +872,29 @@ __global__ void __launch_bounds__(1024) k_batch_bases(const unsigned int* __rest
   }
 }
 
-// Vertex sort keys of a capped batch build: graph << (32 + dbits) | degree
-// << 32 | id, the keys k_vertex_keys and k_batch_vertex_graph make together;
-// vertices past the union (vbase[G] <= i < n) take all-ones graph and
-// degree bits and so rank last.  A degree wider than dbits sets C_OVERFLOW.
+// Vertex sort keys of a batch's totals build: graph << (32 + dbits) | degree
+// digit (its top dbits bits) << 32 | id; vertices past the union (vbase[G] <=
+// i < n, a capped build) take all-ones graph and degree bits and so rank
+// last.
 __global__ void k_batch_vertex_keys(const uint32_t* __restrict__ deg, uint32_t n,
                                     const uint64_t* __restrict__ vbase, uint32_t G,
                                     uint64_t per_cta, uint32_t dbits, uint32_t gbits,
-                                    uint64_t* __restrict__ vkeys,
-                                    unsigned long long* __restrict__ ctr) {
+                                    uint64_t* __restrict__ vkeys) {
   const uint64_t begin = (uint64_t)blockIdx.x * per_cta;
   const uint64_t end = begin + per_cta < n ? begin + per_cta : n;
   if (begin >= end) return;
   const uint64_t nreal = vbase[G];
   const uint64_t pad = ((1ull << (dbits + gbits)) - 1) << 32;
   uint32_t g = begin < nreal ? first_segment(vbase, G, begin) : 0;
-  bool over = false;
   for (uint64_t i = begin + threadIdx.x; i < end; i += blockDim.x) {
     if (i >= nreal) {
       vkeys[i] = pad | i;
       continue;
     }
     while (vbase[g + 1] <= i) g++;
-    uint64_t d = deg[i];
-    if (d >> dbits) {
-      over = true;
-      d = (1ull << dbits) - 1;
-    }
+    const uint64_t d = degree_digit(deg[i]) >> (8 - dbits);
     vkeys[i] = (gbits ? (uint64_t)g << (32 + dbits) : 0ull) | (d << 32) | i;
   }
-  if (over) atomicExch(ctr + C_OVERFLOW, 1ull);
 }
 
 // UniqueFlag over all m sorted arc keys, the self-loop sentinels (sorted
@@ -725,25 +912,24 @@ struct UniqueArcFlag {
 };
 
 // Steps 2-6 of the totals path, after the ids (g.n, g.bits, g.m_valid set):
-// degrees over the edge copies (sampled on dense graphs), (degree, id) rank
-// (graph-major for a batch with vertex bases d_vbase), arc keys of every
-// copy, their sort, the first of each run of equal arcs, offsets.  g.ukeys
-// stays null.  With `caps` (a batch whose sizes stay on the device) nothing
-// is read back: g.n is the vertex capacity, the degree bits and sample shift
-// come from caps, and g.m_fwd is the arc capacity (m) with the arc count in
-// C_BATCH_MU (g.m_dev).
+// degrees over the edge copies (sampled on dense graphs; `hubs` is
+// k_find_hubs's table or null), (degree digit, id) rank (graph-major for a
+// batch with vertex bases d_vbase), arc keys of every copy, their sort, the
+// first of each run of equal arcs, offsets.  g.ukeys and g.verts stay null.
+// With `caps` (a batch whose sizes stay on the device) nothing is read back:
+// g.n is the vertex capacity, the sample shift comes from caps, and g.m_fwd
+// is the arc capacity (m) with the arc count in C_BATCH_MU (g.m_dev).
 void build_totals(stc_ctx* c, const EdgeIds& e, const int8_t* d_sign, uint64_t m, DeviceGraph& g,
-                  const uint64_t* d_vbase, uint32_t G, const BatchCaps* caps = nullptr) {
+                  const uint64_t* d_vbase, uint32_t G, const uint32_t* hubs = nullptr,
+                  const BatchCaps* caps = nullptr) {
   cudaStream_t st = c->stream;
   unsigned long long* ctr = (unsigned long long*)counters(c);
-  uint32_t* sort_ws = buffer<uint32_t>(c, B_SORT_WS, sort_workspace_words(std::max<uint64_t>(m, g.n)));
+  uint32_t* sort_ws = buffer<uint32_t>(c, B_SORT_WS, std::max(sort_workspace_words(std::max<uint64_t>(m, g.n)), rank_workspace_words(g.n)));
   uint64_t* sums = buffer<uint64_t>(c, B_SCAN_SUMS, kMaxSortGrid + 1);
   g.ukeys = nullptr;
   g.deg = buffer<uint32_t>(c, B_DEG, g.n);
   g.rank = buffer<uint32_t>(c, B_RANK, g.n);
-  g.verts = buffer<uint32_t>(c, B_VERTS, g.n);
   g.fdeg = buffer<uint32_t>(c, B_FDEG, g.n);
-  const RangePartition ep = range_partition(m, kSortTile, kMaxSortGrid);
   if (g.n) {
     STC_CUDA(cudaMemsetAsync(g.deg, 0, (size_t)g.n * sizeof(uint32_t), st));
     STC_CUDA(cudaMemsetAsync(g.fdeg, 0, (size_t)g.n * sizeof(uint32_t), st));
@@ -752,47 +938,40 @@ void build_totals(stc_ctx* c, const EdgeIds& e, const int8_t* d_sign, uint64_t m
     // Sample 1 in 2^shift edges once the average degree reaches 8 (2 m / n
     // >= 8): shift = bit width of m / n, less 2, at most 3.  (From degree 16
     // on the 1,024-graph batch counted 6 ms slower and built 17 ms faster;
-    // RMAT scale 24 moved by under 0.5 ms either way.)
+    // RMAT scale 24 moved by under 0.5 ms either way.)  Degrees that outgrow
+    // L2 cost a DRAM access each, which outweighs a sparse graph's better
+    // order: with 2^26 vertices and 2^27 edges, shift 0 / 1 / 2 / 3 took 6.7 /
+    // 3.6 / 2.0 / 1.2 ms here and 5.0 / 5.6 / 5.7 / 5.8 ms to count.
     const uint64_t ratio = g.m_valid / std::max<uint64_t>(1, g.n);
     const uint32_t bw = bit_width64(ratio);
-    g.shift = caps ? caps->shift : bw > 2 ? std::min<uint32_t>(3, bw - 2) : 0;
-    k_degree_raw<<<ep.grid, kThreads, 0, st>>>(e, m, g.shift, g.n, g.deg);
+    g.shift = bw > 2 ? std::min<uint32_t>(3, bw - 2) : 0;
+    if (g.n > 1u << 24) g.shift = std::max<uint32_t>(g.shift, g.n > 1u << 25 ? 3 : 2);
+    if (caps) g.shift = caps->shift;
+    auto kernel = hubs ? k_degree_raw<true> : k_degree_raw<false>;
+    kernel<<<edge_grid(m), kThreads, 0, st>>>(e, m, edge_chunk(m), g.shift, g.n, hubs, g.deg);
     c->launches++;
   }
   STC_CUDA(cudaGetLastError());
   mark(c, 2);
 
-  if (g.n) {
+  if (g.n && !d_vbase) {
+    const uint32_t tiles = (uint32_t)(((uint64_t)g.n + kRankTile - 1) / kRankTile);
+    STC_CUDA(cudaMemsetAsync(sort_ws, 0, rank_workspace_words(g.n) * sizeof(uint32_t), st));
+    k_degree_hist<<<grid_for(g.n, 16), kSortThreads, 0, st>>>(g.deg, g.n, sort_ws);
+    k_degree_rank<<<tiles, kSortThreads, 0, st>>>(g.deg, g.n, sort_ws, g.rank, sort_error(c));
+    c->launches += 2;
+  } else if (g.n) {
     uint64_t* va = buffer<uint64_t>(c, B_VKEYS_A, g.n);
     uint64_t* vb = buffer<uint64_t>(c, B_VKEYS_B, g.n);
-    const int gbits = d_vbase ? (int)bit_width64(G > 1 ? G - 1 : 0) : 0;
-    if (caps) {
-      g.dbits = caps->dbits;
-      if (32 + (int)g.dbits + gbits > 64)
-        fail(STC_ERR_LIMIT, "batch too large for the vertex sort key");
-      const RangePartition vp = range_partition(g.n, kSortTile, kMaxSortGrid);
-      k_batch_vertex_keys<<<vp.grid, kThreads, 0, st>>>(g.deg, g.n, d_vbase, G, vp.per_cta,
-                                                        g.dbits, (uint32_t)gbits, va, ctr);
-      c->launches++;
-    } else {
-      k_vertex_keys<<<grid_for(g.n, 4), kThreads, 0, st>>>(g.deg, g.n, va, ctr);
-      c->launches++;
-      read_counters(c, C_MAX_DEG, 1);
-      g.max_deg = (uint32_t)c->h_pinned[C_MAX_DEG];
-      g.dbits = bit_width64(g.max_deg);
-      if (32 + (int)g.dbits + gbits > 64)
-        fail(STC_ERR_LIMIT, "batch too large for the vertex sort key");
-      if (gbits) {
-        const RangePartition vp = range_partition(g.n, kSortTile, kMaxSortGrid);
-        k_batch_vertex_graph<<<vp.grid, kThreads, 0, st>>>(va, g.n, d_vbase, G, vp.per_cta,
-                                                           32 + g.dbits);
-        c->launches++;
-      }
-    }
-    uint64_t* vs = radix_sort(va, vb, g.n, 32, 32 + (int)g.dbits + gbits, sort_ws, sort_error(c), st,
+    const uint32_t gbits = bit_width64(G > 1 ? G - 1 : 0);
+    const uint32_t dbits = std::min<uint32_t>(8, 32 - gbits);
+    const RangePartition vp = range_partition(g.n, kSortTile, kMaxSortGrid);
+    k_batch_vertex_keys<<<vp.grid, kThreads, 0, st>>>(g.deg, g.n, d_vbase, G, vp.per_cta, dbits,
+                                                      gbits, va);
+    uint64_t* vs = radix_sort(va, vb, g.n, 32, (int)(32 + dbits + gbits), sort_ws, sort_error(c), st,
                               &c->launches);
-    k_rank<<<grid_for(g.n, 4), kThreads, 0, st>>>(vs, g.n, g.verts, g.rank);
-    c->launches++;
+    k_rank<<<grid_for(g.n, 4), kThreads, 0, st>>>(vs, g.n, nullptr, g.rank);
+    c->launches += 2;
   }
   STC_CUDA(cudaGetLastError());
   mark(c, 3);
@@ -802,7 +981,8 @@ void build_totals(stc_ctx* c, const EdgeIds& e, const int8_t* d_sign, uint64_t m
     uint64_t* ka = buffer<uint64_t>(c, B_KEYS_A, m);
     uint64_t* kb = buffer<uint64_t>(c, B_KEYS_B, m);
     wait_sign(c);  // a host sign array may still be on its way (stc_count)
-    k_arc_keys_raw<<<ep.grid, kThreads, 0, st>>>(e, d_sign, m, g.bits, g.n, g.rank, ka, ctr);
+    k_arc_keys_raw<<<edge_grid(m), kThreads, 0, st>>>(e, d_sign, m, edge_chunk(m), g.bits, g.n,
+                                                      g.rank, ka, ctr);
     c->launches++;
     uint64_t* sorted = radix_sort(ka, kb, m, 0, 2 * (int)g.bits, sort_ws, sort_error(c), st, &c->launches);
     const uint64_t mask = (1ull << (2 * g.bits)) - 1;
@@ -951,6 +1131,16 @@ void build_graph(stc_ctx* c, const uint32_t* d_src, const uint32_t* d_dst, const
     k_scan_ids<<<grid_for(m, 4), kThreads, 0, st>>>(d_src, d_dst, m, ctr);
     c->launches++;
   }
+  const uint32_t* hubs = nullptr;
+  if (totals && m >= kHubMinEdges) {
+    const uint32_t sample = hub_sample(m);
+    uint32_t* h = buffer<uint32_t>(c, B_HUBS, kHubSlots);
+    STC_CUDA(cudaFuncSetAttribute(k_find_hubs, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)hub_smem(8192)));
+    k_find_hubs<<<1, 1024, hub_smem(sample), st>>>(d_src, d_dst, m, sample, h);
+    c->launches++;
+    hubs = h;
+  }
   read_counters(c, C_MAX_ID, 2);
   uint64_t max_id = c->h_pinned[C_MAX_ID];
   const uint64_t self = c->h_pinned[C_SELF];
@@ -960,12 +1150,13 @@ void build_graph(stc_ctx* c, const uint32_t* d_src, const uint32_t* d_dst, const
   if (max_id >= (1ull << 31) - 1) {
     if (!totals) fail(STC_ERR_LIMIT, "vertex id " + std::to_string(max_id) + " >= 2^31 - 1");
     max_id = relabel_dense(c, &d_src, &d_dst, m) - 1;
+    hubs = nullptr;  // named by the ids of the list as given
   }
   g.n = m ? (uint32_t)max_id + 1 : 0;
   g.m_valid = m - self;
   g.bits = std::max<uint32_t>(1, bit_width64(max_id));
   if (totals) {
-    build_totals(c, EdgeIds{d_src, d_dst, nullptr, nullptr, 0}, d_sign, m, g, nullptr, 0);
+    build_totals(c, EdgeIds{d_src, d_dst, nullptr, nullptr, 0}, d_sign, m, g, nullptr, 0, hubs);
     return;
   }
   uint32_t* sort_ws = buffer<uint32_t>(c, B_SORT_WS, sort_workspace_words(std::max<uint64_t>(m, g.n)));
@@ -1217,7 +1408,7 @@ void build_graph_batch_capped(stc_ctx* c, const uint32_t* d_src, const uint32_t*
   g.m_valid = m;
   g.bits = caps.bits;
   g.gbase = d_vbase;
-  build_totals(c, EdgeIds{d_src, d_dst, d_eoff, d_vbase, G}, d_sign, m, g, d_vbase, G, &caps);
+  build_totals(c, EdgeIds{d_src, d_dst, d_eoff, d_vbase, G}, d_sign, m, g, d_vbase, G, nullptr, &caps);
 }
 
 void export_forward_csr(stc_ctx* c, const DeviceGraph& g, stc_forward_csr* out) {

@@ -192,7 +192,6 @@ bool caps_from(const DeviceGraph& g, BatchCaps& caps) {
   caps.bits = std::max<uint32_t>(1, bit_width64(g.n - 1));
   const uint64_t room = std::min<uint64_t>(1ull << caps.bits, (1ull << 31) - 2);
   caps.n = (uint32_t)std::max<uint64_t>(g.n, std::min<uint64_t>(g.n + g.n / 16 + 64, room));
-  caps.dbits = g.dbits;
   caps.shift = g.shift;
   return true;
 }

@@ -50,6 +50,7 @@ enum BufId {
   B_NKEY,                         // arcs: head << 1 | negative (m + 8)
   B_SBITS,                        // arcs: sign bits, one byte per 8 arcs (the head bitmap's stream)
   B_RELABEL,                      // ids >= 2^31 - 1: the edges relabelled to dense ids (2 m)
+  B_HUBS,                         // ids with very many edges (totals path)
   B_DISTINCT,                     // ids >= 2^31 - 1: the sorted distinct ids
   B_COUNT_
 };
@@ -117,13 +118,12 @@ struct Tuning {
 
 // Sizes a batch group's build is launched with when nothing is read back to
 // the host between its stages: vertex capacity of the union, id bits of the
-// arc keys, degree bits of the vertex sort key and the degree sample shift.
+// arc keys and the degree sample shift.
 // They come from an earlier build of a group of the same shape; the device
 // checks the new group against them (C_OVERFLOW).
 struct BatchCaps {
   uint32_t n = 0;
   uint32_t bits = 1;
-  uint32_t dbits = 0;
   uint32_t shift = 0;
 };
 
@@ -223,7 +223,7 @@ struct DeviceGraph {
   uint64_t* ukeys = nullptr;  // sorted unique keys: min << bits | max, sign in bit 63
   uint32_t* deg = nullptr;    // undirected degree, by id
   uint32_t* rank = nullptr;   // id -> rank
-  uint32_t* verts = nullptr;  // rank -> id
+  uint32_t* verts = nullptr;  // rank -> id (not of a totals build)
   uint64_t* off = nullptr;    // n + 1, rank space
   uint32_t* nbr = nullptr;    // arcs: head vertex (rank), sorted within each list
   int8_t* sgn = nullptr;      // arcs: +1 / -1
@@ -235,7 +235,6 @@ struct DeviceGraph {
   // arc count is then on the device (m_dev), vertices past the union's last
   // rank have no arcs.
   const unsigned long long* m_dev = nullptr;
-  uint32_t dbits = 0;  // degree bits of the vertex sort key (totals path)
   uint32_t shift = 0;  // degree sample shift (totals path)
   // Batches: G graphs whose vertices (ids and ranks) are contiguous; graph
   // g owns [gbase[g], gbase[g + 1]).  G == 0 for a single graph.
@@ -255,8 +254,8 @@ void mark(stc_ctx* c, int slot);
 void wait_sign(stc_ctx* c);
 
 // Graph build: input device arrays -> DeviceGraph (all fields).  With
-// `totals`, for counts of totals only: the vertex order is (degree over the
-// input's edge copies, id), so no dedup runs before the orientation (the
+// `totals`, for counts of totals only: the vertex order is (degree step over
+// the input's edge copies, id), so no dedup runs before the orientation (the
 // arc sort drops the copies, keeping the first), and g.ukeys stays null.
 // Without it, the reference's (unique degree, id) order, which per-vertex
 // counts, shards, CSR export, the timing recorder and the autotuner use.

@@ -136,6 +136,42 @@ struct TileState {
 };
 constexpr uint32_t kLookbackPolls = 1u << 22;  // bound of one wait, a few seconds
 
+// Thread d of tile `tile`: the count of digit d in all tiles before it (its
+// own state at `own`, holding its count `cnt`, becomes the sum), four
+// predecessors' states in flight at a time.  A wait that expires raises the
+// abort flag.
+template <class W>
+__device__ __forceinline__ W look_back(W* own, uint32_t tile, uint32_t cnt, uint32_t* ws,
+                                       uint32_t& abort) {
+  using TS = TileState<W>;
+  W before = 0;
+  if (tile == 0) return before;
+  const W* p = own - kRadix;
+  uint32_t left = tile, polls = 0;  // predecessors not yet added
+  bool done = false;
+  while (!done) {
+    W s[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) s[q] = (uint32_t)q < left ? TS::get(p - (size_t)q * kRadix) : 0;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      if (done || s[q] == 0) break;
+      before += s[q] & TS::kCount;
+      done = (s[q] & TS::kPrefix) != 0;
+      p -= kRadix;
+      left--;
+    }
+    if (!done && ++polls > kLookbackPolls) {
+      ((volatile uint32_t*)ws)[kSortAbort] = 1;
+      done = true;
+    }
+    if (!done && (polls & 1023u) == 0 && ((volatile uint32_t*)ws)[kSortAbort]) done = true;
+  }
+  if (polls >= 1023u && ((volatile uint32_t*)ws)[kSortAbort]) abort = 1;
+  TS::put(own, TS::kPrefix | (before + cnt));
+  return before;
+}
+
 // The digit (key >> shift) & dmask; kHigh: it lies in the upper word.
 template <bool kHigh>
 __device__ __forceinline__ uint32_t key_digit(uint64_t key, int shift, uint32_t dmask) {
@@ -166,7 +202,8 @@ struct PassSmem {
 template <int ITEMS, bool kHigh, bool kFullTile>
 __device__ __forceinline__ void rank_keys(const uint64_t (&k)[ITEMS], uint32_t wbase,
                                           uint32_t valid, int shift, uint32_t dmask,
-                                          PassSmem<ITEMS>& sm, uint32_t (&r)[ITEMS / 2]) {
+                                          uint32_t (*mask)[kSortWarps][kRadix], uint32_t* whist,
+                                          uint32_t (&r)[ITEMS / 2]) {
   const unsigned lane = lane_id(), warp = threadIdx.x >> 5, lt = lanemask_lt();
 #pragma unroll
   for (int j0 = 0; j0 < ITEMS; j0 += 2) {
@@ -176,7 +213,7 @@ __device__ __forceinline__ void rank_keys(const uint64_t (&k)[ITEMS], uint32_t w
     for (int q = 0; q < 2; q++) {
       uint32_t dg = key_digit<kHigh>(k[j0 + q], shift, dmask);
       if (!kFullTile && wbase + 32 * (j0 + q) >= valid) dg = kRadix - 1;
-      uint32_t* word = &sm.mask[q][warp][dg];
+      uint32_t* word = &mask[q][warp][dg];
       atomicOr(word, 1u << lane);
       __syncwarp();
       peers[q] = *word;
@@ -184,7 +221,7 @@ __device__ __forceinline__ void rank_keys(const uint64_t (&k)[ITEMS], uint32_t w
       old[q] = 0;
       if ((peers[q] & lt) == 0) {
         *word = 0;
-        old[q] = atomicAdd(&sm.whist[warp][dg], (uint32_t)__popc(peers[q]));
+        old[q] = atomicAdd(whist + dg, (uint32_t)__popc(peers[q]));
       }
     }
     uint32_t x[2];
@@ -238,13 +275,13 @@ static __global__ void __launch_bounds__(kSortThreads, 4) k_radix_pass(
   if (valid == kTile) {
 #pragma unroll
     for (int j = 0; j < ITEMS; j++) k[j] = __ldcs(src + 32 * j);
-    rank_keys<ITEMS, kHigh, true>(k, wbase, valid, shift, dmask, sm, r);
+    rank_keys<ITEMS, kHigh, true>(k, wbase, valid, shift, dmask, sm.mask, sm.whist[warp], r);
   } else {
     // Keys past the end take the last digit: they are last in the tile, so
     // they rank behind every real key.
 #pragma unroll
     for (int j = 0; j < ITEMS; j++) k[j] = wbase + 32 * j < valid ? __ldcs(src + 32 * j) : ~0ull;
-    rank_keys<ITEMS, kHigh, false>(k, wbase, valid, shift, dmask, sm, r);
+    rank_keys<ITEMS, kHigh, false>(k, wbase, valid, shift, dmask, sm.mask, sm.whist[warp], r);
   }
   __syncthreads();
   // Thread d: the tile's count of digit d, its first position in the tile
@@ -273,33 +310,7 @@ static __global__ void __launch_bounds__(kSortThreads, 4) k_radix_pass(
     if (valid == kTile || wbase + 32 * j < valid)
       sm.keys[wh[key_digit<kHigh>(k[j], shift, dmask)] + ((r[j / 2] >> (16 * (j & 1))) & 0xFFFFu)] =
           k[j];
-  // Look back: four predecessors' states in flight at a time.
-  W before = 0;
-  if (tile > 0) {
-    const W* p = own - kRadix;
-    uint32_t left = tile, polls = 0;  // predecessors not yet added
-    bool done = false;
-    while (!done) {
-      W s[4];
-#pragma unroll
-      for (int q = 0; q < 4; q++) s[q] = (uint32_t)q < left ? TS::get(p - (size_t)q * kRadix) : 0;
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        if (done || s[q] == 0) break;
-        before += s[q] & TS::kCount;
-        done = (s[q] & TS::kPrefix) != 0;
-        p -= kRadix;
-        left--;
-      }
-      if (!done && ++polls > kLookbackPolls) {
-        ((volatile uint32_t*)ws)[kSortAbort] = 1;
-        done = true;
-      }
-      if (!done && (polls & 1023u) == 0 && ((volatile uint32_t*)ws)[kSortAbort]) done = true;
-    }
-    if (polls >= 1023u && ((volatile uint32_t*)ws)[kSortAbort]) sm.abort = 1;
-    TS::put(own, TS::kPrefix | (before + cnt));
-  }
+  const W before = look_back(own, tile, cnt, ws, sm.abort);
   sm.gofs[tid] = ws[pass * kRadix + tid] + (uint32_t)before - st;
   __syncthreads();
   if (sm.abort) {  // a wait expired: keep every index in range, and report it
