@@ -1335,13 +1335,14 @@ void launch_classes(cudaStream_t st, const Csr& csr, const uint32_t* lists, cons
 constexpr uint32_t kHeadMaxB = kLargeCap - 1;  // |N+(v)| of a HEAD arc: bucket <= 12
 static_assert(32 - __builtin_clz(kHeadMaxB) == 12 && 32 - __builtin_clz(kHeadMaxB + 1) == 13,
               "HEAD cells (bucket |B| <= 12) are exactly the arcs whose head fits the large class");
-constexpr int kHeadClasses = 4;
-constexpr uint32_t kHeadBits = 3;        // the bitmap class (k_head_bits)
+constexpr int kHeadClasses = 5;
+constexpr uint32_t kHeadBits = 3;   // the bitmap classes (k_head_bits): ranks streamed whole,
+constexpr uint32_t kHeadShort = 4;  // or as their low 16 bits
 constexpr uint32_t kHeadItemMin = 2048;  // the smallest class item size
 
 // In-arcs per work item of head class c (powers of two).
 __host__ __device__ __forceinline__ uint32_t head_item(uint32_t c) {
-  return c == 0 ? kHeadItemMin : c == 2 ? 16384u : 8192u;
+  return c == 0 ? kHeadItemMin : c == 2 ? 16384u : 8192u;  // (both bitmap classes: 8,192)
 }
 
 // Table class of a list of d arcs (tiny lists use the warp class's table).
@@ -1354,27 +1355,32 @@ __device__ __forceinline__ uint32_t head_class(uint32_t d) {
   return d <= kWarpCap ? 0u : d <= kBlockCap ? 1u : 2u;
 }
 
-// Ranks a bitmap covers (two bits each: 64 KB, so two CTAs of 512 threads and
-// an L1 for the stream share an SM), and the shortest |N+(v)| that is worth a
-// CTA and a bitmap of its own.  At RMAT scale 24 the top 2^18 ranks are the
-// heads of 90% of the arcs and 97% of the probes; the heads below keep the
-// hash.
+// Ranks a bitmap covers, two bits each, and the shortest |N+(v)| that is worth
+// a CTA and a bitmap of its own.  The wide window takes 64 KB (two CTAs of 512
+// threads and an L1 for the stream share an SM); at RMAT scale 24 the top
+// 2^18 ranks are the heads of 90% of the arcs and 97% of the probes, and the
+// heads below keep the hash.  In the short window, 16 KB, a rank's low 16 bits
+// are enough, so it streams 16-bit heads: half the bytes for the 83% of the
+// probes whose heads it holds there.  Its CTAs are small, so it takes lists
+// down to 33 entries from the warp class's hash (128-graph batch: 22.2 ms at
+// 129 entries, 19.5 at 65, 19.4 at 33, 19.8 at 9).
 constexpr uint32_t kBitsWindow = 1u << 18;
-constexpr uint32_t kBitsWords = kBitsWindow / 16;
-constexpr uint32_t kBitsMinB = kWarpCap;
-constexpr int kBitsThreads = 512;
+constexpr uint32_t kShortWindow = 1u << 16;
+constexpr uint32_t kBitsMinB = kWarpCap, kShortMinB = 32;
+constexpr int kBitsThreads = 512, kBitsCtas = 2;  // wide window; CTAs per SM
+constexpr int kShortThreads = 128, kShortCtas = 10;
 
 // Which head vertices take the bitmap: v's list and every A' of its in-arcs
 // lie in (v, last rank of v's graph], so the bitmap, indexed by the low bits
-// of the rank, holds them without collision when that range is at most
-// `window` long (0: no bitmap).
+// of the rank, holds them without collision when that range is at most a
+// window long (`window` 0: no bitmap).
 struct BitsRule {
   uint32_t window;
   uint32_t n;
   const uint64_t* gbase;  // G + 1 rank boundaries of a batch, or null
   uint32_t G;
   __device__ __forceinline__ uint32_t head_class_of(uint32_t v, uint32_t d) const {
-    if (d > kBitsMinB && window) {
+    if (d > min(kBitsMinB, kShortMinB) && window) {
       uint32_t end = n;
       if (gbase) {
         uint32_t lo = 0, hi = G;
@@ -1384,7 +1390,8 @@ struct BitsRule {
         }
         end = (uint32_t)gbase[lo + 1];
       }
-      if (end - v <= window) return kHeadBits;
+      if (end - v <= kShortWindow && d > kShortMinB) return kHeadShort;
+      if (end - v <= window && d > kBitsMinB) return kHeadBits;
     }
     return head_class(d);
   }
@@ -1422,17 +1429,16 @@ struct HeadKey {
   }
 };
 
-// The work items (first entries) of the head classes, in two arrays of `cap`
-// words filled from both ends: class 0 from the front of `a`, class 3 from
-// its back, classes 1 and 2 likewise in `b`.  A head has one class, so the
-// two lists of an array never meet, and no counting pass is needed.
+// The work items (first entries) of the head classes, in three arrays of
+// `cap` words, two of them filled from both ends: classes 0 and 1 from the
+// front and the back of the first, 2 and 3 likewise in the second, 4 in the
+// third.  A head has one class, so the two lists of an array never meet, and
+// no counting pass is needed.
 struct HeadLists {
-  uint32_t* a;
-  uint32_t* b;
+  uint32_t* base;
   uint32_t cap;
   __device__ __forceinline__ uint32_t& at(uint32_t c, uint32_t pos) const {
-    uint32_t* p = c == 0 || c == kHeadBits ? a : b;
-    return p[c == 0 || c == 1 ? pos : cap - 1 - pos];
+    return base[(size_t)(c >> 1) * cap + (c & 1 ? cap - 1 - pos : pos)];
   }
 };
 
@@ -1825,26 +1831,47 @@ __global__ void __launch_bounds__(THREADS) k_head_block(Csr g, HeadArcs h,
   if (!kVC) flush_counts<THREADS>(tc, ctr);
 }
 
-// Sign bits of the arcs, one byte per eight: entry e of the group at bit
-// 7 - e (the order in which k_head_bits collects its hits).
-__global__ void __launch_bounds__(256) k_sign_bits(const int8_t* __restrict__ sgn, uint64_t m,
-                                                   const unsigned long long* __restrict__ m_dev,
-                                                   uint8_t* __restrict__ sbits) {
+// The arcs as the bitmap classes stream them: sign bits, one byte per eight
+// arcs (entry e of the group at bit 7 - e, the order in which k_head_bits
+// collects its hits), and the low 16 bits of the heads.
+struct HeadStream {
+  uint8_t* sbits;
+  uint16_t* low;
+};
+
+__global__ void __launch_bounds__(256) k_head_stream(const uint32_t* __restrict__ nbr,
+                                                     const int8_t* __restrict__ sgn, uint64_t m,
+                                                     const unsigned long long* __restrict__ m_dev,
+                                                     HeadStream hs) {
   if (m_dev) m = min(m, (uint64_t)*m_dev);
   const uint64_t groups = (m + 7) / 8;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < groups; i += stride) {
     const uint2 q = reinterpret_cast<const uint2*>(sgn)[i];
+    const uint4 x = reinterpret_cast<const uint4*>(nbr)[2 * i];
+    const uint4 y = reinterpret_cast<const uint4*>(nbr)[2 * i + 1];
     // Sign bits at 7, 15, 23, 31; the multiply gathers them at 31..28.
     const uint32_t a = ((q.x >> 7) & 0x01010101u) * 0x80402010u >> 28;
     const uint32_t b = ((q.y >> 7) & 0x01010101u) * 0x80402010u >> 28;
-    sbits[i] = (uint8_t)((a << 4) | b);
+    hs.sbits[i] = (uint8_t)((a << 4) | b);
+    reinterpret_cast<uint4*>(hs.low)[i] =
+        make_uint4(__byte_perm(x.x, x.y, 0x5410), __byte_perm(x.z, x.w, 0x5410),
+                   __byte_perm(y.x, y.y, 0x5410), __byte_perm(y.z, y.w, 0x5410));
   }
 }
 
+// Eight consecutive heads by one 32-byte load: with two of 16 bytes a lane,
+// each instruction spread over twice the lines it used.
+__device__ __forceinline__ void load8(const uint32_t* __restrict__ p, uint32_t (&x)[8]) {
+  asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]), "=r"(x[4]), "=r"(x[5]),
+                 "=r"(x[6]), "=r"(x[7])
+               : "l"(p));
+}
+
 // Head vertices whose lists fit a bitmap: one CTA per work item from a
-// dynamic queue.  N+(v) is staged as a bitmap over the ranks (mod
-// kBitsWindow), two bits per rank, 16 ranks per 32-bit word: for rank x, the
+// dynamic queue.  N+(v) is staged as a bitmap over the ranks (mod the
+// window), two bits per rank, 16 ranks per 32-bit word: for rank x, the
 // bit at x & 31 says that x is in N+(v) with a positive sign, the bit at
 // (x & 31) ^ 16 that it is with a negative one.  Rotating the word right by x
 // brings the two to bits 0 and 16, so a streamed entry costs one 4-byte
@@ -1867,26 +1894,34 @@ __global__ void __launch_bounds__(256) k_sign_bits(const int8_t* __restrict__ sg
 // off in the step that sets the new ones, a claim's keys are loaded while the
 // claim before is streamed, and small items are claimed in small pieces.
 //
-// RMAT scale 24 (97% of the 41.8 G probes): 37.6 ms, against 78.8 ms of hash
-// probes for the same heads (42.4 ms before the steps of the last
-// paragraph); scale 22: 4.2 G warp instructions against 10.0 G, issue slots
-// 51% used, DRAM at 1.4 TB/s.
-template <int THREADS, class Sink>
-__global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_head_bits(
-    Csr g, HeadArcs h, const uint8_t* __restrict__ sbits, unsigned long long* __restrict__ ctr,
-    Sink sink) {
+// RMAT scale 24 (97% of the 41.8 G probes): 28.8 ms for the two windows,
+// against 78.8 ms of hash probes for the same heads; the short one 1.7 T
+// probes/s.  Bound by
+// the shared-memory pipe (3.2 wavefronts a probe's load, ranks being random
+// over the banks) and, at that scale, DRAM.  One 32-byte load a chunk instead
+// of two of 16 took 3.4 ms off, the short window 1.6, its CTAs of 128
+// threads, ten an SM, instead of 512, two an SM, 3.8 (fewer warps wait at an
+// item's barriers; 256 x 5 was 0.4 slower, 128 x 12 2.3); chunks in flight 1,
+// 3 or 4 instead of 2 were slower.
+//
+// kShort: the heads of the short window, streamed as 16-bit ranks.
+template <int THREADS, bool kShort, class Sink>
+__global__ void __launch_bounds__(THREADS, kShort ? kShortCtas : kBitsCtas) k_head_bits(
+    Csr g, HeadArcs h, HeadStream hs, unsigned long long* __restrict__ ctr, Sink sink) {
+  constexpr uint32_t kClass = kShort ? kHeadShort : kHeadBits;
+  constexpr uint32_t kWords = (kShort ? kShortWindow : kBitsWindow) / 16;
   constexpr bool kVC = Sink::kPerVertex;
   constexpr uint32_t kWarps = THREADS / 32;
   constexpr int U = 2;  // chunks in flight per lane
   constexpr uint32_t kDrainRounds = 255 / (8 * U);  // 8-bit fields, 8 adds a chunk at most
-  extern __shared__ __align__(16) uint32_t bm[];  // kBitsWords
+  extern __shared__ __align__(16) uint32_t bm[];  // kWords
   struct Item {
     uint32_t v, j0, arcs, vb, d;  // arcs 0: no more items
   };
   __shared__ Item s_item[2];
   __shared__ uint32_t s_next;
   const uint32_t lane = lane_id(), le = lanemask_lt() | (1u << lane);
-  const uint32_t cnt = (uint32_t)ctr[C_HEAD_COUNT + kHeadBits];
+  const uint32_t cnt = (uint32_t)ctr[C_HEAD_COUNT + kClass];
   TypeCounts tc;
   uint32_t cur = 0xFFFFFFFFu;  // per-key counts as in k_head_block
   auto flush = [&]() {
@@ -1897,12 +1932,12 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_head_bits(
   };
   // Thread 0: the next work item, by four dependent loads.
   auto fetch = [&](Item& it) {
-    const uint32_t item = (uint32_t)atomicAdd(ctr + C_HEAD_QUEUE + kHeadBits, 1ull);
+    const uint32_t item = (uint32_t)atomicAdd(ctr + C_HEAD_QUEUE + kClass, 1ull);
     it.arcs = 0;
     if (item >= cnt) return;
     uint32_t j1;
-    it.j0 = h.lists.at(kHeadBits, item);
-    h.item(it.j0, kHeadBits, it.v, j1);
+    it.j0 = h.lists.at(kClass, item);
+    h.item(it.j0, kClass, it.v, j1);
     it.arcs = j1 - it.j0;
     it.vb = (uint32_t)g.off[it.v];
     it.d = (uint32_t)g.off[it.v + 1] - it.vb;
@@ -1912,10 +1947,10 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_head_bits(
     for (uint32_t i = threadIdx.x; i < d; i += THREADS) {
       const uint32_t x = g.nbr[vb + i];
       const uint32_t neg = g.sgn[vb + i] < 0;
-      atomicXor(&bm[(x >> 4) & (kBitsWords - 1)], 1u << ((x & 31u) ^ (neg << 4)));
+      atomicXor(&bm[(x >> 4) & (kWords - 1)], 1u << ((x & 31u) ^ (neg << 4)));
     }
   };
-  for (uint32_t i = threadIdx.x; i < kBitsWords; i += THREADS) bm[i] = 0;
+  for (uint32_t i = threadIdx.x; i < kWords; i += THREADS) bm[i] = 0;
   if (threadIdx.x == 0) fetch(s_item[0]);
   __syncthreads();
   uint32_t ovb = 0, od = 0, p = 0;  // the list whose bits are on
@@ -1957,41 +1992,48 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_head_bits(
       const uint32_t b = nb;
       const uint64_t key = nkey;
       nb = take(nkey);  // in flight while this claim is streamed
-      // This lane's in-arc: A' extent [lo, hi), chunks, 8 * (arc negative).
-      uint32_t lo = 0, hi = 0, c = 0;
-      const uint32_t sh = (uint32_t)(key >> 63) << 3;
+      // This lane's in-arc: A' extent [lo, hi), its chunks, and in one word the
+      // masks of its first and last chunk and 8 * (arc negative).
+      uint32_t lo = 0, hi = 1, c = 0;
       if (lane < claim && b + lane < it.arcs) {
         h.extent(key, lo, hi);
         c = ((hi + 7) >> 3) - (lo >> 3);
       }
+      const uint32_t arc = (0xFFu >> (lo & 7)) | ((0xFFu << (7 - ((hi - 1) & 7))) & 0xFFu) << 8 |
+                           (uint32_t)(key >> 63) << 19;
       const uint32_t inc = warp_inclusive_scan(c);
       const uint32_t start = c ? inc - c : 0xFFFFFFFFu;
       const uint32_t cb = (lo >> 3) - start;  // group index = cb + chunk index
       const uint32_t total = __shfl_sync(kFull, inc, 31);
       uint32_t k0 = 0xFFFFFFFFu;  // arcs started before the round, less one
+      // Which of the next 32 chunks start an arc.
+      uint32_t ahead = __reduce_or_sync(kFull, start < 32u ? 1u << start : 0u);
       for (uint32_t base = 0; base < total; base += 32 * U) {
-        uint4 qa[U], qb[U];
-        uint32_t sb[U], vm[U], ash[U];
+        uint32_t q[U][kShort ? 4 : 8], sb[U], vm[U], ash[U];
 #pragma unroll
         for (int u = 0; u < U; u++) {
           const uint32_t w0 = base + 32 * u;
-          const uint32_t rel = start - w0;
-          const uint32_t starts = __reduce_or_sync(kFull, rel < 32u ? 1u << rel : 0u);
+          const uint32_t starts = ahead, rel = start - w0 - 32;
+          ahead = __reduce_or_sync(kFull, rel < 32u ? 1u << rel : 0u);
           const uint32_t k = k0 + __popc(starts & le);
           k0 += __popc(starts);
           const uint32_t ci = __shfl_sync(kFull, cb, k) + w0 + lane;
-          const uint32_t klo = __shfl_sync(kFull, lo, k), khi = __shfl_sync(kFull, hi, k);
-          ash[u] = __shfl_sync(kFull, sh, k);
+          const uint32_t ka = __shfl_sync(kFull, arc, k);
           vm[u] = 0;
           if (w0 + lane < total) {
-            const uint4* src = reinterpret_cast<const uint4*>(g.nbr) + 2ull * ci;
-            qa[u] = src[0];
-            qb[u] = src[1];
-            sb[u] = sbits[ci];
-            const uint32_t g0 = 8 * ci;
-            const uint32_t first = klo > g0 ? klo - g0 : 0u;
-            const uint32_t last = min(khi - g0, 8u);
-            vm[u] = (0xFFu >> first) & (0xFFu << (8u - last));
+            if constexpr (kShort) {
+              const uint4 x = reinterpret_cast<const uint4*>(hs.low)[ci];
+              q[u][0] = x.x, q[u][1] = x.y, q[u][2] = x.z, q[u][3] = x.w;
+            } else {
+              load8(g.nbr + 8ull * ci, q[u]);
+            }
+            sb[u] = hs.sbits[ci];
+            // The chunk is its arc's last if the next one starts another.
+            const bool first = (starts >> lane) & 1u;
+            const bool last = (__funnelshift_r(starts, ahead, 1) >> lane) & 1u;
+            vm[u] = (first ? ka & 0xFFu : 0xFFu) &
+                    (last || w0 + lane + 1 == total ? (ka >> 8) & 0xFFu : 0xFFu);
+            ash[u] = ka >> 16;
           }
         }
 #pragma unroll
@@ -2000,8 +2042,8 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_head_bits(
           uint32_t acc = 0;  // hits: positive in bits 0-7, negative in bits 16-23
 #pragma unroll
           for (uint32_t e = 0; e < 8; e++) {
-            const uint32_t x = e < 4 ? pick4(qa[u], e) : pick4(qb[u], e - 4);
-            const uint32_t w = bm[(x >> 4) & (kBitsWords - 1)];
+            const uint32_t x = !kShort ? q[u][e] : e & 1 ? q[u][e / 2] >> 16 : q[u][e / 2];
+            const uint32_t w = bm[(x >> 4) & (kWords - 1)];
             acc = 2 * acc + (__funnelshift_r(w, w, x) & 0x10001u);
           }
           acc &= vm[u] * 0x10001u;
@@ -2034,7 +2076,7 @@ struct HeadBufs {
   HeadLists lists{};         // the classes' work items
   uint8_t* need = nullptr;   // per tail: it keeps arcs for the tail side
   uint32_t* sort_ws = nullptr;
-  uint8_t* sbits = nullptr;  // sign bits of the arcs
+  HeadStream stream{};       // the arcs as the bitmap classes stream them
 };
 
 HeadBufs head_buffers(stc_ctx* c, const DeviceGraph& g) {
@@ -2046,12 +2088,12 @@ HeadBufs head_buffers(stc_ctx* c, const DeviceGraph& g) {
   // Items: at most one per run (a head with an in-arc and a list) plus one
   // per multiple of the smallest item size.
   const size_t items = (size_t)std::min<uint64_t>(g.n, g.m_fwd) + g.m_fwd / kHeadItemMin + 1;
-  b.lists.a = buffer<uint32_t>(c, B_HEAD_LIST, 2 * items + (g.n + 3) / 4);
-  b.lists.b = b.lists.a + items;
+  b.lists.base = buffer<uint32_t>(c, B_HEAD_LIST, 3 * items + (g.n + 3) / 4);
   b.lists.cap = (uint32_t)items;
-  b.need = reinterpret_cast<uint8_t*>(b.lists.b + items);
+  b.need = reinterpret_cast<uint8_t*>(b.lists.base + 3 * items);
   b.sort_ws = buffer<uint32_t>(c, B_SORT_WS, sort_workspace_words(g.m_fwd));
-  b.sbits = buffer<uint8_t>(c, B_SBITS, (g.m_fwd + 7) / 8);
+  b.stream.low = buffer<uint16_t>(c, B_HEAD_LOW, (g.m_fwd + 7) / 8 * 8);
+  b.stream.sbits = buffer<uint8_t>(c, B_SBITS, (g.m_fwd + 7) / 8);
   return b;
 }
 
@@ -2078,9 +2120,9 @@ void prepare_head(const Tuning& tu) {
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sl));
   });
   if constexpr (!kTime)
-    STC_CUDA(cudaFuncSetAttribute(k_head_bits<kBitsThreads, Sink>,
+    STC_CUDA(cudaFuncSetAttribute(k_head_bits<kBitsThreads, false, Sink>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)(kBitsWords * sizeof(uint32_t))));
+                                  (int)(kBitsWindow / 4)));
 }
 
 // The head-side pass is enqueued on `st` (no host synchronisation) in two
@@ -2125,13 +2167,16 @@ void enqueue_head(cudaStream_t st, const Csr& csr, const uint32_t* asrc, uint64_
                                                                     b.lists, end, ctr);
   const HeadArcs h{sorted, b.aend, end, asrc, fmt, b.lists};
   launches += 1;
+  const bool wide = kTime || gbase || n > kShortWindow;
   if constexpr (!kTime) {
     if (class_mask & 4u) {
-      k_sign_bits<<<kSMs * 8, 256, 0, st>>>(csr.sgn, m, m_dev, b.sbits);
-      k_head_bits<kBitsThreads, Sink>
-          <<<kSMs * (1024 / kBitsThreads), kBitsThreads, kBitsWords * sizeof(uint32_t), st>>>(
-              csr, h, b.sbits, ctr, sink);
-      launches += 2;
+      k_head_stream<<<kSMs * 8, 256, 0, st>>>(csr.nbr, csr.sgn, m, m_dev, b.stream);
+      k_head_bits<kShortThreads, true, Sink>
+          <<<kSMs * kShortCtas, kShortThreads, kShortWindow / 4, st>>>(csr, h, b.stream, ctr, sink);
+      if (wide)
+        k_head_bits<kBitsThreads, false, Sink>
+            <<<kSMs * kBitsCtas, kBitsThreads, kBitsWindow / 4, st>>>(csr, h, b.stream, ctr, sink);
+      launches += wide ? 3 : 2;
     }
   }
   // With every rank inside the window the bitmap takes all lists longer than
@@ -2301,7 +2346,7 @@ void enqueue_persistent(cudaStream_t st, const Csr& csr, const ClassBounds& cb, 
 // Identity of a captured persistent sequence: every pointer and size its
 // kernels were given.
 struct PersistentKey {
-  const void* p[19];
+  const void* p[20];
   uint64_t v[6];
 };
 
@@ -2331,8 +2376,9 @@ void count_persistent(stc_ctx* c, const Csr& csr, const ClassBounds& cb, uint32_
   }
   PersistentKey key{};
   const HeadBufs hb = hp.bufs ? *hp.bufs : HeadBufs{};
-  const void* ptrs[19] = {csr.off, csr.nbr, csr.sgn, csr.verts, lists, plan, ctr, d_tables, s0,
-                          hp.asrc, hb.keys, hb.alt, hb.aend, hb.runs, hb.lists.a, hp.fdeg, csr.nkey, hb.sbits, hp.gbase};
+  const void* ptrs[20] = {csr.off, csr.nbr, csr.sgn, csr.verts, lists, plan, ctr, d_tables, s0,
+                          hp.asrc, hb.keys, hb.alt, hb.aend, hb.runs, hb.lists.base, hp.fdeg, csr.nkey, hb.stream.sbits, hp.gbase,
+                          hb.stream.low};
   memcpy(key.p, ptrs, sizeof(ptrs));
   key.v[0] = csr.n;
   key.v[1] = cb.tiny_max;

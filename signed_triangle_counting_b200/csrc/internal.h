@@ -48,7 +48,8 @@ enum BufId {
   B_HEAD_RUNS,                    // head-side pass: end of each head's in-arc run (n)
   B_HEAD_LIST,                    // head-side pass: work items by class, flags per tail
   B_NKEY,                         // arcs: head << 1 | negative (m + 8)
-  B_SBITS,                        // arcs: sign bits, one byte per 8 arcs (the head bitmap's stream)
+  B_SBITS,                        // arcs: sign bits, one byte per 8 arcs (the head bitmaps' stream)
+  B_HEAD_LOW,                     // arcs: low 16 bits of the heads (the same)
   B_RELABEL,                      // ids >= 2^31 - 1: the edges relabelled to dense ids (2 m)
   B_HUBS,                         // ids with very many edges (totals path)
   B_DISTINCT,                     // ids >= 2^31 - 1: the sorted distinct ids
@@ -78,9 +79,9 @@ enum CounterSlot {
   C_BATCH_MU = 33,             // capped batch build: unique edges (= arcs)
   C_OVERFLOW = 34,             // capped batch build: a capacity was exceeded (results void)
   C_HEAD_NKEYS = 35,           // head-side pass: keys (HEAD arcs) appended,
-  C_HEAD_COUNT = 36,           // work items per class (4 slots)
-  C_HEAD_QUEUE = 40,           // and the classes' work queues (4 slots)
-  C_SLOTS = 44
+  C_HEAD_COUNT = 36,           // work items per class (5 slots)
+  C_HEAD_QUEUE = 41,           // and the classes' work queues (5 slots)
+  C_SLOTS = 46
 };
 
 // Values of the device error word: 1 = malformed forward CSR,

@@ -1,7 +1,8 @@
-"""The head side's bitmap class (heads with more than 128 out-neighbours whose
-later ranks span at most 2^18): extents at every chunk remainder, lists at the
-class edges, several graphs in one union, and ranks on both sides of the
-window, against the oracle or the tail side's strategies."""
+"""The head side's bitmap classes (heads with more than 32 out-neighbours whose
+later ranks span at most 2^16, or more than 128 and at most 2^18): extents at
+every chunk remainder, lists at the class edges, several graphs in one union,
+and ranks on both sides of both windows, against the oracle or the tail
+side's strategies."""
 import numpy as np
 import pytest
 
@@ -25,7 +26,7 @@ def clique_with_fringe(k, fringe, seed):
     return src, dst, np.where(h % 5 < 3, 1, -1).astype(np.int8)
 
 
-@pytest.mark.parametrize("k,fringe", [(129, 0), (130, 1), (131, 5), (137, 64), (160, 333),
+@pytest.mark.parametrize("k,fringe", [(33, 0), (34, 3), (35, 40), (66, 2), (129, 0), (130, 1), (131, 5), (137, 64), (160, 333),
                                       (257, 2), (1030, 7), (1300, 1111)])
 def test_clique_sizes(ctx, k, fringe):
     g = clique_with_fringe(k, fringe, k)
@@ -43,10 +44,10 @@ def test_union_of_graphs(ctx):
         assert [c.as_tuple() for c in got] == want
 
 
-def test_both_sides_of_the_window(ctx):
+def test_both_sides_of_the_windows(ctx):
     import torch
     # Uniform random: out-degrees around 140 at every rank, and 2^18 + 20,000
-    # vertices, so heads lie inside and below the window.
+    # vertices, so heads lie inside and below the windows.
     n, m = (1 << 18) + 20_000, 40_000_000
     gen = torch.Generator(device="cuda").manual_seed(5)
     src, dst = (torch.randint(0, n, (m,), dtype=torch.int32, device="cuda", generator=gen)
