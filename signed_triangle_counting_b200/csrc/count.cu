@@ -485,14 +485,24 @@ __device__ __forceinline__ void process_keyed_chunk8(const StageMem& m, const Ge
   }
 }
 
+// Adds a chunk's packed counts (8-bit fields) to an arc's two words of 16-bit
+// fields.
+__device__ __forceinline__ void add_to_arc(uint32_t p, uint32_t* w0, uint32_t* w1) {
+  const uint32_t a = (p & 0xFFu) | ((p << 8) & 0xFF0000u);
+  const uint32_t b = ((p >> 16) & 0xFFu) | ((p >> 8) & 0xFF0000u);
+  if (a) atomicAdd(w0, a);
+  if (b) atomicAdd(w1, b);
+}
+
 // The head side's stream: the staged in-arcs' A' extents of signed heads
 // (g.nkey) as one sequence of aligned 8-entry (32-byte) chunks, shared out
 // as in stream_pass (warp shares, lanes on consecutive chunks, the last
 // eighth claimed from `next`).  A lane loads a chunk with two 16-byte
 // loads, UK chunks per round, and the cursor, mask and branch work per
 // chunk is spread over eight keys instead of four.  pre[] counts 8-entry
-// chunks (block_chunk_scan / warp_chunk_scan with kWide).
-template <int UK>
+// chunks (block_chunk_scan / warp_chunk_scan with kWide).  kArc: each arc's
+// counts go to its words in m.a and m.sp (zero on entry) instead of tc.
+template <int UK, bool kArc>
 __device__ __forceinline__ void stream_pass_keyed(const Csr& g, const StageMem& m, uint32_t d,
                                                   uint32_t warp, uint32_t warps, uint32_t lane,
                                                   const Geo& geo, TypeCounts& tc,
@@ -531,7 +541,7 @@ __device__ __forceinline__ void stream_pass_keyed(const Csr& g, const StageMem& 
       }
       for (uint32_t base = seg_begin; base < seg_end; base += 32 * UK) {
         uint4 qa[UK], qb[UK];
-        uint32_t vm[UK], snuv[UK];
+        uint32_t vm[UK], snuv[UK], sk[UK];
 #pragma unroll
         for (int u = 0; u < UK; u++) {
           const uint32_t c = base + 32 * u + lane;
@@ -548,11 +558,18 @@ __device__ __forceinline__ void stream_pass_keyed(const Csr& g, const StageMem& 
             qb[u] = src[2 * ci + 1];
             vm[u] = (c == pk ? mf : 0xFFu) & (c + 1 == pk1 ? ml : 0xFFu);
             snuv[u] = anuv;
+            sk[u] = k;
           }
         }
 #pragma unroll
-        for (int u = 0; u < UK; u++)
-          if (vm[u]) process_keyed_chunk8(m, geo, qa[u], qb[u], vm[u], snuv[u], p8);
+        for (int u = 0; u < UK; u++) {
+          if (!vm[u]) continue;
+          process_keyed_chunk8(m, geo, qa[u], qb[u], vm[u], snuv[u], p8);
+          if (kArc) {
+            add_to_arc(p8.w, m.a + sk[u], m.sp + sk[u]);
+            p8.w = 0;
+          }
+        }
         if (++rounds == kDrainRounds) {
           p8.drain(tc);
           rounds = 0;
@@ -776,30 +793,35 @@ __device__ __forceinline__ void flush_counts(const TypeCounts& tc, unsigned long
 }
 
 // Where per-vertex totals go when a kernel reports per vertex.
+// kKeyed: the head side adds up the items of one key (sink.key(head)) and
+// hands them over together; kPerArc: it hands over each in-arc's counts, which
+// belong to the arc's tail.
 struct TotalSink {  // only the four global counters
-  static constexpr bool kPerVertex = false;
+  static constexpr bool kPerVertex = false, kKeyed = false, kPerArc = false;
   __device__ void put(uint32_t, const unsigned long long*) const {}
-  __device__ uint32_t key(uint32_t) const { return 0; }
-  __device__ void put_key(uint32_t, const unsigned long long*) const {}
 };
 struct VertexSink {  // per-source counts by original id: vcounts[4 * id + type]
-  static constexpr bool kPerVertex = true;
+  static constexpr bool kPerVertex = true, kKeyed = false, kPerArc = true;
   unsigned long long* vcounts;
   const uint32_t* verts;
   __device__ void put(uint32_t u, const unsigned long long* c) const {
 #pragma unroll
     for (int k = 0; k < 4; k++) vcounts[4ull * verts[u] + (3 - k)] = c[k];
   }
-  // Keyed form (the head side adds up the items of one key): the vertex.
-  __device__ uint32_t key(uint32_t u) const { return u; }
-  __device__ void put_key(uint32_t u, const unsigned long long* c) const {
-#pragma unroll
-    for (int k = 0; k < 4; k++)
-      if (c[k]) atomicAdd(vcounts + 4ull * verts[u] + (3 - k), c[k]);
+  // The head side's counts of one arc with tail u, added to those the tail
+  // side stored (its kernels run first): fewer than 2^16 of each number of
+  // negative edges, 0 and 1 in w0, 2 and 3 in w1.
+  __device__ void add_arc(uint32_t u, uint32_t w0, uint32_t w1) const {
+    if ((w0 | w1) == 0) return;
+    unsigned long long* c = vcounts + 4ull * verts[u];
+    if (w0 & 0xFFFFu) atomicAdd(c + 3, (unsigned long long)(w0 & 0xFFFFu));
+    if (w0 >> 16) atomicAdd(c + 2, (unsigned long long)(w0 >> 16));
+    if (w1 & 0xFFFFu) atomicAdd(c + 1, (unsigned long long)(w1 & 0xFFFFu));
+    if (w1 >> 16) atomicAdd(c + 0, (unsigned long long)(w1 >> 16));
   }
 };
 struct GraphSink {  // per-graph counts of a batch: gcounts[4 * graph + type]
-  static constexpr bool kPerVertex = true;
+  static constexpr bool kPerVertex = true, kKeyed = true, kPerArc = false;
   unsigned long long* gcounts;
   const uint64_t* gbase;  // G + 1 rank boundaries (graphs are contiguous in rank space)
   uint32_t G;
@@ -1646,7 +1668,7 @@ __device__ __forceinline__ void stage_hash(const Csr& g, uint64_t vb, uint32_t d
 }
 
 // In-arcs [j0, j0 + tn) of a head vertex as the arcs of the staged tile.
-template <int TS, class Sync>
+template <int TS, bool kArc, class Sync>
 __device__ __forceinline__ void stage_in_arcs(const Csr& g, const HeadArcs& h, uint32_t j0,
                                               uint32_t tn, uint32_t t, const StageMem& m,
                                               Sync sync) {
@@ -1655,6 +1677,7 @@ __device__ __forceinline__ void stage_in_arcs(const Csr& g, const HeadArcs& h, u
     h.extent(key, m.lo[k], m.hi[k]);
     m.s[k] = (key >> 63) ? (int8_t)-1 : (int8_t)1;
     m.st[k] = STC_STRATEGY_HASH;
+    if (kArc) m.a[k] = m.sp[k] = 0;
   }
   sync();
 }
@@ -1690,7 +1713,7 @@ template <class Sink, bool kTime, int U>
 __global__ void __launch_bounds__(256) k_head_warp(Csr g, HeadArcs h,
                                                    unsigned long long* __restrict__ ctr, Sink sink,
                                                    ArcTimes at, uint32_t hf) {
-  constexpr bool kVC = Sink::kPerVertex;
+  constexpr bool kVC = Sink::kKeyed, kArc = Sink::kPerArc;
   constexpr int kWarps = 8;
   __shared__ __align__(16) unsigned char smem[kWarps * kWarpStageBytes];
   const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
@@ -1702,7 +1725,8 @@ __global__ void __launch_bounds__(256) k_head_warp(Csr g, HeadArcs h,
   // and handed to the sink once, when the key changes.
   uint32_t cur = 0xFFFFFFFFu;
   auto flush = [&]() {
-    if (kVC && cur != 0xFFFFFFFFu) {
+    if constexpr (kVC) {
+      if (cur == 0xFFFFFFFFu) return;
       unsigned long long s[4];
 #pragma unroll
       for (int k = 0; k < 4; k++) s[k] = warp_sum(tc.c[k]);
@@ -1724,7 +1748,7 @@ __global__ void __launch_bounds__(256) k_head_warp(Csr g, HeadArcs h,
       if (lane == 0) atomicExch(ctr + C_ERROR, kErrStageCapacity);
       continue;
     }
-    if (kVC) {
+    if constexpr (kVC) {
       const uint32_t key = sink.key(v);
       if (key != cur) {
         flush();
@@ -1737,7 +1761,7 @@ __global__ void __launch_bounds__(256) k_head_warp(Csr g, HeadArcs h,
     PackedCounts pc;
     for (uint32_t j0 = j00; j0 < j1; j0 += kWarpCap) {
       const uint32_t tn = min(kWarpCap, j1 - j0);
-      stage_in_arcs<32>(g, h, j0, tn, lane, m, WarpSync{});
+      stage_in_arcs<32, kArc>(g, h, j0, tn, lane, m, WarpSync{});
       if (kTime) {
         timed_head_pass(g, h, m, tn, d, 0, 1, lane, geo, pc, out, at);
       } else {
@@ -1745,15 +1769,20 @@ __global__ void __launch_bounds__(256) k_head_warp(Csr g, HeadArcs h,
         // U / 2 chunks of 8 entries: U 16-byte loads in flight per lane, as
         // in the tail side (more raise the registers above 64 and cost
         // this kernel a CTA per SM).
-        stream_pass_keyed<(U > 1 ? U / 2 : 1)>(g, m, tn, 0, 1, lane, geo, out, nullptr);
+        stream_pass_keyed<(U > 1 ? U / 2 : 1), kArc>(g, m, tn, 0, 1, lane, geo, out, nullptr);
       }
       __syncwarp();
+      if constexpr (kArc) {
+        for (uint32_t k = lane; k < tn; k += 32)
+          sink.add_arc(h.asrc[m.lo[k] - 1], m.a[k], m.sp[k]);
+        __syncwarp();
+      }
     }
     pc.drain(out);
     __syncwarp();
   }
   flush();
-  if (!kVC) flush_counts<256>(tc, ctr);
+  if (!Sink::kPerVertex) flush_counts<256>(tc, ctr);
 }
 
 // Head vertices of the block and large classes: one CTA per vertex from a
@@ -1765,7 +1794,7 @@ __global__ void __launch_bounds__(THREADS) k_head_block(Csr g, HeadArcs h,
                                                         uint32_t hf,
                                                         unsigned long long* __restrict__ ctr,
                                                         Sink sink, ArcTimes at) {
-  constexpr bool kVC = Sink::kPerVertex;
+  constexpr bool kVC = Sink::kKeyed, kArc = Sink::kPerArc;
   constexpr uint32_t kWarps = THREADS / 32;
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ uint32_t scan_tmp[THREADS / 32 + 2];
@@ -1779,7 +1808,8 @@ __global__ void __launch_bounds__(THREADS) k_head_block(Csr g, HeadArcs h,
   // Per-key counts as in k_head_warp, reduced over the CTA at a key change.
   uint32_t cur = 0xFFFFFFFFu;
   auto flush = [&]() {
-    if (kVC && cur != 0xFFFFFFFFu) {
+    if constexpr (kVC) {
+      if (cur == 0xFFFFFFFFu) return;
       block_key_flush<THREADS>(tc, cur, sink);
       tc = TypeCounts{};
     }
@@ -1799,7 +1829,7 @@ __global__ void __launch_bounds__(THREADS) k_head_block(Csr g, HeadArcs h,
       if (threadIdx.x == 0) atomicExch(ctr + C_ERROR, kErrStageCapacity);
       continue;
     }
-    if (kVC) {
+    if constexpr (kVC) {
       const uint32_t key = sink.key(v);  // uniform over the CTA
       if (key != cur) {
         flush();
@@ -1815,20 +1845,25 @@ __global__ void __launch_bounds__(THREADS) k_head_block(Csr g, HeadArcs h,
       // Every warp left the previous tile's stream (barrier at its end), and
       // the staging below passes a barrier before the counter is used.
       if (threadIdx.x == 0) *next = 0;
-      stage_in_arcs<THREADS>(g, h, j0, tn, threadIdx.x, m, BlockSync{});
+      stage_in_arcs<THREADS, kArc>(g, h, j0, tn, threadIdx.x, m, BlockSync{});
       if (kTime) {
         timed_head_pass(g, h, m, tn, d, w, kWarps, lane, geo, pc, out, at);
       } else {
         block_chunk_scan<THREADS, true>(m, tn, scan_tmp);
         // U chunks of 8 entries: 2 U 16-byte loads in flight per lane.
-        stream_pass_keyed<U>(g, m, tn, w, kWarps, lane, geo, out, next);
+        stream_pass_keyed<U, kArc>(g, m, tn, w, kWarps, lane, geo, out, next);
       }
       __syncthreads();
+      if constexpr (kArc) {
+        for (uint32_t k = threadIdx.x; k < tn; k += THREADS)
+          sink.add_arc(h.asrc[m.lo[k] - 1], m.a[k], m.sp[k]);
+        __syncthreads();
+      }
     }
     pc.drain(out);
   }
   flush();
-  if (!kVC) flush_counts<THREADS>(tc, ctr);
+  if (!Sink::kPerVertex) flush_counts<THREADS>(tc, ctr);
 }
 
 // The arcs as the bitmap classes stream them: sign bits, one byte per eight
@@ -1910,7 +1945,7 @@ __global__ void __launch_bounds__(THREADS, kShort ? kShortCtas : kBitsCtas) k_he
     Csr g, HeadArcs h, HeadStream hs, unsigned long long* __restrict__ ctr, Sink sink) {
   constexpr uint32_t kClass = kShort ? kHeadShort : kHeadBits;
   constexpr uint32_t kWords = (kShort ? kShortWindow : kBitsWindow) / 16;
-  constexpr bool kVC = Sink::kPerVertex;
+  constexpr bool kVC = Sink::kKeyed, kArc = Sink::kPerArc;
   constexpr uint32_t kWarps = THREADS / 32;
   constexpr int U = 2;  // chunks in flight per lane
   constexpr uint32_t kDrainRounds = 255 / (8 * U);  // 8-bit fields, 8 adds a chunk at most
@@ -1920,12 +1955,14 @@ __global__ void __launch_bounds__(THREADS, kShort ? kShortCtas : kBitsCtas) k_he
   };
   __shared__ Item s_item[2];
   __shared__ uint32_t s_next;
+  __shared__ uint32_t arc_counts[kArc ? kWarps : 1][2][32];  // of a warp's 32 in-arcs
   const uint32_t lane = lane_id(), le = lanemask_lt() | (1u << lane);
   const uint32_t cnt = (uint32_t)ctr[C_HEAD_COUNT + kClass];
   TypeCounts tc;
   uint32_t cur = 0xFFFFFFFFu;  // per-key counts as in k_head_block
   auto flush = [&]() {
-    if (kVC && cur != 0xFFFFFFFFu) {
+    if constexpr (kVC) {
+      if (cur == 0xFFFFFFFFu) return;
       block_key_flush<THREADS>(tc, cur, sink);
       tc = TypeCounts{};
     }
@@ -1957,7 +1994,7 @@ __global__ void __launch_bounds__(THREADS, kShort ? kShortCtas : kBitsCtas) k_he
   while (true) {
     const Item it = s_item[p];
     if (it.arcs == 0) break;
-    if (kVC) {
+    if constexpr (kVC) {
       const uint32_t key = sink.key(it.v);  // uniform over the CTA
       if (key != cur) {
         flush();
@@ -2006,10 +2043,15 @@ __global__ void __launch_bounds__(THREADS, kShort ? kShortCtas : kBitsCtas) k_he
       const uint32_t cb = (lo >> 3) - start;  // group index = cb + chunk index
       const uint32_t total = __shfl_sync(kFull, inc, 31);
       uint32_t k0 = 0xFFFFFFFFu;  // arcs started before the round, less one
+      uint32_t* ac = arc_counts[kArc ? threadIdx.x >> 5 : 0][0];
+      if (kArc) {
+        ac[lane] = ac[32 + lane] = 0;
+        __syncwarp();
+      }
       // Which of the next 32 chunks start an arc.
       uint32_t ahead = __reduce_or_sync(kFull, start < 32u ? 1u << start : 0u);
       for (uint32_t base = 0; base < total; base += 32 * U) {
-        uint32_t q[U][kShort ? 4 : 8], sb[U], vm[U], ash[U];
+        uint32_t q[U][kShort ? 4 : 8], sb[U], vm[U], ash[U], ak[U];
 #pragma unroll
         for (int u = 0; u < U; u++) {
           const uint32_t w0 = base + 32 * u;
@@ -2034,6 +2076,7 @@ __global__ void __launch_bounds__(THREADS, kShort ? kShortCtas : kBitsCtas) k_he
             vm[u] = (first ? ka & 0xFFu : 0xFFu) &
                     (last || w0 + lane + 1 == total ? (ka >> 8) & 0xFFu : 0xFFu);
             ash[u] = ka >> 16;
+            ak[u] = k;
           }
         }
 #pragma unroll
@@ -2051,12 +2094,19 @@ __global__ void __launch_bounds__(THREADS, kShort ? kShortCtas : kBitsCtas) k_he
           const uint32_t e2 = __popc(neg >> 16);
           const uint32_t e0 = __popc((acc ^ neg) & 0xFFFFu);
           const uint32_t e1 = __popc(acc) - e0 - e2;
-          p8.w += (e0 + (e1 << 8) + (e2 << 16)) << ash[u];
+          const uint32_t add = (e0 + (e1 << 8) + (e2 << 16)) << ash[u];
+          if (kArc) add_to_arc(add, ac + ak[u], ac + 32 + ak[u]);
+          else p8.w += add;
         }
-        if (++rounds == kDrainRounds) {
+        if (!kArc && ++rounds == kDrainRounds) {
           p8.drain(tc);
           rounds = 0;
         }
+      }
+      if constexpr (kArc) {
+        __syncwarp();
+        if (c) sink.add_arc(h.asrc[h.fmt.arc(key)], ac[lane], ac[32 + lane]);
+        __syncwarp();
       }
     }
     p8.drain(tc);
@@ -2064,7 +2114,7 @@ __global__ void __launch_bounds__(THREADS, kShort ? kShortCtas : kBitsCtas) k_he
     __syncthreads();
   }
   flush();
-  if (!kVC) flush_counts<THREADS>(tc, ctr);
+  if (!Sink::kPerVertex) flush_counts<THREADS>(tc, ctr);
 }
 
 // Device buffers of the head-side pass (allocated before any capture).
@@ -2545,7 +2595,7 @@ void shard_range(stc_ctx* c, const DeviceGraph& g, uint32_t shard, uint32_t shar
 // when B is at least 16x longer than A', MERGE when both are short, HASH
 // otherwise (the giant class, which stages no hash, merges instead of
 // hashing).  Without `head`, the tail-side table of the first version (no
-// HEAD cells), which per-vertex counts and the no-allocation path use.
+// HEAD cells), which the no-allocation path uses.
 void fixed_dispatch_tables(uint8_t* out, bool head) {
   for (int t = 0; t < kTableClasses; t++)
     for (int a = 0; a < 16; a++)
@@ -2560,24 +2610,24 @@ void fixed_dispatch_tables(uint8_t* out, bool head) {
 }
 
 namespace {
-// Cached tables in B_DISPATCH_FIXED: the fixed tables with and without HEAD,
-// and the forced-HEAD tables (HEAD wherever it applies, HASH elsewhere).
-enum { kFixedHead = 0, kFixedNoHead = 1, kForcedHead = 2, kCachedTables = 3 };
+// Cached tables in B_DISPATCH_FIXED: the fixed tables, and the forced-HEAD
+// tables (HEAD wherever it applies, HASH elsewhere).
+enum { kFixedHead = 0, kForcedHead = 1, kCachedTables = 2 };
 }  // namespace
 
 // Device copy of the dispatch tables a call uses: a forced strategy fills
 // every cell (HEAD only the cells where it applies); otherwise the learned
 // tables when the context holds a model and the call asks for them, else
-// the fixed ones.  Per-vertex counts take tables without HEAD (the head
-// side reports per graph, not per source vertex).  `uses_head` (optional)
+// the fixed ones.  Per-vertex counts take the fixed tables, and no forced HEAD
+// (the head side keeps an arc's counts in 16 bits, which |A'| <= 4095, as in
+// the fixed tables' HEAD cells, cannot exceed).  `uses_head` (optional)
 // receives whether the tables send any cell to the head side.
 const uint8_t* dispatch_tables(stc_ctx* c, const CountConfig& cfg, bool* uses_head) {
-  const bool head_ok = cfg.vertex_counts == nullptr;
+  const bool totals = cfg.vertex_counts == nullptr;
   if (uses_head) *uses_head = false;
   if (!c->fixed_ready) {
     uint8_t h[kCachedTables * kTableBytes];
     fixed_dispatch_tables(h + kFixedHead * kTableBytes, true);
-    fixed_dispatch_tables(h + kFixedNoHead * kTableBytes, false);
     for (size_t i = 0; i < kTableBytes; i++)
       h[kForcedHead * kTableBytes + i] =
           (i & 15) <= 12 ? (uint8_t)STC_STRATEGY_HEAD : (uint8_t)STC_STRATEGY_HASH;
@@ -2588,8 +2638,8 @@ const uint8_t* dispatch_tables(stc_ctx* c, const CountConfig& cfg, bool* uses_he
   }
   const uint8_t* cached = buffer<uint8_t>(c, B_DISPATCH_FIXED, kCachedTables * kTableBytes);
   if (cfg.strategy == STC_STRATEGY_HEAD) {
-    if (uses_head) *uses_head = head_ok;
-    if (head_ok) return cached + kForcedHead * kTableBytes;
+    if (uses_head) *uses_head = totals;
+    if (totals) return cached + kForcedHead * kTableBytes;
     uint8_t* t = buffer<uint8_t>(c, B_WORK2, kTableBytes);
     STC_CUDA(cudaMemsetAsync(t, (int)STC_STRATEGY_HASH, kTableBytes, c->stream));
     return t;
@@ -2599,8 +2649,7 @@ const uint8_t* dispatch_tables(stc_ctx* c, const CountConfig& cfg, bool* uses_he
     STC_CUDA(cudaMemsetAsync(t, (int)cfg.strategy, kTableBytes, c->stream));
     return t;
   }
-  if (!head_ok) return cached + kFixedNoHead * kTableBytes;
-  if (cfg.dispatch == STC_DISPATCH_LEARNED && c->model_loaded) {
+  if (totals && cfg.dispatch == STC_DISPATCH_LEARNED && c->model_loaded) {
     if (uses_head) *uses_head = c->learned_uses_head;
     return buffer<uint8_t>(c, B_DISPATCH, kTableBytes);
   }
@@ -2630,8 +2679,7 @@ void count_triangles(stc_ctx* c, const DeviceGraph& gin, const CountConfig& cfg)
   unsigned long long* ctr = (unsigned long long*)counters(c);
   bool uses_head = false;
   const uint8_t* d_table = dispatch_tables(c, cfg, &uses_head);
-  // The head-side pass runs when the tables send arcs there (never for
-  // per-vertex counts, whose tables have no HEAD cells).
+  // The head-side pass runs when the tables send arcs there.
   const bool head = uses_head && (cfg.class_mask & 0x20u) && g.asrc != nullptr &&
                     g.nkey != nullptr && g.n >= 2;
   HeadBufs hb;

@@ -58,3 +58,21 @@ def test_both_sides_of_the_windows(ctx):
     assert sum(want) > 3_000_000
     for strategy in ("auto", "head"):
         assert ctx.count(src, dst, sign, strategy=strategy).as_tuple() == want
+
+
+@pytest.mark.parametrize("k,fringe", [(9, 4), (33, 0), (36, 7), (130, 1), (140, 200), (300, 33)])
+def test_vertex_counts_of_cliques(ctx, k, fringe):
+    g = clique_with_fringe(k, fringe, 3 * k)
+    want = oracle.ForwardCSR(*g).vertex_counts()
+    for persistent in (False, True):
+        np.testing.assert_array_equal(ctx.vertex_counts(*g, persistent=persistent), want)
+
+
+def test_vertex_counts_both_sides_of_the_windows(ctx):
+    rng = np.random.default_rng(11)
+    n, m = (1 << 18) + 20_000, 36_000_000
+    src, dst = (rng.integers(0, n, m, dtype=np.uint32) for _ in range(2))
+    sign = (((src ^ dst) & 7) < 3).astype(np.int8) * -2 + 1
+    want = ctx.vertex_counts(src, dst, sign, strategy="hash")
+    assert want.sum() > 2_000_000
+    np.testing.assert_array_equal(ctx.vertex_counts(src, dst, sign), want)
