@@ -139,7 +139,20 @@ class _EdgeBuffers:
             pass
 
 
-def _view(ptr, ctype, m: int, owner: _EdgeBuffers, dtype) -> np.ndarray:
+class _CsrBuffers:
+    """Owns the five malloc'd arrays of one stc_forward_csr, as _EdgeBuffers."""
+
+    def __init__(self, csr: _capi.stc_forward_csr):
+        self._csr = csr
+
+    def __del__(self):
+        try:
+            lib().stc_free_forward_csr(C.byref(self._csr))
+        except Exception:
+            pass
+
+
+def _view(ptr, ctype, m: int, owner, dtype) -> np.ndarray:
     arr = (ctype * m).from_address(C.cast(ptr, C.c_void_p).value)
     arr._owner = owner  # the ctypes array, numpy's base, keeps the owner alive
     return np.frombuffer(arr, dtype=dtype)
@@ -326,17 +339,18 @@ class Context:
         o = self._opts()
         _check(lib().stc_build_forward_csr(self._h, _ptr(src), _ptr(dst), _ptr(sign), len(src),
                                            C.byref(o), C.byref(out)), self._h)
-        try:
-            n, m = out.n, out.m
-            return ForwardCSR(
-                n=n, m=m,
-                offsets=np.ctypeslib.as_array(out.offsets, (n + 1,)).copy(),
-                edges=np.ctypeslib.as_array(out.edges, (m,)).copy() if m else np.zeros(0, np.uint32),
-                signs=np.ctypeslib.as_array(out.signs, (m,)).copy() if m else np.zeros(0, np.int8),
-                fdeg=np.ctypeslib.as_array(out.fdeg, (n,)).copy() if n else np.zeros(0, np.uint32),
-                rank=np.ctypeslib.as_array(out.rank, (n,)).copy() if n else np.zeros(0, np.uint32))
-        finally:
-            lib().stc_free_forward_csr(C.byref(out))
+        n, m = out.n, out.m
+        owner = _CsrBuffers(out)  # the arrays go with their last view
+
+        def view(ptr, ctype, count, dtype):
+            return _view(ptr, ctype, count, owner, dtype) if count else np.zeros(0, dtype)
+
+        return ForwardCSR(
+            n=n, m=m, offsets=view(out.offsets, C.c_uint64, n + 1, np.uint64),
+            edges=view(out.edges, C.c_uint32, m, np.uint32),
+            signs=view(out.signs, C.c_int8, m, np.int8),
+            fdeg=view(out.fdeg, C.c_uint32, n, np.uint32),
+            rank=view(out.rank, C.c_uint32, n, np.uint32))
 
     def count_triangles(self, csr: ForwardCSR, *, strategy="auto", dispatch="fixed") -> GlobalTriCounts:
         """count_triangles (tc_serial.cpp:138-170) over a reference-layout CSR."""
@@ -363,7 +377,7 @@ class Context:
         n_out = C.c_uint32()
         o = self._opts(strategy, persistent=persistent)
         n_bound = int(max(src.max(initial=0), dst.max(initial=0))) + 1 if len(src) else 0
-        buf = np.zeros(4 * max(n_bound, 1), np.uint64)
+        buf = np.empty(4 * max(n_bound, 1), np.uint64)
         _check(lib().stc_vertex_counts(self._h, _ptr(src), _ptr(dst), _ptr(sign), len(src),
                                        C.byref(o), buf.ctypes.data_as(_capi.u64p), len(buf),
                                        C.byref(n_out)), self._h)

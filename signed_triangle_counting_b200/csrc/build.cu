@@ -1442,28 +1442,19 @@ void export_forward_csr(stc_ctx* c, const DeviceGraph& g, stc_forward_csr* out) 
   STC_CUDA(cudaGetLastError());
   out->n = n;
   out->m = mu;
-  out->offsets = (uint64_t*)malloc(((size_t)n + 1) * sizeof(uint64_t));
-  out->edges = (uint32_t*)malloc((mu ? mu : 1) * sizeof(uint32_t));
-  out->signs = (int8_t*)malloc(mu ? mu : 1);
-  out->fdeg = (uint32_t*)malloc((n ? n : 1) * sizeof(uint32_t));
-  out->rank = (uint32_t*)malloc((n ? n : 1) * sizeof(uint32_t));
+  out->offsets = (uint64_t*)host_alloc(((size_t)n + 1) * sizeof(uint64_t));
+  out->edges = (uint32_t*)host_alloc(mu * sizeof(uint32_t));
+  out->signs = (int8_t*)host_alloc(mu);
+  out->fdeg = (uint32_t*)host_alloc((size_t)n * sizeof(uint32_t));
+  out->rank = (uint32_t*)host_alloc((size_t)n * sizeof(uint32_t));
   if (!out->offsets || !out->edges || !out->signs || !out->fdeg || !out->rank) {
     stc_free_forward_csr(out);
     fail(STC_ERR_OUT_OF_MEMORY, "host allocation for the forward CSR failed");
   }
-  if (n) {
-    STC_CUDA(cudaMemcpyAsync(out->offsets, off_id, ((size_t)n + 1) * sizeof(uint64_t),
-                             cudaMemcpyDeviceToHost, st));
-    STC_CUDA(cudaMemcpyAsync(out->fdeg, fdeg_id, (size_t)n * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    STC_CUDA(cudaMemcpyAsync(out->rank, g.rank, (size_t)n * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-  } else {
-    out->offsets[0] = 0;
-  }
-  if (mu) {
-    STC_CUDA(cudaMemcpyAsync(out->edges, edges, mu * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    STC_CUDA(cudaMemcpyAsync(out->signs, signs, mu, cudaMemcpyDeviceToHost, st));
-  }
-  STC_CUDA(cudaStreamSynchronize(st));
+  if (n == 0) out->offsets[0] = 0;
+  download(c, {piece(off_id, out->offsets, n ? (size_t)n + 1 : 0), piece(fdeg_id, out->fdeg, n),
+               piece(g.rank, out->rank, n), piece(edges, out->edges, mu),
+               piece(signs, out->signs, mu)});
 }
 
 }  // namespace stc

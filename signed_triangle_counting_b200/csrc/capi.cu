@@ -47,6 +47,27 @@ void wait_sign(stc_ctx* c) {
   STC_CUDA(cudaStreamWaitEvent(c->stream, c->ev_sign, 0));
 }
 
+void upload(stc_ctx* c, const std::vector<HostCopier::Piece>& pieces) {
+  std::vector<HostCopier::Piece> staged;
+  for (const auto& p : pieces) {
+    if (p.bytes == 0) continue;
+    if (is_pageable(p.host)) staged.push_back(p);
+    else STC_CUDA(cudaMemcpyAsync(p.device, p.host, p.bytes, cudaMemcpyHostToDevice, c->stream));
+  }
+  c->copier.upload(staged, c->stream);
+}
+
+void download(stc_ctx* c, const std::vector<HostCopier::Piece>& pieces) {
+  std::vector<HostCopier::Piece> staged;
+  for (const auto& p : pieces) {
+    if (p.bytes == 0) continue;
+    if (is_pageable(p.host)) staged.push_back(p);
+    else STC_CUDA(cudaMemcpyAsync(p.host, p.device, p.bytes, cudaMemcpyDeviceToHost, c->stream));
+  }
+  c->copier.download(staged, c->stream);
+  STC_CUDA(cudaStreamSynchronize(c->stream));
+}
+
 void release_pipelines(stc_ctx* c) {
   for (auto& p : c->pipes)
     if (p.exec) cudaGraphExecDestroy(p.exec);
@@ -140,9 +161,9 @@ struct DeviceInput {
 };
 
 // Device copies of host input (device input as it is).  With defer_sign
-// the sign array is copied on the auxiliary stream after the ids, so that
-// it overlaps the id scan, degrees and ranking; the build waits for it
-// (wait_sign) before its first read of the signs.
+// a sign array the driver need not stage is copied on the auxiliary stream
+// after the ids, so that it overlaps the id scan, degrees and ranking; the
+// build waits for it (wait_sign) before its first read of the signs.
 DeviceInput stage_input(stc_ctx* c, const uint32_t* src, const uint32_t* dst, const int8_t* sign,
                         uint64_t m, const stc_opts* o, bool defer_sign = false) {
   if (m && (!src || !dst || !sign)) fail(STC_ERR_INVALID_ARGUMENT, "null edge array");
@@ -151,16 +172,14 @@ DeviceInput stage_input(stc_ctx* c, const uint32_t* src, const uint32_t* dst, co
   uint32_t* dd = buffer<uint32_t>(c, B_IN_DST, m);
   int8_t* dg = buffer<int8_t>(c, B_IN_SIGN, m);
   if (m) {
-    STC_CUDA(cudaMemcpyAsync(ds, src, m * sizeof(uint32_t), cudaMemcpyHostToDevice, c->stream));
-    STC_CUDA(cudaMemcpyAsync(dd, dst, m * sizeof(uint32_t), cudaMemcpyHostToDevice, c->stream));
+    defer_sign = defer_sign && !is_pageable(sign);
+    upload(c, {piece(ds, src, m), piece(dd, dst, m), piece(dg, sign, defer_sign ? 0 : m)});
     if (defer_sign) {
       STC_CUDA(cudaEventRecord(c->ev_ids, c->stream));
       STC_CUDA(cudaStreamWaitEvent(c->aux_stream, c->ev_ids, 0));
       STC_CUDA(cudaMemcpyAsync(dg, sign, m, cudaMemcpyHostToDevice, c->aux_stream));
       STC_CUDA(cudaEventRecord(c->ev_sign, c->aux_stream));
       c->sign_pending = true;
-    } else {
-      STC_CUDA(cudaMemcpyAsync(dg, sign, m, cudaMemcpyHostToDevice, c->stream));
     }
   }
   return DeviceInput{ds, dd, dg};
@@ -464,6 +483,7 @@ void stc_ctx_destroy(stc_ctx* c) {
   if (c->own_stream) cudaStreamSynchronize(c->own_stream);
   if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
   release_pipelines(c);
+  c->copier.release();
   for (auto& b : c->bufs)
     if (b.p) cudaFree(b.p);
   if (c->h_eoff) cudaFreeHost(c->h_eoff);
@@ -498,6 +518,7 @@ stc_status stc_ctx_trim(stc_ctx* c) {
       c->graph_exec = nullptr;
     }
     release_pipelines(c);
+    c->copier.release();
     c->buf_gen++;
     for (int i = 0; i < B_COUNT_; i++) {
       if (i == B_COUNTERS) continue;
@@ -558,8 +579,10 @@ uint64_t stage_and_parse_text(stc_ctx* c, const char* data, uint64_t size, const
   char* d_text = buffer<char>(c, B_TEXT, padded ? padded : 16);
   if (size) {
     const bool dev = o && (o->flags & STC_F_DEVICE_INPUT);
-    STC_CUDA(cudaMemcpyAsync(d_text, data, size, dev ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
-                             c->stream));
+    if (dev)
+      STC_CUDA(cudaMemcpyAsync(d_text, data, size, cudaMemcpyDeviceToDevice, c->stream));
+    else
+      upload(c, {piece(d_text, data, size)});
     if (padded > size) STC_CUDA(cudaMemsetAsync(d_text + size, 0, padded - size, c->stream));
   }
   uint32_t* s = nullptr;
@@ -602,21 +625,16 @@ stc_status stc_parse_edge_text_gpu(stc_ctx* c, const char* data, uint64_t size,
     uint32_t n = 0;
     const uint64_t m = stage_and_parse_text(c, data, size, o, &in, &lines, &n);
     const uint64_t cap = m ? m : 1;
-    out->src = (uint32_t*)malloc(cap * sizeof(uint32_t));
-    out->dst = (uint32_t*)malloc(cap * sizeof(uint32_t));
-    out->sign = (int8_t*)malloc(cap);
+    out->src = (uint32_t*)host_alloc(cap * sizeof(uint32_t));
+    out->dst = (uint32_t*)host_alloc(cap * sizeof(uint32_t));
+    out->sign = (int8_t*)host_alloc(cap);
     if (!out->src || !out->dst || !out->sign) {
       stc_free_edge_list(out);
       fail(STC_ERR_OUT_OF_MEMORY, "host allocation of the edge list failed");
     }
-    if (m) {
-      STC_CUDA(cudaMemcpyAsync(out->src, in.src, m * sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                               c->stream));
-      STC_CUDA(cudaMemcpyAsync(out->dst, in.dst, m * sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                               c->stream));
-      STC_CUDA(cudaMemcpyAsync(out->sign, in.sign, m, cudaMemcpyDeviceToHost, c->stream));
-    }
-    STC_CUDA(cudaStreamSynchronize(c->stream));
+    download(c, {piece(const_cast<uint32_t*>(in.src), out->src, m),
+                 piece(const_cast<uint32_t*>(in.dst), out->dst, m),
+                 piece(const_cast<int8_t*>(in.sign), out->sign, m)});
     out->n = size ? n : 0;
     out->lines = lines;
     out->m = m;
@@ -676,16 +694,8 @@ stc_status stc_count_forward_csr(stc_ctx* c, const stc_forward_csr* csr, const s
     uint32_t* d_edges = buffer<uint32_t>(c, B_IN_SRC, m);
     int8_t* d_signs = buffer<int8_t>(c, B_IN_SIGN, m);
     uint32_t* d_rank = buffer<uint32_t>(c, B_IN_DST, n);
-    STC_CUDA(cudaMemcpyAsync(d_off, csr->offsets, ((size_t)n + 1) * sizeof(uint64_t),
-                             cudaMemcpyHostToDevice, c->stream));
-    if (m) {
-      STC_CUDA(cudaMemcpyAsync(d_edges, csr->edges, m * sizeof(uint32_t), cudaMemcpyHostToDevice,
-                               c->stream));
-      STC_CUDA(cudaMemcpyAsync(d_signs, csr->signs, m, cudaMemcpyHostToDevice, c->stream));
-    }
-    if (n)
-      STC_CUDA(cudaMemcpyAsync(d_rank, csr->rank, (size_t)n * sizeof(uint32_t),
-                               cudaMemcpyHostToDevice, c->stream));
+    upload(c, {piece(d_off, csr->offsets, (size_t)n + 1), piece(d_edges, csr->edges, m),
+               piece(d_signs, csr->signs, m), piece(d_rank, csr->rank, n)});
     DeviceGraph g;
     graph_from_forward_csr(c, n, m, d_off, d_edges, d_signs, d_rank, g);
     count_triangles(c, g, cfg);
@@ -713,9 +723,7 @@ stc_status stc_vertex_counts(stc_ctx* c, const uint32_t* src, const uint32_t* ds
     cfg.vertex_counts = dv;
     count_triangles(c, g, cfg);
     mark(c, 5);
-    if (g.n)
-      STC_CUDA(cudaMemcpyAsync(counts, dv, 4ull * g.n * sizeof(uint64_t), cudaMemcpyDeviceToHost,
-                               c->stream));
+    download(c, {piece(dv, counts, 4ull * g.n)});
     end_call(c, g, nullptr);
   });
 }
@@ -798,16 +806,27 @@ stc_status stc_count_batch(stc_ctx* c, const stc_graph* graphs, uint32_t G, cons
     uint32_t* ds = buffer<uint32_t>(c, B_IN_SRC, M);
     uint32_t* dd = buffer<uint32_t>(c, B_IN_DST, M);
     int8_t* dg = buffer<int8_t>(c, B_IN_SIGN, M);
-    const cudaMemcpyKind kind = dev ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
+    std::vector<HostCopier::Piece> ps, pd, pg;  // host graphs, by array
     for (uint32_t i = 0; i < G; i++) {
       const uint64_t m = graphs[i].m;
       if (!m) continue;
       if (!graphs[i].src || !graphs[i].dst || !graphs[i].sign)
         fail(STC_ERR_INVALID_ARGUMENT, "null edge array in graph " + std::to_string(i));
+      if (!dev) {
+        ps.push_back(piece(ds + off[i], graphs[i].src, m));
+        pd.push_back(piece(dd + off[i], graphs[i].dst, m));
+        pg.push_back(piece(dg + off[i], graphs[i].sign, m));
+        continue;
+      }
+      const cudaMemcpyKind kind = cudaMemcpyDeviceToDevice;
       STC_CUDA(cudaMemcpyAsync(ds + off[i], graphs[i].src, m * sizeof(uint32_t), kind, st));
       STC_CUDA(cudaMemcpyAsync(dd + off[i], graphs[i].dst, m * sizeof(uint32_t), kind, st));
       STC_CUDA(cudaMemcpyAsync(dg + off[i], graphs[i].sign, m, kind, st));
     }
+    c->stream = st;
+    ps.insert(ps.end(), pd.begin(), pd.end());
+    ps.insert(ps.end(), pg.begin(), pg.end());
+    upload(c, ps);
   });
   if (s != STC_OK) return s;
   stc_opts o2 = o ? *o : stc_opts{};

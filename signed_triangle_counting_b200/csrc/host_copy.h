@@ -1,0 +1,263 @@
+// Copies between a caller's pageable host memory and the device, through a
+// small ring of pinned slots that worker threads fill (or drain) while earlier
+// slots cross the bus.
+//
+// A pageable cudaMemcpyAsync stages with one host thread (15 GB/s up; down
+// into fresh pages 5 GB/s, most of it page faults) and costs about 10 us
+// however small it is.  Eight threads fill slots at 58 GB/s, as fast as the
+// bus takes them, and scattered pieces that lie back to back on the device
+// (the graphs of a batch) cross as one copy per slot.
+//
+// The ring and the threads belong to one context, are made on the first use
+// that is worth them, and go with it (or with stc_ctx_trim).
+#pragma once
+#include <cuda_runtime.h>
+#include <sys/mman.h>
+
+#include <algorithm>
+#include <atomic>
+#include <condition_variable>
+#include <cstdlib>
+#include <cstring>
+#include <mutex>
+#include <thread>
+#include <vector>
+
+namespace stc {
+
+void cuda_check(cudaError_t e, const char* what);
+
+// True when p is plain host memory the driver would have to stage.
+inline bool is_pageable(const void* p) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeUnregistered;
+}
+
+// malloc whose large blocks ask for huge pages (release with free): first
+// touches then fault once per 2 MB.
+inline void* host_alloc(size_t bytes) {
+  constexpr size_t kHuge = 2u << 20;
+  if (bytes < 2 * kHuge) return malloc(bytes ? bytes : 1);
+  const size_t n = (bytes + kHuge - 1) / kHuge * kHuge;
+  void* p = aligned_alloc(kHuge, n);
+  if (p) (void)madvise(p, n, MADV_HUGEPAGE);
+  return p;
+}
+
+class HostCopier {
+ public:
+  struct Piece {
+    char* device;
+    char* host;  // only read by upload
+    size_t bytes;
+  };
+
+  HostCopier() = default;
+  HostCopier(const HostCopier&) = delete;
+  HostCopier& operator=(const HostCopier&) = delete;
+  ~HostCopier() { release(); }
+
+  // Host pieces to the device, in stream order; the host memory may be reused
+  // on return.  Pieces that follow each other on the device share copies.
+  void upload(const std::vector<Piece>& pieces, cudaStream_t st) { run(pieces, st, true); }
+  // Device to host pieces; done on return.
+  void download(const std::vector<Piece>& pieces, cudaStream_t st) { run(pieces, st, false); }
+
+  void release() {
+    if (!threads_.empty()) {
+      {
+        std::lock_guard<std::mutex> l(mu_);
+        quit_ = true;
+      }
+      cv_.notify_all();
+      for (auto& t : threads_) t.join();
+      threads_.clear();
+      quit_ = false;
+    }
+    for (int i = 0; i < kSlots; i++) {
+      if (event_[i]) {
+        (void)cudaEventSynchronize(event_[i]);
+        (void)cudaEventDestroy(event_[i]);
+        event_[i] = nullptr;
+      }
+    }
+    if (ring_) (void)cudaFreeHost(ring_);
+    ring_ = nullptr;
+  }
+
+ private:
+  static constexpr int kSlots = 8;
+  static constexpr size_t kSlotBytes = 2u << 20;
+  static constexpr size_t kPart = 256u << 10;           // what a thread copies at a time
+  static constexpr size_t kThreadedBytes = 2u << 20;    // less is not worth waking threads for
+  // A part of one slot's contents, between `ring` and `host`.
+  struct Part {
+    char* ring;
+    char* host;
+    size_t bytes;
+  };
+  struct Chunk {  // one slot's contents: a run of device memory
+    char* device;
+    size_t bytes;
+    uint32_t part0, part1;
+    std::atomic<uint32_t> left{0};  // parts not copied yet
+    Chunk(char* d, uint32_t p) : device(d), bytes(0), part0(p), part1(p) {}
+    Chunk(const Chunk& o) : device(o.device), bytes(o.bytes), part0(o.part0), part1(o.part1) {}
+  };
+
+  void run(const std::vector<Piece>& pieces, cudaStream_t st, bool up) {
+    size_t total = 0;
+    for (const Piece& p : pieces) total += p.bytes;
+    if (total == 0) return;
+    if (!ring_) {
+      cuda_check(cudaMallocHost(reinterpret_cast<void**>(&ring_), kSlots * kSlotBytes),
+                 "cudaMallocHost(staging ring)");
+      for (auto& e : event_)
+        cuda_check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate(staging)");
+    }
+    // Cut the pieces into slots and parts.
+    std::vector<Chunk> chunks;
+    parts_.clear();
+    part_chunk_.clear();
+    for (const Piece& p : pieces) {
+      size_t at = 0;
+      while (at < p.bytes) {
+        if (chunks.empty() || chunks.back().device + chunks.back().bytes != p.device + at ||
+            chunks.back().bytes == kSlotBytes)
+          chunks.emplace_back(p.device + at, (uint32_t)parts_.size());
+        Chunk& c = chunks.back();
+        const size_t n = std::min({p.bytes - at, kSlotBytes - c.bytes, kPart});
+        parts_.push_back(Part{ring_ + ((chunks.size() - 1) % kSlots) * kSlotBytes + c.bytes,
+                              p.host + at, n});
+        part_chunk_.push_back((uint32_t)chunks.size() - 1);
+        c.part1 = (uint32_t)parts_.size();
+        c.bytes += n;
+        at += n;
+      }
+    }
+    for (Chunk& c : chunks) c.left.store(c.part1 - c.part0, std::memory_order_relaxed);
+    const bool threaded = total >= kThreadedBytes;
+    chunks_ = &chunks;
+    up_ = up;
+    next_.store(0);
+    open_.store(0);  // parts below it may be copied
+    cancel_.store(false);
+    if (threaded) wake();
+    struct Guard {  // whatever happens, no thread touches this call's memory after it
+      HostCopier* c;
+      bool threaded;
+      ~Guard() {
+        c->cancel_.store(true);
+        if (threaded) c->settle();
+      }
+    } guard{this, threaded};
+    const uint32_t nc = (uint32_t)chunks.size();
+    auto event_done = [&](uint32_t c) {  // the slot's last transfer
+      cuda_check(cudaEventSynchronize(event_[c % kSlots]), "cudaEventSynchronize(staging)");
+    };
+    auto finish = [&](uint32_t c) {  // the chunk's parts are copied
+      while (chunks[c].left.load(std::memory_order_acquire) != 0)
+        if (!copy_part()) std::this_thread::yield();
+    };
+    if (up) {
+      uint32_t opened = 0;
+      for (uint32_t c = 0; c < nc; c++) {
+        for (; opened < nc && opened < c + kSlots - 1; opened++) {
+          event_done(opened);  // recorded by the chunk kSlots before, or an earlier call
+          open_.store(chunks[opened].part1, std::memory_order_release);
+        }
+        finish(c);
+        cuda_check(cudaMemcpyAsync(chunks[c].device, ring_ + (c % kSlots) * kSlotBytes,
+                                   chunks[c].bytes, cudaMemcpyHostToDevice, st),
+                   "cudaMemcpyAsync(staging)");
+        cuda_check(cudaEventRecord(event_[c % kSlots], st), "cudaEventRecord(staging)");
+      }
+    } else {
+      uint32_t issued = 0;
+      for (uint32_t c = 0; c < nc; c++) {
+        for (; issued < nc && issued < c + kSlots; issued++) {
+          if (issued >= kSlots) finish(issued - kSlots);  // the slot is drained
+          else event_done(issued);                        // an earlier call's transfer
+          cuda_check(cudaMemcpyAsync(ring_ + (issued % kSlots) * kSlotBytes, chunks[issued].device,
+                                     chunks[issued].bytes, cudaMemcpyDeviceToHost, st),
+                     "cudaMemcpyAsync(staging)");
+          cuda_check(cudaEventRecord(event_[issued % kSlots], st), "cudaEventRecord(staging)");
+        }
+        event_done(c);
+        open_.store(chunks[c].part1, std::memory_order_release);
+      }
+      for (uint32_t c = 0; c < nc; c++) finish(c);
+    }
+  }
+
+  // Copies the next part if one is open.
+  bool copy_part() {
+    uint32_t i = next_.load(std::memory_order_relaxed);
+    do {
+      if (i >= open_.load(std::memory_order_acquire)) return false;
+    } while (!next_.compare_exchange_weak(i, i + 1, std::memory_order_relaxed));
+    const Part& p = parts_[i];
+    if (up_) memcpy(p.ring, p.host, p.bytes);
+    else memcpy(p.host, p.ring, p.bytes);
+    (*chunks_)[part_chunk_[i]].left.fetch_sub(1, std::memory_order_release);
+    return true;
+  }
+
+  void wake() {
+    if (threads_.empty()) {
+      const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
+      const unsigned n = std::min(7u, hw > 2 ? hw / 2 : 1u);  // the caller is one more
+      // They have seen the calls so far (the ring may have been released since).
+      for (unsigned i = 0; i < n; i++)
+        threads_.emplace_back([this, seen = generation_] { work(seen); });
+    }
+    {
+      std::lock_guard<std::mutex> l(mu_);
+      generation_++;
+      busy_ = (int)threads_.size();
+    }
+    cv_.notify_all();
+  }
+
+  void settle() {
+    std::unique_lock<std::mutex> l(mu_);
+    idle_.wait(l, [this] { return busy_ == 0; });
+  }
+
+  void work(uint64_t seen) {
+    while (true) {
+      {
+        std::unique_lock<std::mutex> l(mu_);
+        cv_.wait(l, [&] { return quit_ || generation_ != seen; });
+        if (quit_) return;
+        seen = generation_;
+      }
+      const uint32_t n = (uint32_t)parts_.size();
+      while (!cancel_.load(std::memory_order_relaxed) && next_.load(std::memory_order_relaxed) < n)
+        if (!copy_part()) std::this_thread::yield();
+      std::lock_guard<std::mutex> l(mu_);
+      if (--busy_ == 0) idle_.notify_all();
+    }
+  }
+
+  char* ring_ = nullptr;
+  cudaEvent_t event_[kSlots] = {};
+  std::vector<Part> parts_;
+  std::vector<uint32_t> part_chunk_;
+  std::vector<Chunk>* chunks_ = nullptr;
+  bool up_ = true;
+  std::atomic<uint32_t> next_{0}, open_{0};
+  std::atomic<bool> cancel_{false};
+  std::vector<std::thread> threads_;
+  std::mutex mu_;
+  std::condition_variable cv_, idle_;
+  uint64_t generation_ = 0;
+  int busy_ = 0;
+  bool quit_ = false;
+};
+
+}  // namespace stc

@@ -7,6 +7,7 @@
 #include <string>
 #include <vector>
 
+#include "host_copy.h"
 #include "stc.h"
 
 namespace stc {
@@ -171,6 +172,7 @@ struct stc_ctx {
   uint64_t graph_key[32] = {};
   int graph_launches = 0;  // kernels per replay of graph_exec
   stc::Tuning tuning;
+  stc::HostCopier copier;  // staging of pageable host memory
   // Batch groups captured whole (at most four, the least recently used
   // replaced), the pinned staging of a group's edge offsets they copy from,
   // and the buffer generation: bumped whenever a device buffer or the
@@ -247,6 +249,16 @@ struct DeviceGraph {
   uint32_t* nbr_split = nullptr;
   uint32_t* psplit = nullptr;
 };
+
+// Copies host arrays to the device (stream order; host memory reusable on
+// return) and back (done on return): pageable memory through the context's
+// staging, anything else by the driver.
+void upload(stc_ctx* c, const std::vector<HostCopier::Piece>& pieces);
+void download(stc_ctx* c, const std::vector<HostCopier::Piece>& pieces);
+template <class T>
+HostCopier::Piece piece(T* device, const T* host, size_t count) {
+  return HostCopier::Piece{(char*)device, (char*)host, count * sizeof(T)};
+}
 
 // Stage timing helper: records an event when the context is timing.
 void mark(stc_ctx* c, int slot);
