@@ -73,6 +73,9 @@ struct Csr {
   // Heads with their signs, id << 1 | negative (same offsets, padded
   // likewise): what the head side streams, one 16-byte load per chunk.
   const uint32_t* __restrict__ nkey = nullptr;
+  // Arcs whose shorter list has at most so many entries are counted where the
+  // head side's keys are made; the tail side's kernels skip them (0: none).
+  uint32_t short_max = 0;
 };
 
 // Per-thread type counters indexed by the number of negative edges.
@@ -293,7 +296,8 @@ __device__ __forceinline__ void stage(const Csr& g, uint64_t ub, uint32_t d, uin
       b = (b + 1) & (geo.nb - 1);
     const uint32_t blen = m.hi[i] - m.lo[i];
     uint8_t st = (i + 1 < d && blen) ? table[size_bucket(d - i - 1)][size_bucket(blen)] : kNoArc;
-    if (st == STC_STRATEGY_HEAD) st = kNoArc;  // counted by the head-side pass
+    if (st == STC_STRATEGY_HEAD || min(d - i - 1, blen) <= g.short_max)
+      st = kNoArc;  // counted by the head-side pass, or with its keys
     m.st[i] = st;
     if (st == STC_STRATEGY_SPLIT) m.sp[i] = m.lo[i] + g.psplit[x];
   }
@@ -806,11 +810,14 @@ struct VertexSink {  // per-source counts by original id: vcounts[4 * id + type]
   const uint32_t* verts;
   __device__ void put(uint32_t u, const unsigned long long* c) const {
 #pragma unroll
-    for (int k = 0; k < 4; k++) vcounts[4ull * verts[u] + (3 - k)] = c[k];
+    for (int k = 0; k < 4; k++)
+      if (c[k]) atomicAdd(vcounts + 4ull * verts[u] + (3 - k), c[k]);
   }
-  // The head side's counts of one arc with tail u, added to those the tail
-  // side stored (its kernels run first): fewer than 2^16 of each number of
-  // negative edges, 0 and 1 in w0, 2 and 3 in w1.
+  __device__ void add(uint32_t u, uint32_t neg) const {
+    atomicAdd(vcounts + 4ull * verts[u] + (3 - neg), 1ull);
+  }
+  // The head side's counts of one arc with tail u: fewer than 2^16 of each
+  // number of negative edges, 0 and 1 in w0, 2 and 3 in w1.
   __device__ void add_arc(uint32_t u, uint32_t w0, uint32_t w1) const {
     if ((w0 | w1) == 0) return;
     unsigned long long* c = vcounts + 4ull * verts[u];
@@ -959,6 +966,7 @@ __global__ void k_classify_fill(const uint64_t* __restrict__ off, uint32_t n, Cl
        base += gridDim.x * blockDim.x) {
     const uint32_t u = base + lane_id();
     const uint32_t c = (u >= u1 || (need && !need[u])) ? 5u : cb.of((uint32_t)(off[u + 1] - off[u]));
+    if (!__any_sync(kFull, c < kClasses)) continue;
     const unsigned peers = __match_any_sync(kFull, c);
     const uint32_t leader = __ffs(peers) - 1;
     uint32_t pos = 0;
@@ -991,7 +999,9 @@ __device__ __forceinline__ void tiny_vertex(const Csr& g, uint32_t u, const Sink
     if (k + 1 >= (int)d) break;
     const uint64_t vb = g.off[a[k]];
     const uint32_t blen = (uint32_t)(g.off[a[k] + 1] - vb);
-    if (table[size_bucket(d - k - 1)][size_bucket(blen)] == STC_STRATEGY_HEAD) continue;
+    if (table[size_bucket(d - k - 1)][size_bucket(blen)] == STC_STRATEGY_HEAD ||
+        min(d - k - 1, blen) <= g.short_max)
+      continue;
     const uint32_t* b = g.nbr + vb;
     uint32_t pos = 0;
 #pragma unroll
@@ -1193,7 +1203,8 @@ __global__ void __launch_bounds__(THREADS) k_giant(Csr g, const uint32_t* __rest
       const uint32_t blen = (uint32_t)(g.off[v + 1] - vb);
       if (blen == 0) continue;
       const uint32_t st = table[size_bucket(d - k - 1)][size_bucket(blen)];
-      if (st == STC_STRATEGY_HEAD) continue;  // counted by the head-side pass
+      if (st == STC_STRATEGY_HEAD || min(d - k - 1, blen) <= g.short_max)
+        continue;  // counted by the head-side pass, or with its keys
       long long t0 = 0;
       if (kTime) {
         __syncwarp();
@@ -1484,6 +1495,75 @@ struct HeadArcs {
   }
 };
 
+// An arc counted by one thread: the entries of the shorter of its lists
+// A' = [i + 1, i + 1 + alen) and B = [vb, vb + blen), searched in the longer
+// one from the last hit on; hit(negative edges) per triangle.
+template <class Hit>
+__device__ __forceinline__ void short_arc(const Csr& g, uint32_t i, uint32_t alen, uint32_t vb,
+                                          uint32_t blen, uint32_t nuv, Hit hit) {
+  const bool swap = alen > blen;
+  const uint32_t s0 = swap ? vb : i + 1, l0 = swap ? i + 1 : vb;
+  const uint32_t sn = swap ? blen : alen, ln = swap ? alen : blen;
+  const uint32_t* l = g.nbr + l0;
+  uint32_t pos = 0;
+  for (uint32_t k = 0; k < sn; k++) {
+    const uint32_t x = g.nbr[s0 + k];
+    pos += lower_bound(l + pos, ln - pos, x);
+    if (pos >= ln) return;
+    if (l[pos] == x) {
+      hit(nuv + (g.sgn[s0 + k] < 0) + (g.sgn[l0 + pos] < 0));
+      pos++;
+    }
+  }
+}
+// The longest shorter list of an arc counted that way: staging a list for it
+// costs more than so many searches (128-graph batch: 19.4 ms without, 16.3
+// with lists up to 4, 15.7 up to 8, 15.9 up to 16, 16.3 up to 32; the skewed
+// workload 19.2 -> 17.4 ms from 8 on).
+constexpr uint32_t kShortArc = 8;
+
+// Where k_head_keys's short arcs are counted.  Totals add up per thread.  A
+// batch adds up per warp while the warp's arcs stay in one graph, whose rank
+// range it keeps; a warp whose arcs of a tile span graphs hands over hit by
+// hit.  Per-vertex counts go to the tail hit by hit.
+template <class Sink>
+struct ShortCounts {
+  static constexpr bool kGraph = Sink::kKeyed;
+  TypeCounts tc;
+  uint32_t graph = 0, lo = 1, hi = 0;  // the warp's graph and its ranks [lo, hi)
+  bool spans = false;
+  // The warp's arcs of a tile have tails in [first, last].
+  __device__ __forceinline__ void tile(const Sink& sink, uint32_t first, uint32_t last) {
+    if constexpr (kGraph) {
+      if (first < lo || first >= hi) {
+        flush(sink);
+        graph = sink.graph_of(first);
+        lo = (uint32_t)sink.gbase[graph];
+        hi = (uint32_t)sink.gbase[graph + 1];
+      }
+      spans = last >= hi;
+    }
+  }
+  __device__ __forceinline__ void hit(const Sink& sink, uint32_t u, uint32_t neg) {
+    if constexpr (Sink::kPerArc) {
+      sink.add(u, neg);
+    } else if (kGraph && spans) {
+      if constexpr (kGraph) atomicAdd(sink.gcounts + 4ull * sink.graph_of(u) + (3 - neg), 1ull);
+    } else {
+      tc.add(neg);
+    }
+  }
+  __device__ __forceinline__ void flush(const Sink& sink) {
+    if constexpr (kGraph) {
+      unsigned long long c[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) c[k] = warp_sum(tc.c[k]);
+      if (lane_id() == 0) sink.put_key(graph, c);
+      tc = TypeCounts{};
+    }
+  }
+};
+
 // Appends the keys of the HEAD arcs (count in ctr[C_HEAD_NKEYS]), records
 // the list end of each HEAD arc whose |A'| its key cannot hold, and sets
 // need[u] = 1 for each tail u with an arc left to the tail side (the array
@@ -1493,7 +1573,10 @@ struct HeadArcs {
 // it reads anyway: a pass of its own took 0.82 ms at RMAT scale 24.
 // A CTA appends a tile of 1,024 arcs with one atomic; with one per warp and
 // load the 8 M atomics on the one counter took 6.8 ms at RMAT scale 24.
-template <bool kBytes>
+// With kShort, an arc that is not HEAD and whose shorter list has at most
+// kShortArc entries is counted on the spot, by its thread: its extents are at
+// hand, and no list is classified, queued or staged for it.
+template <class Sink, bool kBytes, bool kShort>
 __global__ void __launch_bounds__(256) k_head_keys(Csr g, const uint32_t* __restrict__ asrc,
                                                    const uint32_t* __restrict__ fdeg, uint64_t m,
                                                    const unsigned long long* __restrict__ m_dev,
@@ -1502,7 +1585,7 @@ __global__ void __launch_bounds__(256) k_head_keys(Csr g, const uint32_t* __rest
                                                    HeadKey fmt, uint64_t* __restrict__ keys,
                                                    uint32_t* __restrict__ aend,
                                                    uint8_t* __restrict__ need,
-                                                   unsigned long long* __restrict__ ctr) {
+                                                   unsigned long long* __restrict__ ctr, Sink sink) {
   constexpr int kItems = 4;  // arcs per lane with their gathers in flight together
   constexpr int kWarps = 8;
   __shared__ uint8_t tab[kTableBytes];
@@ -1515,6 +1598,7 @@ __global__ void __launch_bounds__(256) k_head_keys(Csr g, const uint32_t* __rest
   const uint32_t r1 = range ? (uint32_t)range[1] : 0xFFFFFFFFu;
   const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
   unsigned long long bytes = 0, probe = 0;
+  ShortCounts<Sink> sc;
   uint32_t flip = 0;
   for (uint64_t tile = (uint64_t)blockIdx.x * (256 * kItems); tile < m;
        tile += (uint64_t)gridDim.x * (256 * kItems), flip ^= 1) {
@@ -1536,6 +1620,7 @@ __global__ void __launch_bounds__(256) k_head_keys(Csr g, const uint32_t* __rest
       blen[q] = i < m ? fdeg[v[q]] : 0u;
     }
     uint32_t heads = 0, mine = 0, total = 0;  // HEAD flags; keys of the lanes below; of the warp
+    uint32_t shorts = 0;                      // arcs counted here
 #pragma unroll
     for (int q = 0; q < kItems; q++) {
       const uint64_t i = base + 32 * q;
@@ -1549,7 +1634,10 @@ __global__ void __launch_bounds__(256) k_head_keys(Csr g, const uint32_t* __rest
         if (alen && blen[q] && u[q] >= r0 && u[q] < r1) {
           head = tab[256 * table_class(d) + 16 * size_bucket(alen) + size_bucket(blen[q])] ==
                  STC_STRATEGY_HEAD;
-          if (!head) need[u[q]] = 1;  // u keeps an arc for the tail side
+          if (!head) {
+            if (kShort && min(alen, blen[q]) <= kShortArc) shorts |= 1u << q;
+            else need[u[q]] = 1;  // u keeps an arc for the tail side
+          }
         }
       }
       const unsigned hb = __ballot_sync(kFull, head);
@@ -1568,6 +1656,11 @@ __global__ void __launch_bounds__(256) k_head_keys(Csr g, const uint32_t* __rest
       }
       tbase[flip] = run ? (uint32_t)atomicAdd(ctr + C_HEAD_NKEYS, (unsigned long long)run) : 0u;
     }
+    uint32_t vb[kItems];
+    if (kShort) {
+#pragma unroll
+      for (int q = 0; q < kItems; q++) vb[q] = (shorts >> q) & 1u ? (uint32_t)g.off[v[q]] : 0u;
+    }
     __syncthreads();
     // The keys of one lane in a row: any order within the tile will do.
     uint32_t at = tbase[flip] + wcnt[flip][warp] + mine;
@@ -1580,6 +1673,26 @@ __global__ void __launch_bounds__(256) k_head_keys(Csr g, const uint32_t* __rest
         if (alen >= fmt.amax) aend[i] = ue[q];
       }
     }
+    if (kShort && __any_sync(kFull, shorts != 0)) {
+      if (ShortCounts<Sink>::kGraph) {
+        const uint32_t first = __shfl_sync(kFull, u[0], 0);
+        uint32_t last = 0;
+#pragma unroll
+        for (int q = 0; q < kItems; q++) last = max(last, u[q]);  // past the end: 0
+        sc.tile(sink, first, __reduce_max_sync(kFull, last));
+      }
+#pragma unroll
+      for (int q = 0; q < kItems; q++) {
+        if (!((shorts >> q) & 1u)) continue;
+        const uint32_t i = (uint32_t)(base + 32 * q), tail = u[q];
+        short_arc(g, i, ue[q] - i - 1, vb[q], blen[q], (neg >> q) & 1u,
+                  [&](uint32_t n) { sc.hit(sink, tail, n); });
+      }
+    }
+  }
+  if (kShort) {
+    if (ShortCounts<Sink>::kGraph) sc.flush(sink);
+    else if (!Sink::kPerVertex) flush_counts<256>(sc.tc, ctr);
   }
   if (kBytes) {
     bytes = warp_sum(bytes);
@@ -2180,21 +2293,23 @@ void prepare_head(const Tuning& tu) {
 // tails left without arcs), then the sort, runs, plan and the three
 // head-class kernels.  The launch parameters of the block and large classes
 // follow the tuning of the tail side's same classes.
-inline void enqueue_head_keys(cudaStream_t st, const Csr& csr, const uint32_t* asrc,
+template <class Sink>
+void enqueue_head_keys(cudaStream_t st, const Csr& csr, const uint32_t* asrc,
                               const uint32_t* fdeg, uint64_t m,
-                              const unsigned long long* m_dev, bool bytes, const HeadBufs& b,
-                              const uint8_t* d_tables,
+                              const unsigned long long* m_dev, bool bytes, bool short_arcs,
+                              const HeadBufs& b, const uint8_t* d_tables,
                               const unsigned long long* range, unsigned long long* ctr,
-                              int& launches) {
+                              const Sink& sink, int& launches) {
   STC_CUDA(cudaMemsetAsync(ctr + C_HEAD_NKEYS, 0,
                            (C_HEAD_QUEUE + kHeadClasses - C_HEAD_NKEYS) * sizeof(unsigned long long),
                            st));
   STC_CUDA(cudaMemsetAsync(b.need, 0, csr.n, st));
   const uint32_t grid = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((m + 1023) / 1024, kSMs * 8));
   const HeadKey fmt = HeadKey::of(csr.n, m);
-  auto kernel = bytes ? k_head_keys<true> : k_head_keys<false>;
+  auto kernel = bytes ? (short_arcs ? k_head_keys<Sink, true, true> : k_head_keys<Sink, true, false>)
+                      : (short_arcs ? k_head_keys<Sink, false, true> : k_head_keys<Sink, false, false>);
   kernel<<<grid, 256, 0, st>>>(csr, asrc, fdeg, m, m_dev, d_tables, range, fmt, b.keys, b.aend,
-                               b.need, ctr);
+                               b.need, ctr, sink);
   launches += 1;
 }
 
@@ -2354,7 +2469,8 @@ struct HeadPlan {
   const uint32_t* asrc = nullptr;
   const uint32_t* fdeg = nullptr;
   uint64_t m = 0;
-  bool bytes = false;  // the key pass adds up the arcs' algorithmic bytes
+  bool bytes = false;       // the key pass adds up the arcs' algorithmic bytes
+  bool short_arcs = false;  // ... and counts the short arcs
   const unsigned long long* m_dev = nullptr;  // arc count on the device when m is a capacity
   const uint64_t* gbase = nullptr;  // G + 1 rank boundaries of a batch
   uint32_t G = 0;
@@ -2369,8 +2485,8 @@ void enqueue_persistent(cudaStream_t st, const Csr& csr, const ClassBounds& cb, 
   const ArcTimes none{nullptr, nullptr};
   const uint8_t* need = nullptr;
   if (hp.bufs) {
-    enqueue_head_keys(st, csr, hp.asrc, hp.fdeg, hp.m, hp.m_dev, hp.bytes, *hp.bufs, d_tables,
-                      nullptr, ctr, launches);
+    enqueue_head_keys(st, csr, hp.asrc, hp.fdeg, hp.m, hp.m_dev, hp.bytes, hp.short_arcs, *hp.bufs,
+                      d_tables, nullptr, ctr, sink, launches);
     need = hp.bufs->need;
   }
   STC_CUDA(cudaMemsetAsync(ctr + C_WORK, 0, 8 * sizeof(uint64_t), st));
@@ -2439,7 +2555,8 @@ void count_persistent(stc_ctx* c, const Csr& csr, const ClassBounds& cb, uint32_
              ((uint64_t)hp.tuning.block_threads << 48) ^ ((uint64_t)hp.tuning.unroll[0] << 56) ^
              ((uint64_t)hp.tuning.unroll[1] << 58) ^ ((uint64_t)hp.tuning.unroll[2] << 60) ^
              ((uint64_t)hp.tuning.hash_factor[0] << 40) ^ ((uint64_t)hp.tuning.hash_factor[1] << 42) ^
-             ((uint64_t)hp.tuning.hash_factor[2] << 44) ^ ((uint64_t)hp.bytes << 62);
+             ((uint64_t)hp.tuning.hash_factor[2] << 44) ^ ((uint64_t)hp.bytes << 62) ^
+             ((uint64_t)hp.short_arcs << 63);
   static_assert(sizeof(PersistentKey) <= sizeof(c->graph_key), "graph key size");
   if (c->graph_exec && memcmp(c->graph_key, &key, sizeof(key)) == 0) {
     STC_CUDA(cudaGraphLaunch(c->graph_exec, st));
@@ -2699,6 +2816,11 @@ void count_triangles(stc_ctx* c, const DeviceGraph& gin, const CountConfig& cfg)
   const bool tiny =
       !timed && (cfg.strategy == STC_STRATEGY_AUTO || cfg.strategy == STC_STRATEGY_SEARCH);
   const ClassBounds cb{tiny ? kTinyMax : 1u, kWarpCap, kBlockCap, kLargeCap};
+  // Short arcs are counted where the head side's keys are made, unless a
+  // strategy is forced, arcs are timed or classes are counted one at a time.
+  const bool short_arcs =
+      head && !timed && cfg.strategy == STC_STRATEGY_AUTO && cfg.class_mask == 0x3Fu;
+  if (short_arcs) csr.short_max = kShortArc;
 
   // The persistent engine has no SPLIT path: counts that use SPLIT take the
   // per-class kernels.
@@ -2712,6 +2834,7 @@ void count_triangles(stc_ctx* c, const DeviceGraph& gin, const CountConfig& cfg)
       hp.fdeg = g.fdeg;
       hp.m = g.m_fwd;
       hp.bytes = !g.bytes_done;
+      hp.short_arcs = short_arcs;
       hp.m_dev = g.m_dev;
       hp.gbase = g.G ? g.gbase : nullptr;
       hp.G = g.G;
@@ -2730,10 +2853,18 @@ void count_triangles(stc_ctx* c, const DeviceGraph& gin, const CountConfig& cfg)
     }
     return;
   }
+  // Runs f with the sink of this count.
+  auto with_sink = [&](auto f) {
+    if (cfg.vertex_counts) f(VertexSink{(unsigned long long*)cfg.vertex_counts, g.verts});
+    else if (cfg.graph_counts) f(GraphSink{(unsigned long long*)cfg.graph_counts, g.gbase, g.G});
+    else f(TotalSink{});
+  };
   const uint8_t* need = nullptr;
   if (head) {
-    enqueue_head_keys(st, csr, g.asrc, g.fdeg, g.m_fwd, g.m_dev, !g.bytes_done, hb, d_table, range,
-                      ctr, c->launches);
+    with_sink([&](const auto& sink) {
+      enqueue_head_keys(st, csr, g.asrc, g.fdeg, g.m_fwd, g.m_dev, !g.bytes_done, short_arcs, hb,
+                        d_table, range, ctr, sink, c->launches);
+    });
     need = hb.need;
   }
   k_classify_count<<<kSMs * 4, 256, 0, st>>>(g.off, g.n, cb, ctr, range, need);
@@ -2768,15 +2899,8 @@ void count_triangles(stc_ctx* c, const DeviceGraph& gin, const CountConfig& cfg)
                              ctr, sink, at, c->tuning, c->launches, cfg.class_mask);
     }
   };
-  if (timed) {
-    run(TotalSink{}, std::true_type{});
-  } else if (cfg.vertex_counts) {
-    run(VertexSink{(unsigned long long*)cfg.vertex_counts, g.verts}, std::false_type{});
-  } else if (cfg.graph_counts) {
-    run(GraphSink{(unsigned long long*)cfg.graph_counts, g.gbase, g.G}, std::false_type{});
-  } else {
-    run(TotalSink{}, std::false_type{});
-  }
+  if (timed) run(TotalSink{}, std::true_type{});
+  else with_sink([&](const auto& sink) { run(sink, std::false_type{}); });
   STC_CUDA(cudaGetLastError());
 }
 
