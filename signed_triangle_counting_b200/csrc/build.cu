@@ -266,22 +266,33 @@ __global__ void k_csr_fill(const uint64_t* __restrict__ akeys, uint64_t ma, uint
   }
 }
 
-// Arc keys of a reference-layout CSR: one warp per vertex.
+// Arc keys of a reference-layout CSR: one warp per vertex.  Checks the CSR on
+// the way, before anything it holds is used as an index: offsets that decrease
+// or pass m, ranks that are no permutation of [0, n) (`seen` starts at 0) and
+// edges that leave the rank order set C_ERROR.
 __global__ void k_csr_arc_keys(const uint64_t* __restrict__ off, const uint32_t* __restrict__ edges,
                                const int8_t* __restrict__ signs, const uint32_t* __restrict__ rank,
-                               uint32_t n, uint32_t bits, uint64_t* __restrict__ akeys,
-                               uint32_t* __restrict__ fdeg, unsigned long long* __restrict__ ctr) {
+                               uint32_t n, uint64_t m, uint32_t bits, uint64_t* __restrict__ akeys,
+                               uint32_t* __restrict__ fdeg, uint32_t* __restrict__ seen,
+                               unsigned long long* __restrict__ ctr) {
   const uint32_t warps = gridDim.x * (blockDim.x / 32);
   for (uint32_t u = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5); u < n; u += warps) {
     const uint64_t b = off[u], e = off[u + 1];
     const uint32_t ru = rank[u];
+    bool bad = e < b || e > m || ru >= n;
+    if (lane_id() == 0 && ru < n) bad |= atomicExch(seen + ru, 1u) != 0;
+    if (__any_sync(kFull, bad)) {
+      if (lane_id() == 0) atomicExch(ctr + C_ERROR, 1ull);
+      continue;
+    }
     for (uint64_t i = b + lane_id(); i < e; i += 32) {
       const uint32_t w = edges[i];
-      if (w >= n || rank[w] <= ru) {
+      const uint32_t rw = w < n ? rank[w] : 0u;
+      if (rw <= ru || rw >= n) {  // ru >= 0: an id >= n fails too
         atomicExch(ctr + C_ERROR, 1ull);  // not a forward CSR of this rank order
         continue;
       }
-      akeys[i] = ((uint64_t)ru << bits) | rank[w] | ((uint64_t)(signs[i] < 0) << 63);
+      akeys[i] = ((uint64_t)ru << bits) | rw | ((uint64_t)(signs[i] < 0) << 63);
     }
     if (lane_id() == 0) fdeg[ru] = (uint32_t)(e - b);
   }
@@ -1241,17 +1252,22 @@ void graph_from_forward_csr(stc_ctx* c, uint32_t n, uint64_t m, const uint64_t* 
   mark(c, 1);
   mark(c, 2);
   mark(c, 3);
-  if (m) {
-    uint64_t* ka = buffer<uint64_t>(c, B_KEYS_A, m);
-    uint64_t* kb = buffer<uint64_t>(c, B_KEYS_B, m);
-    k_csr_arc_keys<<<kSMs * 8, kThreads, 0, st>>>(d_off, d_edges, d_signs, d_rank, n, g.bits, ka,
-                                                  g.fdeg, ctr);
+  uint64_t* ka = buffer<uint64_t>(c, B_KEYS_A, m);
+  uint64_t* kb = buffer<uint64_t>(c, B_KEYS_B, m);
+  if (n) {
+    uint32_t* seen = buffer<uint32_t>(c, B_DEG, n);
+    STC_CUDA(cudaMemsetAsync(seen, 0, (size_t)n * sizeof(uint32_t), st));
+    k_csr_arc_keys<<<kSMs * 8, kThreads, 0, st>>>(d_off, d_edges, d_signs, d_rank, n, m, g.bits, ka,
+                                                  g.fdeg, seen, ctr);
     c->launches++;
     read_counters(c, C_ERROR, 1);
     if (c->h_pinned[C_ERROR]) {
       fail(STC_ERR_INVALID_ARGUMENT,
-           "forward CSR has an edge that does not go from lower to higher rank or an id >= n");
+           "not a forward CSR: offsets decrease, rank is not a permutation of [0, n), an edge does "
+           "not go from lower to higher rank, or an id is >= n");
     }
+  }
+  if (m) {
     finish_csr_from_arc_keys(c, g, ka, kb);
   } else {
     g.off = buffer<uint64_t>(c, B_OFF, (size_t)n + 1);
