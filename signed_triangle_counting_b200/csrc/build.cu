@@ -325,7 +325,7 @@ void read_counters(stc_ctx* c, int first, int count) {
 
 // Rank-space CSR from unique keys: arc keys, sort, offsets, fill.
 void finish_csr_from_arc_keys(stc_ctx* c, DeviceGraph& g, uint64_t* akeys, uint64_t* alt) {
-  uint32_t* sort_ws = buffer<uint32_t>(c, B_SORT_WS, sort_workspace_words(g.m_fwd));
+  const SortSpace sort_ws = sort_space(c, g.m_fwd);
   uint64_t* sums = buffer<uint64_t>(c, B_SCAN_SUMS, kMaxSortGrid + 1);
   uint64_t* sorted = radix_sort(akeys, alt, g.m_fwd, 0, 2 * (int)g.bits, sort_ws, sort_error(c), c->stream,
                                 &c->launches);
@@ -935,7 +935,8 @@ void build_totals(stc_ctx* c, const EdgeIds& e, const int8_t* d_sign, uint64_t m
                   const BatchCaps* caps = nullptr) {
   cudaStream_t st = c->stream;
   unsigned long long* ctr = (unsigned long long*)counters(c);
-  uint32_t* sort_ws = buffer<uint32_t>(c, B_SORT_WS, std::max(sort_workspace_words(std::max<uint64_t>(m, g.n)), rank_workspace_words(g.n)));
+  const SortSpace sort_ws =
+      sort_space(c, std::max<uint64_t>(m, g.n), rank_workspace_words(g.n));
   uint64_t* sums = buffer<uint64_t>(c, B_SCAN_SUMS, kMaxSortGrid + 1);
   g.ukeys = nullptr;
   g.deg = buffer<uint32_t>(c, B_DEG, g.n);
@@ -967,9 +968,9 @@ void build_totals(stc_ctx* c, const EdgeIds& e, const int8_t* d_sign, uint64_t m
 
   if (g.n && !d_vbase) {
     const uint32_t tiles = (uint32_t)(((uint64_t)g.n + kRankTile - 1) / kRankTile);
-    STC_CUDA(cudaMemsetAsync(sort_ws, 0, rank_workspace_words(g.n) * sizeof(uint32_t), st));
-    k_degree_hist<<<grid_for(g.n, 16), kSortThreads, 0, st>>>(g.deg, g.n, sort_ws);
-    k_degree_rank<<<tiles, kSortThreads, 0, st>>>(g.deg, g.n, sort_ws, g.rank, sort_error(c));
+    STC_CUDA(cudaMemsetAsync(sort_ws.words, 0, rank_workspace_words(g.n) * sizeof(uint32_t), st));
+    k_degree_hist<<<grid_for(g.n, 16), kSortThreads, 0, st>>>(g.deg, g.n, sort_ws.words);
+    k_degree_rank<<<tiles, kSortThreads, 0, st>>>(g.deg, g.n, sort_ws.words, g.rank, sort_error(c));
     c->launches += 2;
   } else if (g.n) {
     uint64_t* va = buffer<uint64_t>(c, B_VKEYS_A, g.n);
@@ -1093,7 +1094,7 @@ __global__ void k_relabel(const uint32_t* __restrict__ u, const uint32_t* __rest
 // points *src / *dst at them; returns the number of distinct ids.
 uint64_t relabel_dense(stc_ctx* c, const uint32_t** src, const uint32_t** dst, uint64_t m) {
   cudaStream_t st = c->stream;
-  uint32_t* sort_ws = buffer<uint32_t>(c, B_SORT_WS, sort_workspace_words(2 * m));
+  const SortSpace sort_ws = sort_space(c, 2 * m);
   uint64_t* sums = buffer<uint64_t>(c, B_SCAN_SUMS, kMaxSortGrid + 1);
   uint64_t* ka = buffer<uint64_t>(c, B_KEYS_A, 2 * m);
   uint64_t* kb = buffer<uint64_t>(c, B_KEYS_B, 2 * m);
@@ -1170,7 +1171,7 @@ void build_graph(stc_ctx* c, const uint32_t* d_src, const uint32_t* d_dst, const
     build_totals(c, EdgeIds{d_src, d_dst, nullptr, nullptr, 0}, d_sign, m, g, nullptr, 0, hubs);
     return;
   }
-  uint32_t* sort_ws = buffer<uint32_t>(c, B_SORT_WS, sort_workspace_words(std::max<uint64_t>(m, g.n)));
+  const SortSpace sort_ws = sort_space(c, std::max<uint64_t>(m, g.n));
   uint64_t* sums = buffer<uint64_t>(c, B_SCAN_SUMS, kMaxSortGrid + 1);
 
   // 2. dedup.
@@ -1318,7 +1319,7 @@ void build_graph_batch(stc_ctx* c, const uint32_t* d_src, const uint32_t* d_dst,
     build_totals(c, EdgeIds{d_src, d_dst, d_eoff, d_vbase, G}, d_sign, m, g, d_vbase, G);
     return;
   }
-  uint32_t* sort_ws = buffer<uint32_t>(c, B_SORT_WS, sort_workspace_words(std::max<uint64_t>(m, g.n)));
+  const SortSpace sort_ws = sort_space(c, std::max<uint64_t>(m, g.n));
   uint64_t* sums = buffer<uint64_t>(c, B_SCAN_SUMS, kMaxSortGrid + 1);
 
   // 2. dedup over the union.
@@ -1435,7 +1436,7 @@ void export_forward_csr(stc_ctx* c, const DeviceGraph& g, stc_forward_csr* out) 
   uint64_t* off_id = buffer<uint64_t>(c, B_EXPORT_OFF, (size_t)n + 1);
   uint64_t* ka = buffer<uint64_t>(c, B_KEYS_A, mu);
   uint64_t* kb = buffer<uint64_t>(c, B_KEYS_B, mu);
-  uint32_t* sort_ws = buffer<uint32_t>(c, B_SORT_WS, sort_workspace_words(mu));
+  const SortSpace sort_ws = sort_space(c, mu);
   uint64_t* sums = buffer<uint64_t>(c, B_SCAN_SUMS, kMaxSortGrid + 1);
   uint32_t* edges = buffer<uint32_t>(c, B_NBR, mu);
   int8_t* signs = buffer<int8_t>(c, B_SGN, mu);

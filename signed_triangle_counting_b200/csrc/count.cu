@@ -2240,7 +2240,7 @@ struct HeadBufs {
   uint32_t* runs = nullptr;  // end of each head's run (n)
   HeadLists lists{};         // the classes' work items
   uint8_t* need = nullptr;   // per tail: it keeps arcs for the tail side
-  uint32_t* sort_ws = nullptr;
+  SortSpace sort_ws;
   HeadStream stream{};       // the arcs as the bitmap classes stream them
 };
 
@@ -2256,7 +2256,7 @@ HeadBufs head_buffers(stc_ctx* c, const DeviceGraph& g) {
   b.lists.base = buffer<uint32_t>(c, B_HEAD_LIST, 3 * items + (g.n + 3) / 4);
   b.lists.cap = (uint32_t)items;
   b.need = reinterpret_cast<uint8_t*>(b.lists.base + 3 * items);
-  b.sort_ws = buffer<uint32_t>(c, B_SORT_WS, sort_workspace_words(g.m_fwd));
+  b.sort_ws = sort_space(c, g.m_fwd);
   b.stream.low = buffer<uint16_t>(c, B_HEAD_LOW, (g.m_fwd + 7) / 8 * 8);
   b.stream.sbits = buffer<uint8_t>(c, B_SBITS, (g.m_fwd + 7) / 8);
   return b;
@@ -2553,7 +2553,7 @@ void count_persistent(stc_ctx* c, const Csr& csr, const ClassBounds& cb, uint32_
   key.v[2] = s2;
   key.v[3] = reinterpret_cast<uint64_t>(s1);
   key.v[4] = hp.m;
-  key.v[5] = reinterpret_cast<uint64_t>(hb.sort_ws) ^
+  key.v[5] = reinterpret_cast<uint64_t>(hb.sort_ws.words) ^
              ((uint64_t)hp.tuning.block_threads << 48) ^ ((uint64_t)hp.tuning.unroll[0] << 56) ^
              ((uint64_t)hp.tuning.unroll[1] << 58) ^ ((uint64_t)hp.tuning.unroll[2] << 60) ^
              ((uint64_t)hp.tuning.hash_factor[0] << 40) ^ ((uint64_t)hp.tuning.hash_factor[1] << 42) ^

@@ -17,9 +17,11 @@
 // Bits of the key outside [lo, hi) ride along untouched, which is how the
 // edge sign travels in bit 63 without a separate payload array.
 #pragma once
+#include <algorithm>
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "internal.h"
 #include "stc_device.cuh"
 
 namespace stc {
@@ -60,11 +62,9 @@ constexpr uint32_t kSortStates = kSortTickets + 2 * kMaxPasses;
 // take smaller tiles, which spreads them over more SMs and shortens each
 // CTA's serial part (a pass over 100,000 keys takes 12 us, over 1,000,000
 // 19 us, over 2,400,000 32 us).
-inline int sort_items(uint64_t m) {
-  return m > (uint64_t)kSMs * 8 * kSortThreads * 8   ? 16
-         : m > (uint64_t)kSMs * 4 * kSortThreads * 4 ? 8
-                                                     : 4;
-}
+constexpr uint64_t kSortMax4 = (uint64_t)kSMs * 4 * kSortThreads * 4;  // the largest sort of 4,
+constexpr uint64_t kSortMax8 = (uint64_t)kSMs * 8 * kSortThreads * 8;  // and of 8 keys a thread
+inline int sort_items(uint64_t m) { return m > kSortMax8 ? 16 : m > kSortMax4 ? 8 : 4; }
 inline uint64_t sort_tiles(uint64_t m) {
   const uint64_t tile = (uint64_t)kSortThreads * sort_items(m);
   return (m + tile - 1) / tile;
@@ -72,8 +72,24 @@ inline uint64_t sort_tiles(uint64_t m) {
 // A tile state holds a count of keys and two flag bits: 32 bits a word while
 // counts stay below 2^30, else 64.
 inline bool sort_wide(uint64_t m) { return m >= (1ull << 30); }
-inline size_t sort_workspace_words(uint64_t m) {
+// What a sort of m keys clears and publishes.
+inline size_t sort_words(uint64_t m) {
   return kSortStates + 2 * (size_t)kRadix * sort_tiles(m) * (sort_wide(m) ? 2 : 1);
+}
+// The workspace of a sort of m keys or of any fewer: one key past a limit
+// above halves the tiles, so the largest sorts of the smaller tiles count too.
+inline size_t sort_workspace_words(uint64_t m) {
+  return std::max({sort_words(m), sort_words(std::min(m, kSortMax4)),
+                   sort_words(std::min(m, kSortMax8))});
+}
+struct SortSpace {
+  uint32_t* words = nullptr;
+  size_t count = 0;
+};
+// The context's workspace for sorts of at most m keys (and at least `words`).
+inline SortSpace sort_space(stc_ctx* c, uint64_t m, size_t words = 0) {
+  const size_t n = std::max(words, sort_workspace_words(m));
+  return SortSpace{buffer<uint32_t>(c, B_SORT_WS, n), n};
 }
 
 // Digit counts of every pass over [lo, hi) into ws[pass][digit]; the last CTA
@@ -344,15 +360,17 @@ inline void launch_radix_pass(const uint64_t* in, uint64_t* out, uint64_t m, int
 }
 
 // Sorts keys[0, m) by bits [lo, hi) stably; returns the buffer that holds the
-// result (`keys` or `alt`).  m must be below 2^32.  `ws` holds
-// sort_workspace_words(m) words; `err` receives 2 if a device-side wait
-// expired.  With `m_dev`, the sort covers only the first min(m, *m_dev) keys,
+// result (`keys` or `alt`).  m must be below 2^32.  `space` is checked to hold
+// sort_words(m) words before anything is launched; `err` receives 2 if a
+// device-side wait expired.  With `m_dev`, the sort covers only the first min(m, *m_dev) keys,
 // a count known on the device alone (the launches are sized for m, so the
 // sequence can be captured).
 inline uint64_t* radix_sort(uint64_t* keys, uint64_t* alt, uint64_t m, int lo, int hi,
-                            uint32_t* ws, unsigned long long* err, cudaStream_t st,
+                            const SortSpace& space, unsigned long long* err, cudaStream_t st,
                             int* launches = nullptr, const unsigned long long* m_dev = nullptr) {
   if (m <= 1 || hi <= lo) return keys;
+  if (space.count < sort_words(m)) fail(STC_ERR_INTERNAL, "sort workspace too small");
+  uint32_t* ws = space.words;
   const uint64_t tiles = sort_tiles(m);
   const int items = sort_items(m);
   const bool wide = sort_wide(m);
