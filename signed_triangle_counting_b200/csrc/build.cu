@@ -1047,7 +1047,7 @@ void build_totals(stc_ctx* c, const EdgeIds& e, const int8_t* d_sign, uint64_t m
 
 // ---------------------------------------------------- dense relabel ----
 // Counts of totals accept any 32-bit id: an edge list whose largest id
-// reaches 2^31 - 1 (where the engine's signed keys and ranks would not fit)
+// reaches 2^31 - 2 (the engine's signed keys and ranks stay below it)
 // is relabelled to dense ids first, the index of each id among the list's
 // distinct ids.  The relabelling keeps the ids' order, so the graph, its
 // (degree, id) order and its counts are those of the original list.
@@ -1107,7 +1107,7 @@ uint64_t relabel_dense(stc_ctx* c, const uint32_t** src, const uint32_t** dst, u
                            cudaMemcpyDeviceToHost, st));
   STC_CUDA(cudaStreamSynchronize(st));
   const uint64_t nd = c->h_pinned[C_WORK];
-  if (nd >= (1ull << 31) - 1)
+  if (nd > kMaxVertices)
     fail(STC_ERR_LIMIT, std::to_string(nd) + " distinct vertex ids >= 2^31 - 1");
   uint32_t* ids = buffer<uint32_t>(c, B_DISTINCT, nd);
   range_apply(flag, DistinctEmit{sorted, ids}, 2 * m, sums, st, &c->launches);
@@ -1156,11 +1156,13 @@ void build_graph(stc_ctx* c, const uint32_t* d_src, const uint32_t* d_dst, const
   read_counters(c, C_MAX_ID, 2);
   uint64_t max_id = c->h_pinned[C_MAX_ID];
   const uint64_t self = c->h_pinned[C_SELF];
-  // Ids (and ranks) stay below 2^31 - 1: the engine keeps a sign in bit 31.
-  // Counts of totals relabel larger ids to dense ones; the other paths
-  // report results by id and keep the limit.
-  if (max_id >= (1ull << 31) - 1) {
-    if (!totals) fail(STC_ERR_LIMIT, "vertex id " + std::to_string(max_id) + " >= 2^31 - 1");
+  // Ranks stay below 2^31 - 2 where triangles are counted (kMaxVertices).
+  // Counts of totals relabel larger ids to dense ones; the other paths report
+  // by id and refuse them, 2^31 - 2 itself only where they count (a forward
+  // CSR may hold it).
+  if (!totals && max_id > kMaxVertices)
+    fail(STC_ERR_LIMIT, "vertex id " + std::to_string(max_id) + " >= 2^31 - 1");
+  if (max_id >= kMaxVertices && totals) {
     max_id = relabel_dense(c, &d_src, &d_dst, m) - 1;
     hubs = nullptr;  // named by the ids of the list as given
   }
@@ -1246,7 +1248,7 @@ void graph_from_forward_csr(stc_ctx* c, uint32_t n, uint64_t m, const uint64_t* 
   g.n = n;
   g.m_input = g.m_valid = g.m_unique = g.m_fwd = m;
   if (m >= (1ull << 32)) fail(STC_ERR_LIMIT, "forward CSR has 2^32 or more edges");
-  if (n >= (1u << 31) - 1) fail(STC_ERR_LIMIT, "forward CSR has 2^31 - 1 or more vertices");
+  if (n > kMaxVertices) fail(STC_ERR_LIMIT, "forward CSR has 2^31 - 1 or more vertices");
   g.bits = std::max<uint32_t>(1, bit_width64(n ? n - 1 : 0));
   g.rank = const_cast<uint32_t*>(d_rank);
   g.fdeg = buffer<uint32_t>(c, B_FDEG, n);
@@ -1307,7 +1309,7 @@ void build_graph_batch(stc_ctx* c, const uint32_t* d_src, const uint32_t* d_dst,
   std::vector<uint64_t> vbase(G + 1, 0);
   for (uint32_t i = 0; i < G; i++) vbase[i + 1] = vbase[i] + space[i];
   const uint64_t ntot = vbase[G];
-  if (ntot >= (1ull << 31) - 1)
+  if (ntot > kMaxVertices)
     fail(STC_ERR_LIMIT, "batch has 2^31 - 1 or more vertices in total");
   STC_CUDA(cudaMemcpyAsync(d_vbase, vbase.data(), (G + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice,
                            st));

@@ -2788,6 +2788,7 @@ void build_split(stc_ctx* c, DeviceGraph& g) {
 
 void count_triangles(stc_ctx* c, const DeviceGraph& gin, const CountConfig& cfg) {
   if (gin.n == 0 || gin.m_fwd == 0) return;
+  if (gin.n > kMaxVertices) fail(STC_ERR_LIMIT, "counts need vertex ids below 2^31 - 2");
   cudaStream_t st = c->stream;
   DeviceGraph g = gin;
   const bool split = cfg.strategy == STC_STRATEGY_SPLIT ||

@@ -51,9 +51,9 @@ enum BufId {
   B_NKEY,                         // arcs: head << 1 | negative (m + 8)
   B_SBITS,                        // arcs: sign bits, one byte per 8 arcs (the head bitmaps' stream)
   B_HEAD_LOW,                     // arcs: low 16 bits of the heads (the same)
-  B_RELABEL,                      // ids >= 2^31 - 1: the edges relabelled to dense ids (2 m)
+  B_RELABEL,                      // ids >= 2^31 - 2: the edges relabelled to dense ids (2 m)
   B_HUBS,                         // ids with very many edges (totals path)
-  B_DISTINCT,                     // ids >= 2^31 - 1: the sorted distinct ids
+  B_DISTINCT,                     // ids >= 2^31 - 2: the sorted distinct ids
   B_COUNT_
 };
 
@@ -84,6 +84,10 @@ enum CounterSlot {
   C_HEAD_QUEUE = 41,           // and the classes' work queues (5 slots)
   C_SLOTS = 46
 };
+
+// Vertices a graph may have where it is counted: the engine pads streams with
+// the id 2^31 - 2 (kNoId in count.cu), which no rank may equal.
+constexpr uint64_t kMaxVertices = (1ull << 31) - 2;
 
 // Values of the device error word: 1 = malformed forward CSR,
 // 2 = a bounded device-side wait expired, 3 = a list exceeded its staged
