@@ -641,12 +641,14 @@ __device__ __forceinline__ uint32_t degree_digit(uint32_t d) {
 // One graph's ranks in (degree digit, id) order without moving a key: the
 // counts of the digits, then one pass like the radix sort's whose output is
 // each vertex's position.  ws is a sort workspace; the last CTA of the count
-// turns the counts into each digit's first rank.
+// turns the counts into each digit's first rank.  From 2^30 vertices on the
+// tile states are 64 bits wide, as the sort's.
 constexpr int kRankItems = 16;
 constexpr uint32_t kRankTile = kSortThreads * kRankItems;
 
 inline size_t rank_workspace_words(uint32_t n) {
-  return kSortStates + (size_t)kRadix * (((uint64_t)n + kRankTile - 1) / kRankTile);
+  const uint64_t tiles = ((uint64_t)n + kRankTile - 1) / kRankTile;
+  return kSortStates + (size_t)kRadix * tiles * (sort_wide(n) ? 2 : 1);
 }
 
 __global__ void __launch_bounds__(kSortThreads) k_degree_hist(const uint32_t* __restrict__ deg,
@@ -673,11 +675,12 @@ __global__ void __launch_bounds__(kSortThreads) k_degree_hist(const uint32_t* __
   ws[tid] = block_exclusive_scan<kSortThreads>(c, scan_tmp, total);
 }
 
+template <class W>
 __global__ void __launch_bounds__(kSortThreads, 4) k_degree_rank(const uint32_t* __restrict__ deg,
                                                                  uint32_t n, uint32_t* __restrict__ ws,
                                                                  uint32_t* __restrict__ rank,
                                                                  unsigned long long* __restrict__ err) {
-  using TS = TileState<uint32_t>;
+  using TS = TileState<W>;
   __shared__ uint32_t mask[2][kSortWarps][kRadix];
   __shared__ uint32_t whist[kSortWarps][kRadix];
   __shared__ uint32_t s_tile, s_abort;
@@ -714,9 +717,9 @@ __global__ void __launch_bounds__(kSortThreads, 4) k_degree_rank(const uint32_t*
     cnt += c[w];
   }
   if (tid == kRadix - 1) cnt -= kRankTile - valid;  // past the end: the last digit
-  uint32_t* own = ws + kSortStates + (size_t)tile * kRadix + tid;
+  W* own = reinterpret_cast<W*>(ws + kSortStates) + (size_t)tile * kRadix + tid;
   TS::put(own, (tile == 0 ? TS::kPrefix : TS::kLocal) | cnt);
-  uint32_t run = ws[tid] + look_back(own, tile, cnt, ws, s_abort);
+  uint32_t run = ws[tid] + (uint32_t)look_back(own, tile, cnt, ws, s_abort);
 #pragma unroll
   for (int w = 0; w < kSortWarps; w++) {
     whist[w][tid] = run;
@@ -970,7 +973,8 @@ void build_totals(stc_ctx* c, const EdgeIds& e, const int8_t* d_sign, uint64_t m
     const uint32_t tiles = (uint32_t)(((uint64_t)g.n + kRankTile - 1) / kRankTile);
     STC_CUDA(cudaMemsetAsync(sort_ws.words, 0, rank_workspace_words(g.n) * sizeof(uint32_t), st));
     k_degree_hist<<<grid_for(g.n, 16), kSortThreads, 0, st>>>(g.deg, g.n, sort_ws.words);
-    k_degree_rank<<<tiles, kSortThreads, 0, st>>>(g.deg, g.n, sort_ws.words, g.rank, sort_error(c));
+    auto rank = sort_wide(g.n) ? k_degree_rank<uint64_t> : k_degree_rank<uint32_t>;
+    rank<<<tiles, kSortThreads, 0, st>>>(g.deg, g.n, sort_ws.words, g.rank, sort_error(c));
     c->launches += 2;
   } else if (g.n) {
     uint64_t* va = buffer<uint64_t>(c, B_VKEYS_A, g.n);

@@ -1,6 +1,7 @@
-"""Counts whose ids reach the id that pads the engine's streams (2^31 - 2):
-totals against the oracle on the same edges with dense ids, in the same order;
-shards, which report by rank, refuse it."""
+"""Counts whose ids lie on both sides of 2^30, from where on a tile's count of
+vertices no longer fits a 32-bit state, or reach the id that pads the engine's
+streams (2^31 - 2): totals against the oracle on the same edges with dense ids,
+in the same order; shards, which report by rank, refuse the last."""
 import numpy as np
 import pytest
 
@@ -10,7 +11,8 @@ import signed_triangle_counting_b200 as stc
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("top", [(1 << 31) - 2])
+@pytest.mark.parametrize("top", [(1 << 30) - 1, 1 << 30, (1 << 30) + 5000,
+                                 (1 << 31) - 3, (1 << 31) - 2])
 def test_ids_around_2_30(top):
     # Vertices in pairs about 2^30 apart, edges among neighbours in a random
     # order of them, and the top id.
