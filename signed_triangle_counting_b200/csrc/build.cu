@@ -1268,11 +1268,12 @@ void graph_from_forward_csr(stc_ctx* c, uint32_t n, uint64_t m, const uint64_t* 
                                                   g.fdeg, seen, ctr);
     c->launches++;
     read_counters(c, C_ERROR, 1);
-    if (c->h_pinned[C_ERROR]) {
+    if (c->h_pinned[C_ERROR] == kDeviceErrCsr) {
       fail(STC_ERR_INVALID_ARGUMENT,
            "not a forward CSR: offsets decrease, rank is not a permutation of [0, n), an edge does "
            "not go from lower to higher rank, or an id is >= n");
     }
+    check_device_error(c->h_pinned[C_ERROR]);
   }
   if (m) {
     finish_csr_from_arc_keys(c, g, ka, kb);

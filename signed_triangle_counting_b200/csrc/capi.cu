@@ -28,6 +28,20 @@ void cuda_check(cudaError_t e, const char* what) {
 
 uint64_t* counters(stc_ctx* c) { return buffer<uint64_t>(c, B_COUNTERS, C_SLOTS); }
 
+void clear_counters(stc_ctx* c) {
+  STC_CUDA(cudaMemsetAsync(counters(c), 0, C_SLOTS * sizeof(uint64_t), c->stream));
+  if (c->preset_error)
+    STC_CUDA(cudaMemsetAsync(counters(c) + C_ERROR, (int)c->preset_error, 1, c->stream));
+}
+
+void check_device_error(uint64_t word) {
+  if (word == 0) return;
+  fail(word == kDeviceErrTimeout ? STC_ERR_DEVICE_TIMEOUT
+       : word == kDeviceErrCsr   ? STC_ERR_INVALID_ARGUMENT
+                                 : STC_ERR_INTERNAL,
+       "device reported error word " + std::to_string(word));
+}
+
 void mark(stc_ctx* c, int slot) {
   if (!c->timing) return;
   // Inside a capture the event becomes a node of the graph that records it
@@ -108,7 +122,7 @@ void begin_call(stc_ctx* c, const stc_opts* o) {
   c->timing = o && (o->flags & STC_F_TIMING);
   c->launches = 0;
   c->stats = stc_stats{};
-  STC_CUDA(cudaMemsetAsync(counters(c), 0, C_SLOTS * sizeof(uint64_t), c->stream));
+  clear_counters(c);
   mark(c, 0);
 }
 
@@ -124,11 +138,7 @@ void end_call(stc_ctx* c, const DeviceGraph& g, stc_counts* out) {
                            cudaMemcpyDeviceToHost, c->stream));
   STC_CUDA(cudaStreamSynchronize(c->stream));
   STC_CUDA(cudaGetLastError());
-  if (c->h_pinned[C_ERROR]) {
-    const uint64_t e = c->h_pinned[C_ERROR];
-    fail(e == kDeviceErrTimeout ? STC_ERR_DEVICE_TIMEOUT : STC_ERR_INTERNAL,
-         "device reported error word " + std::to_string(e));
-  }
+  check_device_error(c->h_pinned[C_ERROR]);
   if (out) {
     out->t0 = c->h_pinned[C_T0];
     out->t1 = c->h_pinned[C_T1];
@@ -247,7 +257,7 @@ struct GroupOut {
 GroupOut eager_group(stc_ctx* c, const DeviceInput& in, uint64_t me,
                      const std::vector<uint64_t>& eoff, uint32_t gn, CountConfig cfg,
                      std::vector<uint64_t>& h, DeviceGraph& g) {
-  STC_CUDA(cudaMemsetAsync(counters(c), 0, C_SLOTS * sizeof(uint64_t), c->stream));
+  clear_counters(c);
   build_graph_batch(c, in.src, in.dst, in.sign, me, eoff.data(), gn, g, /*totals=*/true);
   uint64_t* gc = buffer<uint64_t>(c, B_BATCH_COUNTS, 4ull * gn);
   STC_CUDA(cudaMemsetAsync(gc, 0, 4ull * gn * sizeof(uint64_t), c->stream));
@@ -261,7 +271,7 @@ GroupOut eager_group(stc_ctx* c, const DeviceInput& in, uint64_t me,
 // The capturable sequence of a group at capacities `caps`.
 void enqueue_capped_group(stc_ctx* c, const DeviceInput& in, uint64_t me, uint32_t gn,
                           const BatchCaps& caps, CountConfig cfg) {
-  STC_CUDA(cudaMemsetAsync(counters(c), 0, C_SLOTS * sizeof(uint64_t), c->stream));
+  clear_counters(c);
   uint64_t* gc = buffer<uint64_t>(c, B_BATCH_COUNTS, 4ull * gn);
   STC_CUDA(cudaMemsetAsync(gc, 0, 4ull * gn * sizeof(uint64_t), c->stream));
   DeviceGraph g;
@@ -749,8 +759,7 @@ stc_status stc_count_batch_packed(stc_ctx* c, const uint32_t* src, const uint32_
       }
       std::vector<uint64_t> h(4ull * gn);
       const GroupOut go = count_group(c, in, me, eoff, gn, cfg, h);
-      if (c->h_pinned[C_ERROR])
-        fail(STC_ERR_INTERNAL, "device reported error word " + std::to_string(c->h_pinned[C_ERROR]));
+      check_device_error(c->h_pinned[C_ERROR]);
       if (c->timing) {  // stage times summed over the groups
         total.ms_dedup += elapsed(c, 1, 2);
         total.ms_orient += elapsed(c, 2, 3);
@@ -941,6 +950,12 @@ stc_status stc_ctx_get_tuning(const stc_ctx* c, stc_tuning* out) {
   return STC_OK;
 }
 
+stc_status stc_test_preset_error(stc_ctx* c, uint32_t word) {
+  if (!c || word > 255) return STC_ERR_INVALID_ARGUMENT;
+  c->preset_error = word;
+  return STC_OK;
+}
+
 stc_status stc_autotune(stc_ctx* c, const uint32_t* src, const uint32_t* dst, const int8_t* sign,
                         uint64_t m, const stc_opts* o, uint32_t reps, stc_tuning* out) {
   if (!c || !out || reps == 0 || reps > 100) return STC_ERR_INVALID_ARGUMENT;
@@ -996,8 +1011,7 @@ stc_status stc_autotune(stc_ctx* c, const uint32_t* src, const uint32_t* dst, co
           }
           uint64_t got[C_SLOTS];
           STC_CUDA(cudaMemcpy(got, counters(c), sizeof(got), cudaMemcpyDeviceToHost));
-          if (got[C_ERROR])
-            fail(STC_ERR_INTERNAL, "device reported error word " + std::to_string(got[C_ERROR]));
+          check_device_error(got[C_ERROR]);
           if (first) {
             memcpy(want, got, sizeof(want));
           } else if (memcmp(want, got, sizeof(want)) != 0) {

@@ -175,6 +175,7 @@ struct stc_ctx {
   cudaGraphExec_t graph_exec = nullptr;
   uint64_t graph_key[32] = {};
   int graph_launches = 0;  // kernels per replay of graph_exec
+  uint32_t preset_error = 0;  // device error word a call starts with (tests; 0 = none)
   stc::Tuning tuning;
   stc::HostCopier copier;  // staging of pageable host memory
   // Batch groups captured whole (at most four, the least recently used
@@ -342,5 +343,13 @@ void train_dispatcher(stc_ctx* c, const float* features, const float* targets,
                       uint64_t seed, float* params, float* loss);
 
 uint64_t* counters(stc_ctx* c);
+// Zeroes the counters, in stream order, before a count or a batch group.
+void clear_counters(stc_ctx* c);
+// Fails with the status of a device error word that is not 0.
+void check_device_error(uint64_t word);
 
 }  // namespace stc
+
+// For tests: the context's next calls start with this device error word (0 to
+// 255; 0 ends it), as if a kernel before them had set it.
+extern "C" stc_status stc_test_preset_error(stc_ctx* c, uint32_t word);
