@@ -189,7 +189,8 @@ __global__ void k_vertex_keys(const uint32_t* __restrict__ deg, uint32_t n,
 }
 
 __global__ void k_rank(const uint64_t* __restrict__ vkeys, uint32_t n, uint32_t* __restrict__ verts,
-                       uint32_t* __restrict__ rank) {
+                       uint32_t* __restrict__ rank, const unsigned long long* __restrict__ err) {
+  if (device_failed(err)) return;
   const uint32_t stride = gridDim.x * blockDim.x;
   for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += stride) {
     const uint32_t id = (uint32_t)vkeys[r];
@@ -202,7 +203,9 @@ __global__ void k_rank(const uint64_t* __restrict__ vkeys, uint32_t n, uint32_t*
 // bit 63; out-degree histogram by rank.
 __global__ void k_arc_keys(const uint64_t* __restrict__ ukeys, uint64_t mu, uint32_t bits,
                            const uint32_t* __restrict__ rank, uint64_t* __restrict__ akeys,
-                           uint32_t* __restrict__ fdeg) {
+                           uint32_t* __restrict__ fdeg,
+                           const unsigned long long* __restrict__ err) {
+  if (device_failed(err)) return;
   const uint64_t idmask = (1ull << bits) - 1;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < mu; i += stride) {
@@ -246,6 +249,7 @@ __global__ void k_csr_fill(const uint64_t* __restrict__ akeys, uint64_t ma, uint
                            uint32_t* __restrict__ nbr, int8_t* __restrict__ sgn,
                            uint32_t* __restrict__ asrc, uint32_t* __restrict__ nkey,
                            unsigned long long* __restrict__ ctr) {
+  if (device_failed(ctr + C_ERROR)) return;
   const uint64_t idmask = (1ull << bits) - 1;
   unsigned long long bytes = 0, probe = 0;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
@@ -314,7 +318,8 @@ __global__ void k_export_keys(const uint64_t* __restrict__ ukeys, uint64_t mu, u
   }
 }
 
-// Where a sort reports a device-side wait that expired.
+// Where a sort reports a device-side wait that expired, and where its
+// consumers look.
 unsigned long long* sort_error(stc_ctx* c) { return (unsigned long long*)counters(c) + C_ERROR; }
 
 void read_counters(stc_ctx* c, int first, int count) {
@@ -323,10 +328,20 @@ void read_counters(stc_ctx* c, int first, int count) {
   STC_CUDA(cudaStreamSynchronize(c->stream));
 }
 
+// The total of a range scan over sorted keys (range_reduce_scan with err),
+// read to the host; fails if the sort did.
+uint64_t read_total(stc_ctx* c, const uint64_t* sums, uint32_t grid) {
+  STC_CUDA(cudaMemcpyAsync(c->h_pinned + C_WORK, sums + grid, 2 * sizeof(uint64_t),
+                           cudaMemcpyDeviceToHost, c->stream));
+  STC_CUDA(cudaStreamSynchronize(c->stream));
+  check_device_error(c->h_pinned[C_WORK + 1]);
+  return c->h_pinned[C_WORK];
+}
+
 // Rank-space CSR from unique keys: arc keys, sort, offsets, fill.
 void finish_csr_from_arc_keys(stc_ctx* c, DeviceGraph& g, uint64_t* akeys, uint64_t* alt) {
   const SortSpace sort_ws = sort_space(c, g.m_fwd);
-  uint64_t* sums = buffer<uint64_t>(c, B_SCAN_SUMS, kMaxSortGrid + 1);
+  uint64_t* sums = buffer<uint64_t>(c, B_SCAN_SUMS, kScanSums);
   uint64_t* sorted = radix_sort(akeys, alt, g.m_fwd, 0, 2 * (int)g.bits, sort_ws, sort_error(c), c->stream,
                                 &c->launches);
   g.off = buffer<uint64_t>(c, B_OFF, (size_t)g.n + 1);
@@ -726,7 +741,7 @@ __global__ void __launch_bounds__(kSortThreads, 4) k_degree_rank(const uint32_t*
     run += c[w];
   }
   __syncthreads();
-  if (s_abort && tid == 0) atomicExch(err, 2ull);
+  if (s_abort && tid == 0) atomicExch(err, (unsigned long long)kDeviceErrTimeout);
 #pragma unroll
   for (int j = 0; j < kRankItems; j++) {
     const uint32_t i = wbase + 32 * j;
@@ -826,6 +841,7 @@ __global__ void k_alg_bytes(const uint32_t* __restrict__ asrc, const uint32_t* _
                             uint64_t m, const unsigned long long* __restrict__ m_dev,
                             const uint64_t* __restrict__ off, const uint32_t* __restrict__ fdeg,
                             unsigned long long* __restrict__ ctr) {
+  if (device_failed(ctr + C_ERROR)) return;
   if (m_dev) m = min(m, (uint64_t)*m_dev);
   unsigned long long bytes = 0, probe = 0;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
@@ -940,7 +956,7 @@ void build_totals(stc_ctx* c, const EdgeIds& e, const int8_t* d_sign, uint64_t m
   unsigned long long* ctr = (unsigned long long*)counters(c);
   const SortSpace sort_ws =
       sort_space(c, std::max<uint64_t>(m, g.n), rank_workspace_words(g.n));
-  uint64_t* sums = buffer<uint64_t>(c, B_SCAN_SUMS, kMaxSortGrid + 1);
+  uint64_t* sums = buffer<uint64_t>(c, B_SCAN_SUMS, kScanSums);
   g.ukeys = nullptr;
   g.deg = buffer<uint32_t>(c, B_DEG, g.n);
   g.rank = buffer<uint32_t>(c, B_RANK, g.n);
@@ -986,7 +1002,7 @@ void build_totals(stc_ctx* c, const EdgeIds& e, const int8_t* d_sign, uint64_t m
                                                       gbits, va);
     uint64_t* vs = radix_sort(va, vb, g.n, 32, (int)(32 + dbits + gbits), sort_ws, sort_error(c), st,
                               &c->launches);
-    k_rank<<<grid_for(g.n, 4), kThreads, 0, st>>>(vs, g.n, nullptr, g.rank);
+    k_rank<<<grid_for(g.n, 4), kThreads, 0, st>>>(vs, g.n, nullptr, g.rank, sort_error(c));
     c->launches += 2;
   }
   STC_CUDA(cudaGetLastError());
@@ -1004,7 +1020,8 @@ void build_totals(stc_ctx* c, const EdgeIds& e, const int8_t* d_sign, uint64_t m
     const uint64_t mask = (1ull << (2 * g.bits)) - 1;
     if (caps) {
       const UniqueArcFlag flag{sorted, mask};
-      const uint32_t grid = range_reduce_scan(flag, m, sums, st, &c->launches);
+      // No arcs after an expired wait: the kernels below are bounded by their number.
+      const uint32_t grid = range_reduce_scan(flag, m, sums, st, &c->launches, sort_error(c));
       STC_CUDA(cudaMemcpyAsync(ctr + C_BATCH_MU, sums + grid, sizeof(uint64_t),
                                cudaMemcpyDeviceToDevice, st));
       g.m_unique = g.m_fwd = m;
@@ -1018,11 +1035,9 @@ void build_totals(stc_ctx* c, const EdgeIds& e, const int8_t* d_sign, uint64_t m
     } else {
       // Self-loops sorted last: the first m_valid keys are the real arcs.
       const UniqueFlag flag{sorted, mask};
-      const uint32_t grid = range_reduce_scan(flag, g.m_valid, sums, st, &c->launches);
-      STC_CUDA(cudaMemcpyAsync(c->h_pinned + C_WORK, sums + grid, sizeof(uint64_t),
-                               cudaMemcpyDeviceToHost, st));
-      STC_CUDA(cudaStreamSynchronize(st));
-      g.m_unique = g.m_fwd = c->h_pinned[C_WORK];
+      const uint32_t grid =
+          range_reduce_scan(flag, g.m_valid, sums, st, &c->launches, sort_error(c));
+      g.m_unique = g.m_fwd = read_total(c, sums, grid);
       g.nbr = buffer<uint32_t>(c, B_NBR, g.m_fwd + 8);  // + 8: the engine reads whole 32-byte chunks
       g.sgn = buffer<int8_t>(c, B_SGN, g.m_fwd + 8);
       g.asrc = buffer<uint32_t>(c, B_ASRC, g.m_fwd);
@@ -1099,18 +1114,15 @@ __global__ void k_relabel(const uint32_t* __restrict__ u, const uint32_t* __rest
 uint64_t relabel_dense(stc_ctx* c, const uint32_t** src, const uint32_t** dst, uint64_t m) {
   cudaStream_t st = c->stream;
   const SortSpace sort_ws = sort_space(c, 2 * m);
-  uint64_t* sums = buffer<uint64_t>(c, B_SCAN_SUMS, kMaxSortGrid + 1);
+  uint64_t* sums = buffer<uint64_t>(c, B_SCAN_SUMS, kScanSums);
   uint64_t* ka = buffer<uint64_t>(c, B_KEYS_A, 2 * m);
   uint64_t* kb = buffer<uint64_t>(c, B_KEYS_B, 2 * m);
   k_endpoint_keys<<<grid_for(m, 4), kThreads, 0, st>>>(*src, *dst, m, ka);
   c->launches++;
   const uint64_t* sorted = radix_sort(ka, kb, 2 * m, 0, 32, sort_ws, sort_error(c), st, &c->launches);
   const UniqueFlag flag{sorted, 0xFFFFFFFFull};
-  const uint32_t grid = range_reduce_scan(flag, 2 * m, sums, st, &c->launches);
-  STC_CUDA(cudaMemcpyAsync(c->h_pinned + C_WORK, sums + grid, sizeof(uint64_t),
-                           cudaMemcpyDeviceToHost, st));
-  STC_CUDA(cudaStreamSynchronize(st));
-  const uint64_t nd = c->h_pinned[C_WORK];
+  const uint32_t grid = range_reduce_scan(flag, 2 * m, sums, st, &c->launches, sort_error(c));
+  const uint64_t nd = read_total(c, sums, grid);
   if (nd > kMaxVertices)
     fail(STC_ERR_LIMIT, std::to_string(nd) + " distinct vertex ids >= 2^31 - 1");
   uint32_t* ids = buffer<uint32_t>(c, B_DISTINCT, nd);
@@ -1178,7 +1190,7 @@ void build_graph(stc_ctx* c, const uint32_t* d_src, const uint32_t* d_dst, const
     return;
   }
   const SortSpace sort_ws = sort_space(c, std::max<uint64_t>(m, g.n));
-  uint64_t* sums = buffer<uint64_t>(c, B_SCAN_SUMS, kMaxSortGrid + 1);
+  uint64_t* sums = buffer<uint64_t>(c, B_SCAN_SUMS, kScanSums);
 
   // 2. dedup.
   uint64_t* ka = buffer<uint64_t>(c, B_KEYS_A, m);
@@ -1190,13 +1202,11 @@ void build_graph(stc_ctx* c, const uint32_t* d_src, const uint32_t* d_dst, const
     c->launches++;
     uint64_t* sorted = radix_sort(ka, kb, m, 0, 2 * (int)g.bits, sort_ws, sort_error(c), st, &c->launches);
     const uint64_t mask = (1ull << (2 * g.bits)) - 1;
-    range_scan(UniqueFlag{sorted, mask}, UniqueEmit{sorted, g.ukeys}, g.m_valid, sums, st,
-               &c->launches);
-    const uint32_t grid = range_partition(g.m_valid, kScanTile, kMaxSortGrid).grid;
-    STC_CUDA(cudaMemcpyAsync(c->h_pinned + C_WORK, sums + grid, sizeof(uint64_t),
-                             cudaMemcpyDeviceToHost, st));
-    STC_CUDA(cudaStreamSynchronize(st));
-    g.m_unique = c->h_pinned[C_WORK];
+    const UniqueFlag flag{sorted, mask};
+    const uint32_t grid =
+        range_reduce_scan(flag, g.m_valid, sums, st, &c->launches, sort_error(c));
+    range_apply(flag, UniqueEmit{sorted, g.ukeys}, g.m_valid, sums, st, &c->launches);
+    g.m_unique = read_total(c, sums, grid);
   }
   STC_CUDA(cudaGetLastError());
   mark(c, 2);
@@ -1221,7 +1231,7 @@ void build_graph(stc_ctx* c, const uint32_t* d_src, const uint32_t* d_dst, const
     g.max_deg = (uint32_t)c->h_pinned[C_MAX_DEG];
     uint64_t* vs = radix_sort(va, vb, g.n, 32, 32 + (int)bit_width64(g.max_deg), sort_ws, sort_error(c), st,
                               &c->launches);
-    k_rank<<<grid_for(g.n, 4), kThreads, 0, st>>>(vs, g.n, g.verts, g.rank);
+    k_rank<<<grid_for(g.n, 4), kThreads, 0, st>>>(vs, g.n, g.verts, g.rank, sort_error(c));
     c->launches++;
   }
   STC_CUDA(cudaGetLastError());
@@ -1231,7 +1241,7 @@ void build_graph(stc_ctx* c, const uint32_t* d_src, const uint32_t* d_dst, const
   g.m_fwd = g.m_unique;
   if (g.m_fwd) {
     k_arc_keys<<<grid_for(g.m_fwd, 4), kThreads, 0, st>>>(g.ukeys, g.m_fwd, g.bits, g.rank, ka,
-                                                          g.fdeg);
+                                                          g.fdeg, sort_error(c));
     c->launches++;
     finish_csr_from_arc_keys(c, g, ka, kb);
   } else {
@@ -1327,7 +1337,7 @@ void build_graph_batch(stc_ctx* c, const uint32_t* d_src, const uint32_t* d_dst,
     return;
   }
   const SortSpace sort_ws = sort_space(c, std::max<uint64_t>(m, g.n));
-  uint64_t* sums = buffer<uint64_t>(c, B_SCAN_SUMS, kMaxSortGrid + 1);
+  uint64_t* sums = buffer<uint64_t>(c, B_SCAN_SUMS, kScanSums);
 
   // 2. dedup over the union.
   uint64_t* ka = buffer<uint64_t>(c, B_KEYS_A, m);
@@ -1339,13 +1349,11 @@ void build_graph_batch(stc_ctx* c, const uint32_t* d_src, const uint32_t* d_dst,
     c->launches++;
     uint64_t* sorted = radix_sort(ka, kb, m, 0, 2 * (int)g.bits, sort_ws, sort_error(c), st, &c->launches);
     const uint64_t mask = (1ull << (2 * g.bits)) - 1;
-    range_scan(UniqueFlag{sorted, mask}, UniqueEmit{sorted, g.ukeys}, g.m_valid, sums, st,
-               &c->launches);
-    const uint32_t grid = range_partition(g.m_valid, kScanTile, kMaxSortGrid).grid;
-    STC_CUDA(cudaMemcpyAsync(c->h_pinned + C_WORK, sums + grid, sizeof(uint64_t),
-                             cudaMemcpyDeviceToHost, st));
-    STC_CUDA(cudaStreamSynchronize(st));
-    g.m_unique = c->h_pinned[C_WORK];
+    const UniqueFlag flag{sorted, mask};
+    const uint32_t grid =
+        range_reduce_scan(flag, g.m_valid, sums, st, &c->launches, sort_error(c));
+    range_apply(flag, UniqueEmit{sorted, g.ukeys}, g.m_valid, sums, st, &c->launches);
+    g.m_unique = read_total(c, sums, grid);
   }
   STC_CUDA(cudaGetLastError());
   mark(c, 2);
@@ -1377,7 +1385,7 @@ void build_graph_batch(stc_ctx* c, const uint32_t* d_src, const uint32_t* d_dst,
       c->launches++;
     }
     uint64_t* vs = radix_sort(va, vb, g.n, 32, 32 + dbits + gbits, sort_ws, sort_error(c), st, &c->launches);
-    k_rank<<<grid_for(g.n, 4), kThreads, 0, st>>>(vs, g.n, g.verts, g.rank);
+    k_rank<<<grid_for(g.n, 4), kThreads, 0, st>>>(vs, g.n, g.verts, g.rank, sort_error(c));
     c->launches++;
   }
   STC_CUDA(cudaGetLastError());
@@ -1387,7 +1395,7 @@ void build_graph_batch(stc_ctx* c, const uint32_t* d_src, const uint32_t* d_dst,
   g.m_fwd = g.m_unique;
   if (g.m_fwd) {
     k_arc_keys<<<grid_for(g.m_fwd, 4), kThreads, 0, st>>>(g.ukeys, g.m_fwd, g.bits, g.rank, ka,
-                                                          g.fdeg);
+                                                          g.fdeg, sort_error(c));
     c->launches++;
     finish_csr_from_arc_keys(c, g, ka, kb);
   } else {
@@ -1444,7 +1452,7 @@ void export_forward_csr(stc_ctx* c, const DeviceGraph& g, stc_forward_csr* out) 
   uint64_t* ka = buffer<uint64_t>(c, B_KEYS_A, mu);
   uint64_t* kb = buffer<uint64_t>(c, B_KEYS_B, mu);
   const SortSpace sort_ws = sort_space(c, mu);
-  uint64_t* sums = buffer<uint64_t>(c, B_SCAN_SUMS, kMaxSortGrid + 1);
+  uint64_t* sums = buffer<uint64_t>(c, B_SCAN_SUMS, kScanSums);
   uint32_t* edges = buffer<uint32_t>(c, B_NBR, mu);
   int8_t* signs = buffer<int8_t>(c, B_SGN, mu);
   if (n) STC_CUDA(cudaMemsetAsync(fdeg_id, 0, (size_t)n * sizeof(uint32_t), st));

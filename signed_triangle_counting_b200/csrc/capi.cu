@@ -663,7 +663,12 @@ stc_status stc_build_forward_csr(stc_ctx* c, const uint32_t* src, const uint32_t
     build_graph(c, in.src, in.dst, in.sign, m, g);
     export_forward_csr(c, g, out);
     mark(c, 5);
-    end_call(c, g, nullptr);
+    try {
+      end_call(c, g, nullptr);
+    } catch (...) {
+      stc_free_forward_csr(out);  // what a failed call leaves there means nothing
+      throw;
+    }
   });
 }
 

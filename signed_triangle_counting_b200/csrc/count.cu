@@ -933,6 +933,7 @@ __global__ void k_classify_count(const uint64_t* __restrict__ off, uint32_t n, C
                                  unsigned long long* __restrict__ ctr,
                                  const unsigned long long* __restrict__ range,
                                  const uint8_t* __restrict__ need = nullptr) {
+  if (device_failed(ctr + C_ERROR)) return;  // no vertex in any class
   uint32_t cnt[kClasses] = {0, 0, 0, 0, 0};
   uint32_t dmax = 0;
   uint32_t u0, u1;
@@ -954,12 +955,14 @@ __global__ void k_classify_count(const uint64_t* __restrict__ off, uint32_t n, C
 }
 
 // Appends each vertex to its class list (order within a class is free: the
-// counts are sums of integers).
+// counts are sums of integers); the cursors are ctr[C_WORK + class].
 __global__ void k_classify_fill(const uint64_t* __restrict__ off, uint32_t n, ClassBounds cb,
                                 uint32_t* __restrict__ lists, const uint32_t* __restrict__ starts,
-                                unsigned long long* __restrict__ cursor,
+                                unsigned long long* __restrict__ ctr,
                                 const unsigned long long* __restrict__ range,
                                 const uint8_t* __restrict__ need = nullptr) {
+  if (device_failed(ctr + C_ERROR)) return;
+  unsigned long long* cursor = ctr + C_WORK;
   uint32_t u0, u1;
   source_range(range, n, u0, u1);
   for (uint32_t base = u0 + blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < u1;
@@ -1593,6 +1596,7 @@ __global__ void __launch_bounds__(256) k_head_keys(Csr g, const uint32_t* __rest
   __shared__ uint8_t tab[kTableBytes];
   __shared__ uint32_t wcnt[2][kWarps];  // alternating tiles
   __shared__ uint32_t tbase[2];
+  if (device_failed(ctr + C_ERROR)) return;  // no keys, so no head-side work
   if (m_dev) m = min(m, (uint64_t)*m_dev);  // m a capacity, *m_dev the arc count
   for (uint32_t i = threadIdx.x; i < kTableBytes; i += blockDim.x) tab[i] = gtables[i];
   __syncthreads();
@@ -1720,6 +1724,7 @@ __global__ void __launch_bounds__(256) k_head_items(const uint64_t* __restrict__
   constexpr int kPer = kItemTile / 256;
   __shared__ uint32_t found[kItemTile];  // first entries, by class: cnt[c] from start[c]
   __shared__ uint32_t cnt[kHeadClasses], start[kHeadClasses], gbase[kHeadClasses];
+  if (device_failed(ctr + C_ERROR)) return;  // no items
   const uint64_t m = ctr[C_HEAD_NKEYS];
   for (uint64_t tile = (uint64_t)blockIdx.x * kItemTile; tile < m;
        tile += (uint64_t)gridDim.x * kItemTile) {
@@ -2494,8 +2499,7 @@ void enqueue_persistent(cudaStream_t st, const Csr& csr, const ClassBounds& cb, 
   STC_CUDA(cudaMemsetAsync(ctr + C_WORK, 0, 8 * sizeof(uint64_t), st));
   k_classify_count<<<kSMs * 4, 256, 0, st>>>(csr.off, csr.n, cb, ctr, nullptr, need);
   k_plan<<<1, 32, 0, st>>>(ctr, plan);
-  k_classify_fill<<<kSMs * 4, 256, 0, st>>>(csr.off, csr.n, cb, lists, plan, ctr + C_WORK, nullptr,
-                                            need);
+  k_classify_fill<<<kSMs * 4, 256, 0, st>>>(csr.off, csr.n, cb, lists, plan, ctr, nullptr, need);
   k_persistent<Sink><<<kSMs * 4, 256, kPersistentSmem, st>>>(csr, lists, plan, ctr, sink,
                                                              d_tables);
   k_block<512, Sink, false, kStreamUnroll, false>
@@ -2602,7 +2606,9 @@ constexpr uint32_t kSplitShort = 32;
 
 __global__ void k_split_csr(const uint64_t* __restrict__ off, const uint32_t* __restrict__ nbr,
                             const int8_t* __restrict__ sgn, uint32_t n,
-                            uint32_t* __restrict__ out, uint32_t* __restrict__ psplit) {
+                            uint32_t* __restrict__ out, uint32_t* __restrict__ psplit,
+                            const unsigned long long* __restrict__ err) {
+  if (device_failed(err)) return;
   const uint32_t lane = lane_id();
   const uint32_t lt = lanemask_lt();
   const uint32_t stride = gridDim.x * blockDim.x;
@@ -2658,7 +2664,9 @@ __global__ void k_split_csr(const uint64_t* __restrict__ off, const uint32_t* __
 struct VertexCost {
   const uint64_t* off;
   const uint32_t* nbr;
+  const unsigned long long* err;
   __device__ uint32_t operator()(uint64_t u) const {
+    if (device_failed(err)) return 1u;
     const uint64_t b = off[u], e = off[u + 1], du = e - b;
     uint64_t cost = 1;
     for (uint64_t i = b; i < e; i++) {
@@ -2696,8 +2704,9 @@ __global__ void k_shard_bounds(const uint64_t* __restrict__ pre, uint32_t n, uin
 // Writes the rank range of cfg.shard into the counters (device side only).
 void shard_range(stc_ctx* c, const DeviceGraph& g, uint32_t shard, uint32_t shards) {
   uint64_t* pre = buffer<uint64_t>(c, B_SHARD_COST, (size_t)g.n + 1);
-  uint64_t* sums = buffer<uint64_t>(c, B_SCAN_SUMS, kMaxSortGrid + 1);
-  range_scan(VertexCost{g.off, g.nbr}, EmitPrefix{pre}, g.n, sums, c->stream, &c->launches);
+  uint64_t* sums = buffer<uint64_t>(c, B_SCAN_SUMS, kScanSums);
+  const unsigned long long* err = (unsigned long long*)counters(c) + C_ERROR;
+  range_scan(VertexCost{g.off, g.nbr, err}, EmitPrefix{pre}, g.n, sums, c->stream, &c->launches);
   STC_CUDA(cudaMemcpyAsync(pre + g.n, sums + range_partition(g.n, kScanTile, kMaxSortGrid).grid,
                            sizeof(uint64_t), cudaMemcpyDeviceToDevice, c->stream));
   k_shard_bounds<<<1, 32, 0, c->stream>>>(pre, g.n, shard, shards, (unsigned long long*)counters(c));
@@ -2781,7 +2790,8 @@ void build_split(stc_ctx* c, DeviceGraph& g) {
   g.nbr_split = buffer<uint32_t>(c, B_SPLIT_NBR, g.m_fwd + 4);
   g.psplit = buffer<uint32_t>(c, B_SPLIT_POS, g.n);
   STC_CUDA(cudaMemsetAsync(g.nbr_split + g.m_fwd, 0, 4 * sizeof(uint32_t), c->stream));
-  k_split_csr<<<kSMs * 8, 256, 0, c->stream>>>(g.off, g.nbr, g.sgn, g.n, g.nbr_split, g.psplit);
+  k_split_csr<<<kSMs * 8, 256, 0, c->stream>>>(g.off, g.nbr, g.sgn, g.n, g.nbr_split, g.psplit,
+                                               (unsigned long long*)counters(c) + C_ERROR);
   c->launches++;
   STC_CUDA(cudaGetLastError());
 }
@@ -2886,8 +2896,7 @@ void count_triangles(stc_ctx* c, const DeviceGraph& gin, const CountConfig& cfg)
   STC_CUDA(cudaMemcpyAsync(d_starts, starts, kClasses * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
   // Cursors of the fill, then the dynamic queues, live in C_WORK ...
   STC_CUDA(cudaMemsetAsync(counters(c) + C_WORK, 0, 8 * sizeof(uint64_t), st));
-  k_classify_fill<<<kSMs * 4, 256, 0, st>>>(g.off, g.n, cb, lists, d_starts, ctr + C_WORK, range,
-                                            need);
+  k_classify_fill<<<kSMs * 4, 256, 0, st>>>(g.off, g.n, cb, lists, d_starts, ctr, range, need);
   STC_CUDA(cudaMemsetAsync(counters(c) + C_WORK, 0, 8 * sizeof(uint64_t), st));
   c->launches += 2;
 
@@ -3093,8 +3102,7 @@ extern "C" stc_status stc_count_oriented_csr_noalloc(const uint64_t* d_offsets,
   uint32_t* d_starts = lists + starts[kClasses];
   STC_NA(cudaMemcpyAsync(d_starts, starts, kClasses * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
   STC_NA(cudaMemsetAsync(ctr + C_WORK, 0, 8 * sizeof(uint64_t), st));
-  k_classify_fill<<<kSMs * 4, 256, 0, st>>>(d_offsets, n, cb, lists, d_starts, ctr + C_WORK,
-                                            nullptr);
+  k_classify_fill<<<kSMs * 4, 256, 0, st>>>(d_offsets, n, cb, lists, d_starts, ctr, nullptr);
   STC_NA(cudaMemsetAsync(ctr + C_WORK, 0, 8 * sizeof(uint64_t), st));
 
   const Csr csr{d_offsets, d_heads, d_signs, nullptr, n, nullptr, nullptr};

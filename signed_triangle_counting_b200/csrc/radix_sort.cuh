@@ -13,7 +13,9 @@
 //              looking back over their published states, and writes each
 //              digit's keys in a row (reads 8 B/key, writes 8 B/key).
 // A CTA waits only for tiles taken before its own, whose CTAs are already
-// running; the wait is bounded all the same.
+// running; the wait is bounded all the same.  A wait that expires ends the
+// sort and leaves the output undefined: the kernels after it see the error
+// word (device_failed) and touch nothing, or the host reads it first.
 // Bits of the key outside [lo, hi) ride along untouched, which is how the
 // edge sign travels in bit 63 without a separate payload array.
 #pragma once
@@ -270,7 +272,7 @@ static __global__ void __launch_bounds__(kSortThreads, 4) k_radix_pass(
   if (m_dev && *m_dev < m) m = *m_dev;
   if (tid == 0) {
     sm.tile = atomicAdd(ws + kSortTickets + pass, 1u);
-    sm.abort = 0;
+    sm.abort = ((volatile uint32_t*)ws)[kSortAbort];
   }
 #pragma unroll
   for (int w = 0; w < kSortWarps; w++) {
@@ -281,7 +283,8 @@ static __global__ void __launch_bounds__(kSortThreads, 4) k_radix_pass(
   __syncthreads();
   const uint32_t tile = sm.tile;
   const uint64_t begin = (uint64_t)tile * kTile;
-  if (begin >= m) return;
+  // After an expired wait the keys no longer match the digit counts.
+  if (begin >= m || sm.abort) return;
   const uint32_t valid = m - begin < kTile ? (uint32_t)(m - begin) : kTile;
   next_state[(size_t)tile * kRadix + tid] = 0;
   const uint32_t wbase = warp * (32 * ITEMS) + lane;
@@ -329,11 +332,8 @@ static __global__ void __launch_bounds__(kSortThreads, 4) k_radix_pass(
   const W before = look_back(own, tile, cnt, ws, sm.abort);
   sm.gofs[tid] = ws[pass * kRadix + tid] + (uint32_t)before - st;
   __syncthreads();
-  if (sm.abort) {  // a wait expired: keep every index in range, and report it
-#pragma unroll
-    for (int j = 0; j < ITEMS; j++)
-      if (wbase + 32 * j < valid) out[begin + wbase + 32 * j] = k[j];
-    if (tid == 0) atomicExch(err, 2ull);
+  if (sm.abort) {  // a wait expired
+    if (tid == 0) atomicExch(err, (unsigned long long)kDeviceErrTimeout);
     return;
   }
   // Position i of the tile goes to gofs[digit] + i (modulo 2^32; below m).
@@ -361,8 +361,9 @@ inline void launch_radix_pass(const uint64_t* in, uint64_t* out, uint64_t m, int
 
 // Sorts keys[0, m) by bits [lo, hi) stably; returns the buffer that holds the
 // result (`keys` or `alt`).  m must be below 2^32.  `space` is checked to hold
-// sort_words(m) words before anything is launched; `err` receives 2 if a
-// device-side wait expired.  With `m_dev`, the sort covers only the first min(m, *m_dev) keys,
+// sort_words(m) words before anything is launched; `err` receives
+// kDeviceErrTimeout if a device-side wait expired, and the result then is
+// not even a permutation of the keys.  With `m_dev`, the sort covers only the first min(m, *m_dev) keys,
 // a count known on the device alone (the launches are sized for m, so the
 // sequence can be captured).
 inline uint64_t* radix_sort(uint64_t* keys, uint64_t* alt, uint64_t m, int lo, int hi,
@@ -426,8 +427,11 @@ __global__ void __launch_bounds__(kScanThreads) k_range_reduce(F f, uint64_t n, 
   }
 }
 
-// Exclusive scan of a[0, n) in place; a[n] receives the total.
-static __global__ void __launch_bounds__(1024) k_scan_small(uint64_t* __restrict__ a, uint32_t n) {
+// Exclusive scan of a[0, n) in place; a[n] receives the total, or with `err`
+// (a scan over what a sort left) 0 once the error word is set, and a[n + 1]
+// the error word.
+static __global__ void __launch_bounds__(1024) k_scan_small(
+    uint64_t* __restrict__ a, uint32_t n, const unsigned long long* __restrict__ err) {
   __shared__ uint64_t tmp[33];
   const uint32_t per = (n + 1023) / 1024;
   const uint32_t b = threadIdx.x * per, e = b + per < n ? b + per : n;
@@ -440,7 +444,11 @@ static __global__ void __launch_bounds__(1024) k_scan_small(uint64_t* __restrict
     a[i] = run;
     run += x;
   }
-  if (threadIdx.x == 0) a[n] = total;
+  if (threadIdx.x == 0) {
+    const uint64_t word = err ? *err : 0;
+    a[n] = word ? 0 : total;
+    a[n + 1] = word;
+  }
 }
 
 // Index into a tile buffer with one padding word per 32: the blocked reads
@@ -496,15 +504,17 @@ __global__ void __launch_bounds__(kScanThreads) k_range_apply(F f, E emit, uint6
 }
 
 // The first two launches of a range scan: per-CTA totals, then their
-// exclusive scan in place; the grand total lands in sums[grid], and the
-// returned grid is what range_apply needs.  `sums` needs kMaxSortGrid + 1
-// words.
+// exclusive scan in place; the grand total and the error word (k_scan_small)
+// land in sums[grid] and sums[grid + 1], and the returned grid is what
+// range_apply needs.  `sums` needs kScanSums words.
+constexpr uint32_t kScanSums = kMaxSortGrid + 2;
 template <class F>
 inline uint32_t range_reduce_scan(F f, uint64_t n, uint64_t* sums, cudaStream_t st,
-                                  int* launches = nullptr) {
+                                  int* launches = nullptr,
+                                  const unsigned long long* err = nullptr) {
   RangePartition p = range_partition(n, kScanTile, kMaxSortGrid);
   k_range_reduce<<<p.grid, kScanThreads, 0, st>>>(f, n, p.per_cta, sums);
-  k_scan_small<<<1, 1024, 0, st>>>(sums, p.grid);
+  k_scan_small<<<1, 1024, 0, st>>>(sums, p.grid, err);
   if (launches) *launches += 2;
   return p.grid;
 }

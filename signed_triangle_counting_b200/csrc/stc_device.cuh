@@ -69,6 +69,12 @@ __device__ __forceinline__ unsigned match_label(uint32_t label) {
   return peers;
 }
 
+// True once an earlier kernel of the call set the error word (an expired wait
+// of a sort, a malformed CSR): what it left must not be used as an index.
+__device__ __forceinline__ bool device_failed(const unsigned long long* __restrict__ err) {
+  return *err != 0;
+}
+
 __host__ __device__ __forceinline__ uint32_t bit_width64(uint64_t x) {
   uint32_t b = 0;
   while (b < 64 && (x >> b) != 0) b++;

@@ -149,7 +149,7 @@ uint64_t parse_text_device(stc_ctx* c, const char* d_text, uint64_t size, uint32
     *sign = buffer<int8_t>(c, B_IN_SIGN, 1);
     return 0;
   }
-  uint64_t* sums = buffer<uint64_t>(c, B_SCAN_SUMS, kMaxSortGrid + 1);
+  uint64_t* sums = buffer<uint64_t>(c, B_SCAN_SUMS, kScanSums);
   unsigned long long* ctr = (unsigned long long*)counters(c);
   const uint64_t chunks = (size + 15) / 16;
   const NewlineCount nl{(const uint4*)d_text};

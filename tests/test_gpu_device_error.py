@@ -58,3 +58,22 @@ def test_every_entry_reports_it(m):
     with stc.Context(0) as c:
         for persistent in (True, True, True, False):
             assert [x.as_tuple() for x in c.count_batch(batch, persistent=persistent)] == each
+
+
+def test_nothing_is_counted_after_it():
+    g = graph(700_000, 7)
+    src, dst, sign = (np.ascontiguousarray(x) for x in g)
+    n = int(max(src.max(), dst.max())) + 1
+    with stc.Context(0) as c:
+        for persistent in (False, True):
+            assert c.vertex_counts(*g, persistent=persistent).sum() > 0
+            buf = np.full(4 * n, 7, np.uint64)
+            n_out, o = C.c_uint32(), c._opts(persistent=persistent)
+            preset(c, 2)
+            rc = _capi.lib().stc_vertex_counts(
+                c._h, src.ctypes.data_as(_capi.u32p), dst.ctypes.data_as(_capi.u32p),
+                sign.ctypes.data_as(_capi.i8p), len(src), C.byref(o),
+                buf.ctypes.data_as(_capi.u64p), len(buf), C.byref(n_out))
+            preset(c, 0)
+            assert rc == _capi.STC_ERR_DEVICE_TIMEOUT
+            assert not buf.any() or (buf == 7).all()
