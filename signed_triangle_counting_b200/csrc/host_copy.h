@@ -2,11 +2,14 @@
 // small ring of pinned slots that worker threads fill (or drain) while earlier
 // slots cross the bus.
 //
-// A pageable cudaMemcpyAsync stages with one host thread (15 GB/s up; down
-// into fresh pages 5 GB/s, most of it page faults) and costs about 10 us
-// however small it is.  Eight threads fill slots at 58 GB/s, as fast as the
-// bus takes them, and scattered pieces that lie back to back on the device
-// (the graphs of a batch) cross as one copy per slot.
+// A pageable cudaMemcpyAsync stages with one host thread (18 GB/s up; down
+// into fresh pages 5 GB/s, most of it page faults) and costs 5 to 10 us
+// however small it is.  Eight threads keep the bus busy (256 MB up in 6.0 ms
+// against 24.6), and scattered pieces that lie back to back on the device (the
+// graphs of a batch) cross as one copy per slot.  But a thread that was asleep
+// copies its first megabytes at a fifth of the caller's rate, so small copies
+// gain nothing from it, parts are small, and nobody waits for a thread that
+// has not joined (upload, begin_call).
 //
 // The ring and the threads belong to one context, are made on the first use
 // that is worth them, and go with it (or with stc_ctx_trim).
@@ -16,6 +19,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <chrono>
 #include <condition_variable>
 #include <cstdlib>
 #include <cstring>
@@ -63,9 +67,30 @@ class HostCopier {
 
   // Host pieces to the device, in stream order; the host memory may be reused
   // on return.  Pieces that follow each other on the device share copies.
-  void upload(const std::vector<Piece>& pieces, cudaStream_t st) { run(pieces, st, true); }
-  // Device to host pieces; done on return.
-  void download(const std::vector<Piece>& pieces, cudaStream_t st) { run(pieces, st, false); }
+  void upload(const std::vector<Piece>& pieces, cudaStream_t st) {
+    const size_t total = bytes_of(pieces);
+    // On a host of 16 virtual CPUs, three pieces of 3 / 8 / 12 / 32 / 256 MB in
+    // all took 189 / 420 / 646 / 1,750 / 24,600 us as plain copies, 228 / 561 /
+    // 846 / 2,370 / 27,000 through the ring by the caller alone, 247 / 410 /
+    // 512 / 1,070 / 9,220 with three helpers and 254 / 553 / 738 / 1,180 /
+    // 6,010 with seven (64 MB: 2,140 with three, 1,850 with seven).  2 MB in
+    // pieces of 8 / 16 / 32 / 64 / 128 KB took 540 / 320 / 207 / 185 / 147 as
+    // plain copies and 215 / 184 / 175 / 170 / 170 through the ring.
+    if (total < kUploadRing && total >= pieces.size() * kUploadPiece) {
+      for (const Piece& p : pieces)
+        cuda_check(cudaMemcpyAsync(p.device, p.host, p.bytes, cudaMemcpyHostToDevice, st),
+                   "cudaMemcpyAsync(pageable)");
+      return;
+    }
+    run(pieces, st, true, total < kUploadRing ? 0u : total < kUploadAll ? 3u : kHelpers);
+  }
+  // Device to host pieces; done on return.  Page faults are most of the work,
+  // so helpers pay from 2 MB on (with them 80 us, without 170, a plain copy
+  // 130; at 1 MB all three within 15 us; 32 MB 2.3 / 4.6 / 6.8 ms): they are
+  // awake by the time the kernels ahead of the copy are done.
+  void download(const std::vector<Piece>& pieces, cudaStream_t st) {
+    run(pieces, st, false, bytes_of(pieces) < kDownloadThreads ? 0u : kHelpers);
+  }
 
   void release() {
     if (!threads_.empty()) {
@@ -92,8 +117,17 @@ class HostCopier {
  private:
   static constexpr int kSlots = 8;
   static constexpr size_t kSlotBytes = 2u << 20;
-  static constexpr size_t kPart = 256u << 10;           // what a thread copies at a time
-  static constexpr size_t kThreadedBytes = 2u << 20;    // less is not worth waking threads for
+  // What a thread copies at a time; with 256 KB the call waited for the last
+  // part of a slow helper (8 MB up with seven: 1,000 us, with 32 KB 553).
+  static constexpr size_t kPart = 32u << 10;
+  static constexpr unsigned kHelpers = 7;
+  static constexpr size_t kUploadRing = 8u << 20;       // less goes up as plain copies,
+  static constexpr size_t kUploadPiece = 64u << 10;     // unless in pieces smaller than this
+  static constexpr size_t kUploadAll = 48u << 20;       // all helpers from here on
+  static constexpr size_t kDownloadThreads = 2u << 20;
+  // How long a helper waits for a part (a count may run before a download)
+  // before it sleeps again.
+  static constexpr std::chrono::milliseconds kIdle{2};
   // A part of one slot's contents, between `ring` and `host`.
   struct Part {
     char* ring;
@@ -109,10 +143,14 @@ class HostCopier {
     Chunk(const Chunk& o) : device(o.device), bytes(o.bytes), part0(o.part0), part1(o.part1) {}
   };
 
-  void run(const std::vector<Piece>& pieces, cudaStream_t st, bool up) {
+  static size_t bytes_of(const std::vector<Piece>& pieces) {
     size_t total = 0;
     for (const Piece& p : pieces) total += p.bytes;
-    if (total == 0) return;
+    return total;
+  }
+
+  void run(const std::vector<Piece>& pieces, cudaStream_t st, bool up, unsigned helpers) {
+    if (bytes_of(pieces) == 0) return;
     if (!ring_) {
       cuda_check(cudaMallocHost(reinterpret_cast<void**>(&ring_), kSlots * kSlotBytes),
                  "cudaMallocHost(staging ring)");
@@ -140,21 +178,16 @@ class HostCopier {
       }
     }
     for (Chunk& c : chunks) c.left.store(c.part1 - c.part0, std::memory_order_relaxed);
-    const bool threaded = total >= kThreadedBytes;
     chunks_ = &chunks;
     up_ = up;
     next_.store(0);
     open_.store(0);  // parts below it may be copied
     cancel_.store(false);
-    if (threaded) wake();
     struct Guard {  // whatever happens, no thread touches this call's memory after it
       HostCopier* c;
-      bool threaded;
-      ~Guard() {
-        c->cancel_.store(true);
-        if (threaded) c->settle();
-      }
-    } guard{this, threaded};
+      ~Guard() { c->end_call(); }
+    } guard{this};
+    if (helpers) begin_call(helpers);
     const uint32_t nc = (uint32_t)chunks.size();
     auto event_done = [&](uint32_t c) {  // the slot's last transfer
       cuda_check(cudaEventSynchronize(event_[c % kSlots]), "cudaEventSynchronize(staging)");
@@ -189,6 +222,7 @@ class HostCopier {
         }
         event_done(c);
         open_.store(chunks[c].part1, std::memory_order_release);
+        if (helpers) wake_again();
       }
       for (uint32_t c = 0; c < nc; c++) finish(c);
     }
@@ -207,40 +241,69 @@ class HostCopier {
     return true;
   }
 
-  void wake() {
+  // Lets up to `helpers` threads join the call and wakes the first; each wakes
+  // the next, so that the caller pays for one wake-up only.  They join under the mutex and end_call waits only for
+  // those that did: a thread that wakes late finds the call over, and delays
+  // nobody.
+  void begin_call(unsigned helpers) {
     if (threads_.empty()) {
       const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-      const unsigned n = std::min(7u, hw > 2 ? hw / 2 : 1u);  // the caller is one more
-      // They have seen the calls so far (the ring may have been released since).
-      for (unsigned i = 0; i < n; i++)
-        threads_.emplace_back([this, seen = generation_] { work(seen); });
+      const unsigned n = std::min(kHelpers, hw > 2 ? hw / 2 : 1u);  // the caller is one more
+      for (unsigned i = 0; i < n; i++) threads_.emplace_back([this] { work(); });
     }
     {
       std::lock_guard<std::mutex> l(mu_);
-      generation_++;
-      busy_ = (int)threads_.size();
+      seats_ = (int)std::min<size_t>(helpers, threads_.size());
+      wakes_ = 1;
     }
-    cv_.notify_all();
+    cv_.notify_one();
   }
-
-  void settle() {
-    std::unique_lock<std::mutex> l(mu_);
-    idle_.wait(l, [this] { return busy_ == 0; });
-  }
-
-  void work(uint64_t seen) {
-    while (true) {
-      {
-        std::unique_lock<std::mutex> l(mu_);
-        cv_.wait(l, [&] { return quit_ || generation_ != seen; });
-        if (quit_) return;
-        seen = generation_;
-      }
-      const uint32_t n = (uint32_t)parts_.size();
-      while (!cancel_.load(std::memory_order_relaxed) && next_.load(std::memory_order_relaxed) < n)
-        if (!copy_part()) std::this_thread::yield();
+  // Wakes a helper if all have left (kIdle without a part).
+  void wake_again() {
+    {
       std::lock_guard<std::mutex> l(mu_);
-      if (--busy_ == 0) idle_.notify_all();
+      if (joined_ > 0 || wakes_ > 0) return;
+      wakes_ = 1;
+    }
+    cv_.notify_one();
+  }
+
+  void end_call() {
+    cancel_.store(true);
+    std::unique_lock<std::mutex> l(mu_);
+    seats_ = wakes_ = 0;
+    idle_.wait(l, [this] { return joined_ == 0; });
+  }
+
+  void work() {
+    std::unique_lock<std::mutex> l(mu_);
+    while (true) {
+      cv_.wait(l, [this] { return quit_ || (wakes_ > 0 && seats_ > 0); });
+      if (quit_) return;
+      wakes_--;
+      seats_--;
+      joined_++;
+      const bool more = seats_ > 0 && wakes_ == 0;
+      if (more) wakes_ = 1;
+      l.unlock();
+      if (more) cv_.notify_one();
+      const uint32_t n = (uint32_t)parts_.size();
+      auto since = std::chrono::steady_clock::now();
+      bool idle = false;  // since then
+      while (!cancel_.load(std::memory_order_relaxed) && next_.load(std::memory_order_relaxed) < n) {
+        if (copy_part()) {
+          idle = false;
+          continue;
+        }
+        const auto t = std::chrono::steady_clock::now();
+        if (!idle) since = t;
+        idle = true;
+        if (t - since > kIdle) break;
+        std::this_thread::yield();
+      }
+      l.lock();
+      seats_ += cancel_.load(std::memory_order_relaxed) ? 0 : 1;
+      if (--joined_ == 0) idle_.notify_one();
     }
   }
 
@@ -255,8 +318,9 @@ class HostCopier {
   std::vector<std::thread> threads_;
   std::mutex mu_;
   std::condition_variable cv_, idle_;
-  uint64_t generation_ = 0;
-  int busy_ = 0;
+  int seats_ = 0;   // threads that may still join the call
+  int wakes_ = 0;   // wake-ups on their way to one
+  int joined_ = 0;  // threads that touch the call's memory
   bool quit_ = false;
 };
 
