@@ -12,7 +12,8 @@
 // has not joined (upload, begin_call).
 //
 // The ring and the threads belong to one context, are made on the first use
-// that is worth them, and go with it (or with stc_ctx_trim).
+// that is worth them, and go with it (or with stc_ctx_trim).  Where they cannot
+// be had (no more pinned memory, a limit on threads) the copies go on without.
 #pragma once
 #include <cuda_runtime.h>
 #include <sys/mman.h>
@@ -24,6 +25,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -76,13 +78,8 @@ class HostCopier {
     // 6,010 with seven (64 MB: 2,140 with three, 1,850 with seven).  2 MB in
     // pieces of 8 / 16 / 32 / 64 / 128 KB took 540 / 320 / 207 / 185 / 147 as
     // plain copies and 215 / 184 / 175 / 170 / 170 through the ring.
-    if (total < kUploadRing && total >= pieces.size() * kUploadPiece) {
-      for (const Piece& p : pieces)
-        cuda_check(cudaMemcpyAsync(p.device, p.host, p.bytes, cudaMemcpyHostToDevice, st),
-                   "cudaMemcpyAsync(pageable)");
-      return;
-    }
-    run(pieces, st, true, total < kUploadRing ? 0u : total < kUploadAll ? 3u : kHelpers);
+    if (total < kUploadRing && total >= pieces.size() * kUploadPiece) plain(pieces, st, true);
+    else run(pieces, st, true, total < kUploadRing ? 0u : total < kUploadAll ? 3u : kHelpers);
   }
   // Device to host pieces; done on return.  Page faults are most of the work,
   // so helpers pay from 2 MB on (with them 80 us, without 170, a plain copy
@@ -103,15 +100,7 @@ class HostCopier {
       threads_.clear();
       quit_ = false;
     }
-    for (int i = 0; i < kSlots; i++) {
-      if (event_[i]) {
-        (void)cudaEventSynchronize(event_[i]);
-        (void)cudaEventDestroy(event_[i]);
-        event_[i] = nullptr;
-      }
-    }
-    if (ring_) (void)cudaFreeHost(ring_);
-    ring_ = nullptr;
+    free_ring();
   }
 
  private:
@@ -149,14 +138,45 @@ class HostCopier {
     return total;
   }
 
+  // The driver's own copies.
+  static void plain(const std::vector<Piece>& pieces, cudaStream_t st, bool up) {
+    for (const Piece& p : pieces)
+      cuda_check(up ? cudaMemcpyAsync(p.device, p.host, p.bytes, cudaMemcpyHostToDevice, st)
+                    : cudaMemcpyAsync(p.host, p.device, p.bytes, cudaMemcpyDeviceToHost, st),
+                 "cudaMemcpyAsync(pageable)");
+    if (!up) cuda_check(cudaStreamSynchronize(st), "cudaStreamSynchronize");
+  }
+
+  // The ring and its events, or neither.
+  bool make_ring() {
+    if (ring_) return true;
+    bool ok = cudaMallocHost(reinterpret_cast<void**>(&ring_), kSlots * kSlotBytes) == cudaSuccess;
+    if (!ok) ring_ = nullptr;
+    for (auto& e : event_)
+      if (ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+        e = nullptr;
+        ok = false;
+      }
+    if (!ok) {
+      (void)cudaGetLastError();
+      free_ring();
+    }
+    return ok;
+  }
+  void free_ring() {
+    for (auto& e : event_) {
+      if (!e) continue;
+      (void)cudaEventSynchronize(e);
+      (void)cudaEventDestroy(e);
+      e = nullptr;
+    }
+    if (ring_) (void)cudaFreeHost(ring_);
+    ring_ = nullptr;
+  }
+
   void run(const std::vector<Piece>& pieces, cudaStream_t st, bool up, unsigned helpers) {
     if (bytes_of(pieces) == 0) return;
-    if (!ring_) {
-      cuda_check(cudaMallocHost(reinterpret_cast<void**>(&ring_), kSlots * kSlotBytes),
-                 "cudaMallocHost(staging ring)");
-      for (auto& e : event_)
-        cuda_check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate(staging)");
-    }
+    if (!make_ring()) return plain(pieces, st, up);
     // Cut the pieces into slots and parts.
     std::vector<Chunk> chunks;
     parts_.clear();
@@ -249,7 +269,10 @@ class HostCopier {
     if (threads_.empty()) {
       const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
       const unsigned n = std::min(kHelpers, hw > 2 ? hw / 2 : 1u);  // the caller is one more
-      for (unsigned i = 0; i < n; i++) threads_.emplace_back([this] { work(); });
+      try {
+        for (unsigned i = 0; i < n; i++) threads_.emplace_back([this] { work(); });
+      } catch (const std::system_error&) {  // with those there are, if any
+      }
     }
     {
       std::lock_guard<std::mutex> l(mu_);

@@ -1,6 +1,7 @@
 """HostCopier (csrc/host_copy.h) on the CPU, over a stand-in for the CUDA
 runtime whose copies are memcpy: contents of random scattered pieces both ways,
-and a call that does not wait for helper threads which wake late."""
+a call that does not wait for helper threads which wake late, and copies where
+no pinned memory, no event or no thread can be had."""
 import shutil
 import subprocess
 from pathlib import Path
@@ -69,6 +70,12 @@ extern "C" int pthread_cond_wait(pthread_cond_t* c, pthread_mutex_t* m) {
   }
   return r;
 }
+static bool fail_threads = false;
+extern "C" int pthread_create(pthread_t* t, const pthread_attr_t* a, void* (*f)(void*), void* x) {
+  using F = int (*)(pthread_t*, const pthread_attr_t*, void* (*)(void*), void*);
+  static F real = (F)dlsym(RTLD_NEXT, "pthread_create");
+  return fail_threads ? EAGAIN : real(t, a, f, x);
+}
 namespace stc {
 void cuda_check(cudaError_t e, const char* what) { if (e) throw std::string(what); }
 }
@@ -123,6 +130,18 @@ int main(int argc, char** argv) {
       usleep(600000);
     }
     late = false;
+  } else if (mode == "scarce") {
+    for (int what = 0; what < 3; what++) {
+      fail_pinned = what == 0;
+      fail_events = what == 1 ? 3 : -1;
+      fail_threads = what == 2;
+      for (int again = 0; again < 2; again++)
+        if (!round_trip(c, {24u << 20, 5000, 3u << 20}, false)) return printf("contents differ (%d)\n", what), 1;
+      fail_pinned = fail_threads = false;  // and once there is enough again
+      fail_events = -1;
+      if (!round_trip(c, {24u << 20, 5000, 3u << 20}, false)) return printf("contents differ (%d)\n", what), 1;
+      c.release();
+    }
   }
   puts("ok");
 }
@@ -141,7 +160,7 @@ def program(tmp_path_factory) -> Path:
     return d / "main"
 
 
-@pytest.mark.parametrize("mode", ["random", "late"])
+@pytest.mark.parametrize("mode", ["random", "late", "scarce"])
 def test_host_copier(program, mode):
     r = subprocess.run([str(program), mode], capture_output=True, text=True, timeout=120)
     assert (r.returncode, r.stdout) == (0, "ok\n"), r.stdout + r.stderr
