@@ -65,8 +65,12 @@ void upload(stc_ctx* c, const std::vector<HostCopier::Piece>& pieces) {
   std::vector<HostCopier::Piece> staged;
   for (const auto& p : pieces) {
     if (p.bytes == 0) continue;
-    if (is_pageable(p.host)) staged.push_back(p);
-    else STC_CUDA(cudaMemcpyAsync(p.device, p.host, p.bytes, cudaMemcpyHostToDevice, c->stream));
+    if (is_pageable(p.host)) {
+      staged.push_back(p);
+    } else {
+      c->host_in_flight = true;
+      STC_CUDA(cudaMemcpyAsync(p.device, p.host, p.bytes, cudaMemcpyHostToDevice, c->stream));
+    }
   }
   c->copier.upload(staged, c->stream);
 }
@@ -75,11 +79,16 @@ void download(stc_ctx* c, const std::vector<HostCopier::Piece>& pieces) {
   std::vector<HostCopier::Piece> staged;
   for (const auto& p : pieces) {
     if (p.bytes == 0) continue;
-    if (is_pageable(p.host)) staged.push_back(p);
-    else STC_CUDA(cudaMemcpyAsync(p.host, p.device, p.bytes, cudaMemcpyDeviceToHost, c->stream));
+    if (is_pageable(p.host)) {
+      staged.push_back(p);
+    } else {
+      c->host_in_flight = true;
+      STC_CUDA(cudaMemcpyAsync(p.host, p.device, p.bytes, cudaMemcpyDeviceToHost, c->stream));
+    }
   }
   c->copier.download(staged, c->stream);
   STC_CUDA(cudaStreamSynchronize(c->stream));
+  c->host_in_flight = false;
 }
 
 void release_pipelines(stc_ctx* c) {
@@ -90,9 +99,21 @@ void release_pipelines(stc_ctx* c) {
 
 namespace {
 
+// A call that fails returns only when no copy of the caller's memory is in
+// flight any more.
+void settle_copies(stc_ctx* c) {
+  if (!c) return;
+  if (c->host_in_flight) (void)cudaStreamSynchronize(c->stream);
+  if (c->sign_pending) (void)cudaStreamSynchronize(c->aux_stream);
+  if (c->host_in_flight || c->sign_pending) (void)cudaGetLastError();
+  c->host_in_flight = c->sign_pending = false;
+}
+
 // Runs `body` with the context's error handling; every ABI entry uses it.
 template <class F>
 stc_status guarded(stc_ctx* c, F body) {
+  stc_status status = STC_ERR_INTERNAL;
+  std::string msg;
   try {
     if (c) {
       c->last_error.clear();
@@ -101,20 +122,17 @@ stc_status guarded(stc_ctx* c, F body) {
     body();
     return STC_OK;
   } catch (const Error& e) {
-    if (c) c->last_error = e.msg;
-    if (c && c->sign_pending) {  // the caller's sign array stays in use until the copy ends
-      c->sign_pending = false;
-      cudaStreamSynchronize(c->aux_stream);
-      (void)cudaGetLastError();
-    }
-    return e.status;
+    status = e.status;
+    msg = e.msg;
   } catch (const std::bad_alloc&) {
-    if (c) c->last_error = "host allocation failed";
-    return STC_ERR_OUT_OF_MEMORY;
+    status = STC_ERR_OUT_OF_MEMORY;
+    msg = "host allocation failed";
   } catch (...) {
-    if (c) c->last_error = "unexpected internal error";
-    return STC_ERR_INTERNAL;
+    msg = "unexpected internal error";
   }
+  settle_copies(c);
+  if (c) c->last_error = msg;
+  return status;
 }
 
 void begin_call(stc_ctx* c, const stc_opts* o) {
@@ -137,6 +155,7 @@ void end_call(stc_ctx* c, const DeviceGraph& g, stc_counts* out) {
   STC_CUDA(cudaMemcpyAsync(c->h_pinned, counters(c), C_SLOTS * sizeof(uint64_t),
                            cudaMemcpyDeviceToHost, c->stream));
   STC_CUDA(cudaStreamSynchronize(c->stream));
+  c->host_in_flight = false;
   STC_CUDA(cudaGetLastError());
   check_device_error(c->h_pinned[C_ERROR]);
   if (out) {
@@ -790,6 +809,7 @@ stc_status stc_count_batch_packed(stc_ctx* c, const uint32_t* src, const uint32_
     }
     mark(c, 7);
     STC_CUDA(cudaStreamSynchronize(c->stream));
+    c->host_in_flight = false;
     total.kernel_launches = (uint32_t)c->launches;
     if (c->timing) total.ms_total = elapsed(c, 0, 7);
     c->stats = total;
@@ -1041,6 +1061,7 @@ stc_status stc_autotune(stc_ctx* c, const uint32_t* src, const uint32_t* dst, co
     c->tuning = best;
     *out = to_abi(best);
     STC_CUDA(cudaStreamSynchronize(c->stream));
+    c->host_in_flight = false;
   });
 }
 

@@ -164,6 +164,7 @@ struct stc_ctx {
   cudaStream_t aux_stream = nullptr;
   cudaEvent_t ev_ids = nullptr, ev_sign = nullptr;
   bool sign_pending = false;
+  bool host_in_flight = false;  // copies from or to the caller's own pinned memory may be under way
   bool timing = false;
   int launches = 0;
   bool fixed_ready = false;   // B_DISPATCH_FIXED holds the fixed tables
@@ -255,9 +256,9 @@ struct DeviceGraph {
   uint32_t* psplit = nullptr;
 };
 
-// Copies host arrays to the device (stream order; host memory reusable on
-// return) and back (done on return): pageable memory through the context's
-// staging, anything else by the driver.
+// Copies host arrays to the device (stream order) and back (done on return):
+// pageable memory, which may be reused on return, through the context's staging,
+// anything else by the driver, which reads it until the stream gets there.
 void upload(stc_ctx* c, const std::vector<HostCopier::Piece>& pieces);
 void download(stc_ctx* c, const std::vector<HostCopier::Piece>& pieces);
 template <class T>
