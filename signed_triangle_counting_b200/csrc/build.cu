@@ -532,8 +532,12 @@ __device__ __forceinline__ bool sampled_edge(uint32_t a, uint32_t b, uint32_t sh
 // Hub table: kHubSlots ids in buckets of two.
 constexpr uint32_t kHubSlots = 1024;
 constexpr uint32_t kNoHub = 0xFFFFFFFFu;
-// Lists of fewer edges have no hub worth the sample.
-constexpr uint64_t kHubMinEdges = 1u << 20;
+// Lists and batches of fewer edges have no hub worth the sample.  (Additions
+// to one address take 0.5 ns each: a shuffled star of 1,000,000 edges counts in
+// 388 us with the table and took 731 without, one of 4,000,000 in a batch 0.85
+// and 2.29 ms; without a hub 1,000,000 edges take 403 and 400 us, a batch of
+// eight lists of 500,000 709 and 699.)
+constexpr uint64_t kHubMinEdges = 1u << 19;
 __device__ __forceinline__ uint32_t hub_bucket(uint32_t x) {
   return ((x * 0x9E3779B1u) >> (32 - 9)) * 2;  // of kHubSlots / 2 buckets
 }
@@ -548,9 +552,8 @@ constexpr uint32_t kHubHits = 4;
 inline uint32_t hub_sample(uint64_t m) { return m < (1u << 24) ? 2048 : 8192; }
 inline size_t hub_smem(uint32_t sample) { return 4ull * sample * sizeof(uint32_t); }
 
-__global__ void __launch_bounds__(1024) k_find_hubs(const uint32_t* __restrict__ u,
-                                                    const uint32_t* __restrict__ v, uint64_t m,
-                                                    uint32_t sample, uint32_t* __restrict__ hubs) {
+__global__ void __launch_bounds__(1024) k_find_hubs(EdgeIds e, uint64_t m, uint32_t sample,
+                                                    uint32_t* __restrict__ hubs) {
   extern __shared__ uint32_t hub_seen[];
   const uint32_t slots = 2 * sample;  // load <= 1/2
   uint32_t* id = hub_seen;
@@ -564,7 +567,11 @@ __global__ void __launch_bounds__(1024) k_find_hubs(const uint32_t* __restrict__
   const uint64_t step = m / (sample / 2);
   for (uint32_t i = threadIdx.x; i < sample; i += 1024) {
     const uint64_t at = (i >> 1) * step;
-    const uint32_t x = (i & 1) ? v[at] : u[at];
+    EdgeCursor cur;
+    uint32_t x, other;
+    cur.start(e, at);
+    if (i & 1) cur.at(e, at, other, x);
+    else cur.at(e, at, x, other);
     if (x == kNoHub) continue;
     uint32_t s = (x * 0x9E3779B1u) & (slots - 1);
     while (true) {  // ends: more slots than endpoints
@@ -577,6 +584,18 @@ __global__ void __launch_bounds__(1024) k_find_hubs(const uint32_t* __restrict__
       if (atomicCAS(b, kNoHub, x) != kNoHub) atomicCAS(b + 1, kNoHub, x);
     }
   }
+}
+
+// The hub table of a list or batch (ids as EdgeIds gives them), or null.
+const uint32_t* find_hubs(stc_ctx* c, const EdgeIds& e, uint64_t m) {
+  if (m < kHubMinEdges) return nullptr;
+  const uint32_t sample = hub_sample(m);
+  uint32_t* hubs = buffer<uint32_t>(c, B_HUBS, kHubSlots);
+  STC_CUDA(cudaFuncSetAttribute(k_find_hubs, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)hub_smem(8192)));
+  k_find_hubs<<<1, 1024, hub_smem(sample), c->stream>>>(e, m, sample, hubs);
+  c->launches++;
+  return hubs;
 }
 
 // `hubs` (kHub only): k_find_hubs's table.  Ids at or past n only reach here
@@ -1159,17 +1178,13 @@ void build_graph(stc_ctx* c, const uint32_t* d_src, const uint32_t* d_dst, const
     k_scan_ids<<<grid_for(m, 4), kThreads, 0, st>>>(d_src, d_dst, m, ctr);
     c->launches++;
   }
-  const uint32_t* hubs = nullptr;
-  if (totals && m >= kHubMinEdges) {
-    const uint32_t sample = hub_sample(m);
-    uint32_t* h = buffer<uint32_t>(c, B_HUBS, kHubSlots);
-    STC_CUDA(cudaFuncSetAttribute(k_find_hubs, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)hub_smem(8192)));
-    k_find_hubs<<<1, 1024, hub_smem(sample), st>>>(d_src, d_dst, m, sample, h);
-    c->launches++;
-    hubs = h;
-  }
-  read_counters(c, C_MAX_ID, 2);
+  // The hubs are found while the host waits for the ids.
+  STC_CUDA(cudaMemcpyAsync(c->h_pinned + C_MAX_ID, counters(c) + C_MAX_ID, 2 * sizeof(uint64_t),
+                           cudaMemcpyDeviceToHost, st));
+  STC_CUDA(cudaEventRecord(c->ev_read, st));
+  const uint32_t* hubs =
+      totals ? find_hubs(c, EdgeIds{d_src, d_dst, nullptr, nullptr, 0}, m) : nullptr;
+  STC_CUDA(cudaEventSynchronize(c->ev_read));
   uint64_t max_id = c->h_pinned[C_MAX_ID];
   const uint64_t self = c->h_pinned[C_SELF];
   // Ranks stay below 2^31 - 2 where triangles are counted (kMaxVertices).
@@ -1333,7 +1348,8 @@ void build_graph_batch(stc_ctx* c, const uint32_t* d_src, const uint32_t* d_dst,
   g.bits = std::max<uint32_t>(1, bit_width64(ntot ? ntot - 1 : 0));
   g.gbase = d_vbase;
   if (totals) {
-    build_totals(c, EdgeIds{d_src, d_dst, d_eoff, d_vbase, G}, d_sign, m, g, d_vbase, G);
+    const EdgeIds e{d_src, d_dst, d_eoff, d_vbase, G};
+    build_totals(c, e, d_sign, m, g, d_vbase, G, find_hubs(c, e, m));
     return;
   }
   const SortSpace sort_ws = sort_space(c, std::max<uint64_t>(m, g.n));
@@ -1440,7 +1456,8 @@ void build_graph_batch_capped(stc_ctx* c, const uint32_t* d_src, const uint32_t*
   g.m_valid = m;
   g.bits = caps.bits;
   g.gbase = d_vbase;
-  build_totals(c, EdgeIds{d_src, d_dst, d_eoff, d_vbase, G}, d_sign, m, g, d_vbase, G, nullptr, &caps);
+  const EdgeIds e{d_src, d_dst, d_eoff, d_vbase, G};
+  build_totals(c, e, d_sign, m, g, d_vbase, G, find_hubs(c, e, m), &caps);
 }
 
 void export_forward_csr(stc_ctx* c, const DeviceGraph& g, stc_forward_csr* out) {

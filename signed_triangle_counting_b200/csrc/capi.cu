@@ -493,6 +493,7 @@ stc_status stc_ctx_create(int device, stc_ctx** out) {
     STC_CUDA(cudaStreamCreateWithFlags(&c->aux_stream, cudaStreamNonBlocking));
     STC_CUDA(cudaEventCreateWithFlags(&c->ev_ids, cudaEventDisableTiming));
     STC_CUDA(cudaEventCreateWithFlags(&c->ev_sign, cudaEventDisableTiming));
+    STC_CUDA(cudaEventCreateWithFlags(&c->ev_read, cudaEventDisableTiming));
     c->stream = c->own_stream;
     STC_CUDA(cudaMallocHost(&c->h_pinned, C_SLOTS * sizeof(uint64_t)));
     for (auto& e : c->ev) STC_CUDA(cudaEventCreate(&e));
@@ -525,6 +526,7 @@ void stc_ctx_destroy(stc_ctx* c) {
   }
   if (c->ev_ids) cudaEventDestroy(c->ev_ids);
   if (c->ev_sign) cudaEventDestroy(c->ev_sign);
+  if (c->ev_read) cudaEventDestroy(c->ev_read);
   if (c->own_stream) cudaStreamDestroy(c->own_stream);
   (void)cudaGetLastError();
   delete c;

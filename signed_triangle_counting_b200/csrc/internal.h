@@ -163,6 +163,7 @@ struct stc_ctx {
   // says the call's stream has not waited for it yet (wait_sign).
   cudaStream_t aux_stream = nullptr;
   cudaEvent_t ev_ids = nullptr, ev_sign = nullptr;
+  cudaEvent_t ev_read = nullptr;  // a readback that later launches do not delay
   bool sign_pending = false;
   bool host_in_flight = false;  // copies from or to the caller's own pinned memory may be under way
   bool timing = false;
