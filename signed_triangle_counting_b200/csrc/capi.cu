@@ -983,6 +983,15 @@ stc_status stc_test_preset_error(stc_ctx* c, uint32_t word) {
   return STC_OK;
 }
 
+stc_status stc_test_counters(stc_ctx* c, stc_counts* out) {
+  if (!c || !out) return STC_ERR_INVALID_ARGUMENT;
+  return guarded(c, [&] {
+    uint64_t t[4];
+    STC_CUDA(cudaMemcpy(t, counters(c), sizeof(t), cudaMemcpyDeviceToHost));
+    *out = stc_counts{t[C_T0], t[C_T1], t[C_T2], t[C_T3]};
+  });
+}
+
 stc_status stc_autotune(stc_ctx* c, const uint32_t* src, const uint32_t* dst, const int8_t* sign,
                         uint64_t m, const stc_opts* o, uint32_t reps, stc_tuning* out) {
   if (!c || !out || reps == 0 || reps > 100) return STC_ERR_INVALID_ARGUMENT;
@@ -1017,8 +1026,9 @@ stc_status stc_autotune(stc_ctx* c, const uint32_t* src, const uint32_t* dst, co
               cands.push_back(t);
             }
         // The class on both sides: the tail side's class k and the head
-        // side's (bit 5 runs the head pass: its keys, sort and runs are the
-        // same for every candidate, its class-k kernel is not).
+        // side's (bit 5 runs the head pass: its keys, sort and items are the
+        // same for every candidate, its class-k kernel is not).  Short arcs are
+        // counted with the keys, as in a whole count.
         cfg.class_mask = (1u << (k + 1)) | 0x20u;
         float best_ms = 0.f;
         bool first = true;

@@ -2830,9 +2830,8 @@ void count_triangles(stc_ctx* c, const DeviceGraph& gin, const CountConfig& cfg)
       !timed && (cfg.strategy == STC_STRATEGY_AUTO || cfg.strategy == STC_STRATEGY_SEARCH);
   const ClassBounds cb{tiny ? kTinyMax : 1u, kWarpCap, kBlockCap, kLargeCap};
   // Short arcs are counted where the head side's keys are made, unless a
-  // strategy is forced, arcs are timed or classes are counted one at a time.
-  const bool short_arcs =
-      head && !timed && cfg.strategy == STC_STRATEGY_AUTO && cfg.class_mask == 0x3Fu;
+  // strategy is forced or arcs are timed.
+  const bool short_arcs = head && !timed && cfg.strategy == STC_STRATEGY_AUTO;
   if (short_arcs) csr.short_max = kShortArc;
 
   // The persistent engine has no SPLIT path: counts that use SPLIT take the

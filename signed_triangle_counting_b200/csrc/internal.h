@@ -355,3 +355,6 @@ void check_device_error(uint64_t word);
 // For tests: the context's next calls start with this device error word (0 to
 // 255; 0 ends it), as if a kernel before them had set it.
 extern "C" stc_status stc_test_preset_error(stc_ctx* c, uint32_t word);
+// For tests: the type counters as the last count on the context left them (of
+// the last timed count, after stc_autotune).
+extern "C" stc_status stc_test_counters(stc_ctx* c, stc_counts* out);
