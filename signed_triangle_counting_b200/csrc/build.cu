@@ -414,47 +414,6 @@ __global__ void __launch_bounds__(256) k_batch_ids(const uint32_t* __restrict__ 
   if (lane_id() == 0 && self) atomicAdd(ctr + C_SELF, (unsigned long long)self);
 }
 
-// Dedup keys of the union (global ids), as k_pack_dedup.
-__global__ void k_batch_pack(const uint32_t* __restrict__ u, const uint32_t* __restrict__ v,
-                             const int8_t* __restrict__ s, uint64_t m,
-                             const uint64_t* __restrict__ eoff, const uint64_t* __restrict__ vbase,
-                             uint32_t G, uint64_t per_cta, uint32_t bits,
-                             uint64_t* __restrict__ keys) {
-  const uint64_t begin = (uint64_t)blockIdx.x * per_cta;
-  const uint64_t end = begin + per_cta < m ? begin + per_cta : m;
-  if (begin >= end) return;
-  const uint64_t sentinel = (bits * 2 >= 64) ? ~0ull >> 1 : ((1ull << (2 * bits)) - 1);
-  uint32_t g = first_segment(eoff, G, begin);
-  for (uint64_t i = begin + threadIdx.x; i < end; i += blockDim.x) {
-    while (eoff[g + 1] <= i) g++;
-    const uint32_t a = u[i], b = v[i];
-    uint64_t k;
-    if (a == b) {
-      k = sentinel;
-    } else {
-      const uint64_t vb = vbase[g];
-      const uint64_t lo = vb + (a < b ? a : b), hi = vb + (a < b ? b : a);
-      k = (lo << bits) | hi | ((uint64_t)(s[i] < 0) << 63);
-    }
-    keys[i] = k;
-  }
-}
-
-// Adds each vertex's graph above its degree in the vertex sort key, so that
-// ranks are graph-major and (degree, id) within a graph.
-__global__ void k_batch_vertex_graph(uint64_t* __restrict__ vkeys, uint32_t n,
-                                     const uint64_t* __restrict__ vbase, uint32_t G,
-                                     uint64_t per_cta, uint32_t shift) {
-  const uint64_t begin = (uint64_t)blockIdx.x * per_cta;
-  const uint64_t end = begin + per_cta < n ? begin + per_cta : n;
-  if (begin >= end) return;
-  uint32_t g = first_segment(vbase, G, begin);
-  for (uint64_t i = begin + threadIdx.x; i < end; i += blockDim.x) {
-    while (vbase[g + 1] <= i) g++;
-    vkeys[i] |= (uint64_t)g << shift;
-  }
-}
-
 // ------------------------------------------------------- totals path ----
 // A count of totals needs an acyclic orientation, not the reference's: every
 // total order of the vertices counts each triangle once, from its lowest
@@ -1313,7 +1272,7 @@ void graph_from_forward_csr(stc_ctx* c, uint32_t n, uint64_t m, const uint64_t* 
 
 void build_graph_batch(stc_ctx* c, const uint32_t* d_src, const uint32_t* d_dst,
                        const int8_t* d_sign, uint64_t m, const uint64_t* h_eoff, uint32_t G,
-                       DeviceGraph& g, bool totals) {
+                       DeviceGraph& g) {
   cudaStream_t st = c->stream;
   unsigned long long* ctr = (unsigned long long*)counters(c);
   g = DeviceGraph{};
@@ -1347,80 +1306,8 @@ void build_graph_batch(stc_ctx* c, const uint32_t* d_src, const uint32_t* d_dst,
   g.m_valid = m - c->h_pinned[C_SELF];
   g.bits = std::max<uint32_t>(1, bit_width64(ntot ? ntot - 1 : 0));
   g.gbase = d_vbase;
-  if (totals) {
-    const EdgeIds e{d_src, d_dst, d_eoff, d_vbase, G};
-    build_totals(c, e, d_sign, m, g, d_vbase, G, find_hubs(c, e, m));
-    return;
-  }
-  const SortSpace sort_ws = sort_space(c, std::max<uint64_t>(m, g.n));
-  uint64_t* sums = buffer<uint64_t>(c, B_SCAN_SUMS, kScanSums);
-
-  // 2. dedup over the union.
-  uint64_t* ka = buffer<uint64_t>(c, B_KEYS_A, m);
-  uint64_t* kb = buffer<uint64_t>(c, B_KEYS_B, m);
-  g.ukeys = buffer<uint64_t>(c, B_UKEYS, g.m_valid);
-  if (g.m_valid) {
-    k_batch_pack<<<ep.grid, kThreads, 0, st>>>(d_src, d_dst, d_sign, m, d_eoff, d_vbase, G,
-                                                ep.per_cta, g.bits, ka);
-    c->launches++;
-    uint64_t* sorted = radix_sort(ka, kb, m, 0, 2 * (int)g.bits, sort_ws, sort_error(c), st, &c->launches);
-    const uint64_t mask = (1ull << (2 * g.bits)) - 1;
-    const UniqueFlag flag{sorted, mask};
-    const uint32_t grid =
-        range_reduce_scan(flag, g.m_valid, sums, st, &c->launches, sort_error(c));
-    range_apply(flag, UniqueEmit{sorted, g.ukeys}, g.m_valid, sums, st, &c->launches);
-    g.m_unique = read_total(c, sums, grid);
-  }
-  STC_CUDA(cudaGetLastError());
-  mark(c, 2);
-
-  // 3-4. degree and graph-major (graph, degree, id) rank.
-  g.deg = buffer<uint32_t>(c, B_DEG, g.n);
-  g.rank = buffer<uint32_t>(c, B_RANK, g.n);
-  g.verts = buffer<uint32_t>(c, B_VERTS, g.n);
-  g.fdeg = buffer<uint32_t>(c, B_FDEG, g.n);
-  if (g.n) {
-    STC_CUDA(cudaMemsetAsync(g.deg, 0, (size_t)g.n * sizeof(uint32_t), st));
-    STC_CUDA(cudaMemsetAsync(g.fdeg, 0, (size_t)g.n * sizeof(uint32_t), st));
-    if (g.m_unique) {
-      k_degree<<<grid_for(g.m_unique, 16), kThreads, 0, st>>>(g.ukeys, g.m_unique, g.bits, g.deg);
-      c->launches++;
-    }
-    uint64_t* va = buffer<uint64_t>(c, B_VKEYS_A, g.n);
-    uint64_t* vb = buffer<uint64_t>(c, B_VKEYS_B, g.n);
-    k_vertex_keys<<<grid_for(g.n, 4), kThreads, 0, st>>>(g.deg, g.n, va, ctr);
-    c->launches++;
-    read_counters(c, C_MAX_DEG, 1);
-    g.max_deg = (uint32_t)c->h_pinned[C_MAX_DEG];
-    const int dbits = (int)bit_width64(g.max_deg);
-    const int gbits = (int)bit_width64(G > 1 ? G - 1 : 0);
-    if (32 + dbits + gbits > 64) fail(STC_ERR_LIMIT, "batch too large for the vertex sort key");
-    if (gbits) {
-      const RangePartition vp = range_partition(g.n, kSortTile, kMaxSortGrid);
-      k_batch_vertex_graph<<<vp.grid, kThreads, 0, st>>>(va, g.n, d_vbase, G, vp.per_cta, 32 + dbits);
-      c->launches++;
-    }
-    uint64_t* vs = radix_sort(va, vb, g.n, 32, 32 + dbits + gbits, sort_ws, sort_error(c), st, &c->launches);
-    k_rank<<<grid_for(g.n, 4), kThreads, 0, st>>>(vs, g.n, g.verts, g.rank, sort_error(c));
-    c->launches++;
-  }
-  STC_CUDA(cudaGetLastError());
-  mark(c, 3);
-
-  // 5-6. orientation and the forward CSR (graphs stay contiguous in rank space).
-  g.m_fwd = g.m_unique;
-  if (g.m_fwd) {
-    k_arc_keys<<<grid_for(g.m_fwd, 4), kThreads, 0, st>>>(g.ukeys, g.m_fwd, g.bits, g.rank, ka,
-                                                          g.fdeg, sort_error(c));
-    c->launches++;
-    finish_csr_from_arc_keys(c, g, ka, kb);
-  } else {
-    g.off = buffer<uint64_t>(c, B_OFF, (size_t)g.n + 1);
-    STC_CUDA(cudaMemsetAsync(g.off, 0, ((size_t)g.n + 1) * sizeof(uint64_t), st));
-    g.nbr = buffer<uint32_t>(c, B_NBR, 4);
-    g.sgn = buffer<int8_t>(c, B_SGN, 4);
-  }
-  mark(c, 4);
+  const EdgeIds e{d_src, d_dst, d_eoff, d_vbase, G};
+  build_totals(c, e, d_sign, m, g, d_vbase, G, find_hubs(c, e, m));
 }
 
 void build_graph_batch_capped(stc_ctx* c, const uint32_t* d_src, const uint32_t* d_dst,

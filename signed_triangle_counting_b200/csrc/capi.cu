@@ -277,7 +277,7 @@ GroupOut eager_group(stc_ctx* c, const DeviceInput& in, uint64_t me,
                      const std::vector<uint64_t>& eoff, uint32_t gn, CountConfig cfg,
                      std::vector<uint64_t>& h, DeviceGraph& g) {
   clear_counters(c);
-  build_graph_batch(c, in.src, in.dst, in.sign, me, eoff.data(), gn, g, /*totals=*/true);
+  build_graph_batch(c, in.src, in.dst, in.sign, me, eoff.data(), gn, g);
   uint64_t* gc = buffer<uint64_t>(c, B_BATCH_COUNTS, 4ull * gn);
   STC_CUDA(cudaMemsetAsync(gc, 0, 4ull * gn * sizeof(uint64_t), c->stream));
   cfg.graph_counts = gc;

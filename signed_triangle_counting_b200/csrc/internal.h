@@ -278,7 +278,7 @@ void wait_sign(stc_ctx* c);
 // the input's edge copies, id), so no dedup runs before the orientation (the
 // arc sort drops the copies, keeping the first), and g.ukeys stays null.
 // Without it, the reference's (unique degree, id) order, which per-vertex
-// counts, shards, CSR export, the timing recorder and the autotuner use.
+// counts, shards, CSR export and the timing recorder use.
 void build_graph(stc_ctx* c, const uint32_t* d_src, const uint32_t* d_dst, const int8_t* d_sign,
                  uint64_t m, DeviceGraph& g, bool totals = false);
 // Rank-space CSR from a reference-layout forward CSR already on the device.
@@ -286,10 +286,11 @@ void graph_from_forward_csr(stc_ctx* c, uint32_t n, uint64_t m, const uint64_t* 
                             const uint32_t* d_edges, const int8_t* d_signs, const uint32_t* d_rank,
                             DeviceGraph& g);
 // Batch of G graphs stored back to back (host edge offsets h_eoff, G + 1
-// entries): the disjoint union with graph-major ranks; sets g.G / g.gbase.
+// entries): the totals build of the disjoint union with graph-major ranks; sets
+// g.G / g.gbase.
 void build_graph_batch(stc_ctx* c, const uint32_t* d_src, const uint32_t* d_dst,
                        const int8_t* d_sign, uint64_t m, const uint64_t* h_eoff, uint32_t G,
-                       DeviceGraph& g, bool totals = false);
+                       DeviceGraph& g);
 // The totals build of a batch at fixed capacities, with no host
 // synchronisation (capturable): edge offsets are copied from the pinned
 // staging c->h_eoff; g.n and g.m_fwd are capacities and g.m_dev the device

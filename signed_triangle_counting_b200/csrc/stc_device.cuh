@@ -55,20 +55,6 @@ __device__ __forceinline__ T block_exclusive_scan(T v, T* smem, T& total) {
   return r;
 }
 
-// Lanes of the warp holding the same BITS-bit label as this lane, computed
-// with one ballot per label bit (a cheaper warp multi-split than
-// __match_any_sync).  All 32 lanes must call it; labels must fit BITS bits.
-template <int BITS>
-__device__ __forceinline__ unsigned match_label(uint32_t label) {
-  unsigned peers = kFull;
-#pragma unroll
-  for (int b = 0; b < BITS; b++) {
-    const unsigned set = __ballot_sync(kFull, (label >> b) & 1u);
-    peers &= ((label >> b) & 1u) ? set : ~set;
-  }
-  return peers;
-}
-
 // True once an earlier kernel of the call set the error word (an expired wait
 // of a sort, a malformed CSR): what it left must not be used as an index.
 __device__ __forceinline__ bool device_failed(const unsigned long long* __restrict__ err) {
