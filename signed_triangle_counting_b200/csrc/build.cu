@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(256) k_batch_ids(const uint32_t* __restrict__ 
     }
     const uint32_t a = u[i], b = v[i];
     self += a == b;
-    space = max(space, max(a, b) + 1);
+    space = max(space, min(max(a, b), 0xFFFFFFFEu) + 1);  // an id of 2^32 - 1 must not wrap to 0
   }
   // The lanes of a warp mostly end in the same graph.
   const bool one = __all_sync(kFull, g == __shfl_sync(kFull, g, 0));
