@@ -577,7 +577,9 @@ def run_gpu(args) -> None:
             "roofline": {"bound": "hbm", "kernel": "intersection engine (count)",
                          "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                          "frac": achieved / peaks["hbm_gbs"], "peak_source": peaks["source"],
-                         "traffic": traffic, "model": "probe: 5 min(|A'|, |B|) + 30 per arc",
+                         "traffic": traffic,
+                         "model": "probe: 5 min(|A'|, |B|) + 30 per arc (a stream of 4-byte ids "
+                                  "and signs; the short window's heads stream 2.1 of the 5 B)",
                          "alg_bytes_per_launch": probe_bytes, "count_ms": cms,
                          "merge_model_bytes": alg_bytes,
                          "merge_model_achieved": merge_achieved,

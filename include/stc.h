@@ -25,7 +25,8 @@
  * the same order first, which changes no count.  Calls that report per
  * vertex or per id need ids below 2^31 - 2 (vertex counts, shards, the
  * timing recorder) or 2^31 - 1 (CSR export).  An edge list stays below
- * 2^32 elements, and a list's distinct ids below 2^31 - 1.
+ * 2^32 elements (2^31 where it is relabelled), and a list's distinct ids
+ * below 2^31 - 1.
  */
 #ifndef STC_H
 #define STC_H

@@ -1091,6 +1091,8 @@ __global__ void k_relabel(const uint32_t* __restrict__ u, const uint32_t* __rest
 // points *src / *dst at them; returns the number of distinct ids.
 uint64_t relabel_dense(stc_ctx* c, const uint32_t** src, const uint32_t** dst, uint64_t m) {
   cudaStream_t st = c->stream;
+  if (2 * m >= (1ull << 32))  // both endpoints of every edge in one sort
+    fail(STC_ERR_LIMIT, "an edge list with ids from 2^31 - 2 on has 2^31 or more elements");
   const SortSpace sort_ws = sort_space(c, 2 * m);
   uint64_t* sums = buffer<uint64_t>(c, B_SCAN_SUMS, kScanSums);
   uint64_t* ka = buffer<uint64_t>(c, B_KEYS_A, 2 * m);

@@ -2049,11 +2049,12 @@ __device__ __forceinline__ void load8(const uint32_t* __restrict__ p, uint32_t (
 // off in the step that sets the new ones, a claim's keys are loaded while the
 // claim before is streamed, and small items are claimed in small pieces.
 //
-// RMAT scale 24 (97% of the 41.8 G probes): 28.8 ms for the two windows,
-// against 78.8 ms of hash probes for the same heads; the short one 1.7 T
-// probes/s.  Bound by
-// the shared-memory pipe (3.2 wavefronts a probe's load, ranks being random
-// over the banks) and, at that scale, DRAM.  One 32-byte load a chunk instead
+// RMAT scale 24 (97% of the 41.8 G probes): 28.8 ms for the two windows (20.5
+// the short one, at 2.9 TB/s of DRAM, 8.3 the wide one, at 3.2), against 78.8
+// ms of hash probes for the same heads.  At scale 22 the short one takes 4.5 ms
+// for 230 M warp loads of the bitmap and is bound by the shared-memory pipe (76%
+// busy, 2.8 wavefronts a load, ranks being random over the banks) and the integer
+// pipe (75%); DRAM is at a tenth of its rate there.  One 32-byte load a chunk instead
 // of two of 16 took 3.4 ms off, the short window 1.6, its CTAs of 128
 // threads, ten an SM, instead of 512, two an SM, 3.8 (fewer warps wait at an
 // item's barriers; 256 x 5 was 0.4 slower, 128 x 12 2.3); chunks in flight 1,

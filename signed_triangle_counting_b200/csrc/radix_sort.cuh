@@ -255,8 +255,10 @@ __device__ __forceinline__ void rank_keys(const uint64_t (&k)[ITEMS], uint32_t w
 }
 
 // One pass: stable by the digit, one tile per CTA.  Bound by the shared-
-// memory pipe (77% busy: about 31 wavefronts per warp and key, for the
-// match, the counts and the exchange), not by DRAM: 2.8 TB/s at 100 M keys.
+// memory pipe, not by DRAM: over the 67 M arc keys of RMAT scale 22, 367 us for
+// an evenly spread digit (83% busy, 32 wavefronts per warp and key for the
+// match, the counts and the exchange; 2.9 TB/s of DRAM) and 534 us for a skewed
+// one (90% busy, 59 wavefronts, lanes or-ing into one word).
 // The version before (a count pass over the keys, a one-CTA scan of 256
 // counts per CTA, then this) took 2.0 ms a pass over 268 M keys, this 1.5 with
 // its share of the histogram; over 2.4 M keys 78 us (58 of them the scan),

@@ -1,7 +1,8 @@
 """Counts whose ids lie on both sides of 2^30, from where on a tile's count of
 vertices no longer fits a 32-bit state, or reach the id that pads the engine's
 streams (2^31 - 2): totals against the oracle on the same edges with dense ids,
-in the same order; shards, which report by rank, refuse the last."""
+in the same order; shards, which report by rank, refuse the last, and so do
+lists whose relabelling would not fit one sort."""
 import numpy as np
 import pytest
 
@@ -45,3 +46,18 @@ def test_shard_limit():
         with pytest.raises(stc.StcError) as e:
             c.count_shard(src, dst, sign, 0, 2)
         assert e.value.status == stc._capi.STC_ERR_LIMIT
+
+
+def test_relabelled_list_limit():
+    import torch
+    m = 1 << 31  # self-loops but for one edge with a large id
+    src = torch.zeros(m, dtype=torch.int32, device="cuda")
+    dst = torch.zeros(m, dtype=torch.int32, device="cuda")
+    sign = torch.ones(m, dtype=torch.int8, device="cuda")
+    src[0] = -1
+    with stc.Context(0) as c:
+        with pytest.raises(stc.StcError) as e:
+            c.count(src, dst, sign)
+        assert e.value.status == stc._capi.STC_ERR_LIMIT
+    del src, dst, sign
+    torch.cuda.empty_cache()
