@@ -262,9 +262,9 @@ class HostCopier {
   }
 
   // Lets up to `helpers` threads join the call and wakes the first; each wakes
-  // the next, so that the caller pays for one wake-up only.  They join under the mutex and end_call waits only for
-  // those that did: a thread that wakes late finds the call over, and delays
-  // nobody.
+  // the next while parts are left, so that the caller pays for one wake-up only.
+  // They join under the mutex and end_call waits only for those that did: a
+  // thread that wakes late finds the call over, and delays nobody.
   void begin_call(unsigned helpers) {
     if (threads_.empty()) {
       const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
@@ -306,11 +306,11 @@ class HostCopier {
       wakes_--;
       seats_--;
       joined_++;
-      const bool more = seats_ > 0 && wakes_ == 0;
+      const uint32_t n = (uint32_t)parts_.size();
+      const bool more = seats_ > 0 && wakes_ == 0 && next_.load(std::memory_order_relaxed) < n;
       if (more) wakes_ = 1;
       l.unlock();
       if (more) cv_.notify_one();
-      const uint32_t n = (uint32_t)parts_.size();
       auto since = std::chrono::steady_clock::now();
       bool idle = false;  // since then
       while (!cancel_.load(std::memory_order_relaxed) && next_.load(std::memory_order_relaxed) < n) {
